@@ -223,6 +223,21 @@ def test_level_chunks_agree_across_batch_sizes():
     assert err < 1e-6, (k, err)
 
 
+@pytest.mark.parametrize('layers,moist', [(2, False), (9, False), (19, True), (24, False)])
+def test_level_chunks_give_the_same_bits(layers, moist):
+  # The column sums are added in the same four parts whatever the chunk count
+  # (one, two or four chunks for these sizes), so batch sizes agree exactly in
+  # the temperature tendency of every member.
+  kw = dict(tracers=_tracers, humidity='specific_humidity') if moist else {}
+  og, oeq, st, g, eq = make('T42', layers=layers, **kw)
+  s1 = to_state(st)
+  batch = pe.State(*[torch.stack([getattr(s1, k)] * 16) for k in KEYS],
+                   tracers={k: torch.stack([v] * 16) for k, v in s1.tracers.items()})
+  ob, o1 = eq.explicit_terms(batch), eq.explicit_terms(s1)
+  for k in KEYS:
+    assert torch.equal(getattr(ob, k)[11], getattr(o1, k)), k
+
+
 def test_dry_tracer_advection_matches_oracle():
   og, oeq, st, g, eq = make(tracers=_tracers)
   got = eq.explicit_terms(to_state(st))
