@@ -131,7 +131,7 @@ struct dino_plan {
   int lw = 0, L = 0, I = 0, J = 0, M = 0, Jh = 0, N = 0;
   int spacing = 0, precision = 0, max_fields = 0, device = 0;
   double radius = 1.0;
-  bool fft_pow2 = false;
+  bool fft = false;  // I / 2 has a real FFT (else longitude sums are direct)
   // FP64 nodes and weights (device and host copies).
   double* d_x64 = nullptr;
   double* d_w64 = nullptr;
@@ -207,6 +207,8 @@ int fourier_forward(dino_plan* p, const float* nodal, float* fourier,
                     int nfields, bool weighted, cudaStream_t st);
 int modal_op(dino_plan* p, int op, const float* in, float* out, int nfields,
              int arg, cudaStream_t st);
+// Whether the real FFT covers a half length I / 2 = n.
+bool fft_supported(int n);
 // Sets kernel attributes ahead of stream capture.
 int sht_prepare(dino_plan* p);
 // FP32 SIMT inverse Legendre contraction for any plan (no precision dispatch).

@@ -135,8 +135,6 @@ __global__ void legendre_table_kernel(int lw, int L, int Jh,
   }
 }
 
-static bool is_pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }
-
 template <typename T>
 static int upload(T** dst, const std::vector<T>& src) {
   DINO_CHECK_CUDA(cudaMalloc((void**)dst, sizeof(T) * (src.empty() ? 1 : src.size())));
@@ -244,11 +242,10 @@ static int plan_build(dino_plan* p, const dino_grid_desc* d) {
     DINO_TRY(upload(&p->d_fbasis, f));
   }
 
-  // Twiddles for the power-of-two real FFT path.
+  // Twiddles for the real FFT path.
   p->N = I / 2;
-  p->fft_pow2 = (I % 2 == 0) && is_pow2(p->N) && p->N >= 8 && p->N <= 512 &&
-                lw <= p->N;
-  if (p->fft_pow2) {
+  p->fft = (I % 2 == 0) && fft_supported(p->N) && lw <= p->N;
+  if (p->fft) {
     std::vector<float2> tn(p->N), ti(p->N);
     for (int k = 0; k < p->N; ++k) {
       double an = 2.0 * M_PI * k / p->N, ai = 2.0 * M_PI * k / I;

@@ -378,110 +378,187 @@ int legendre_forward_fp32(dino_plan* p, const float* G, float* out, int nf,
 }
 
 // ---------------------------------------------------------------------------
-// Real FFT over longitude (power-of-two I = 2N), shared-memory Stockham
-// radix-4/2 on the half-length complex sequence z[n] = x[2n] + i x[2n+1].
+// Real FFT over longitude (I = 2N, N of FftCfg below): shared-memory Stockham
+// passes on the half-length complex sequence z[n] = x[2n] + i x[2n+1].
+//
+// A thread works on two adjacent latitudes at once, so every complex value is
+// a pair of packed f32x2 registers (re of both columns, im of both columns):
+// one issue slot does both columns' add, multiply or FMA at the plain lane
+// rate (126 lane results per SM and clock, measured for fma and fma.f32x2
+// alike).  With one column per thread the kernels issued in 57-70 % of the
+// slots; now 35 %, and they wait on memory (long scoreboard 44 % of the stall
+// cycles at TL255).  T42 x 900 fields: inverse 18.6 -> 12.4 us, forward 14.7 ->
+// 10.6 us; T85 x 128: 10.7 -> 8.4, 10.5 -> 8.4 us; TL255 x 128: 37.0 -> 37.1,
+// 33.0 -> 31.1 us.  Against direct sums for lengths that are no power of two:
+// TL159 x 75 fields 615 -> 10.4 us and 636 -> 10.4 us.
 // ---------------------------------------------------------------------------
 
-constexpr int kFftJS = 16;       // latitudes (columns) per CTA
-constexpr int kFftThreads = 256;
-static_assert(kFftThreads % kFftJS == 0, "a thread keeps one FFT column in every pass");
+// Packed arithmetic on two columns.
+__device__ __forceinline__ float2 padd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 pmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 pfma(float2 a, float2 b, float2 c) {
+  return __ffma2_rn(a, b, c);
+}
+// a - b (one rounding: b * -1 is exact).
+__device__ __forceinline__ float2 psub(float2 a, float2 b) {
+  return __ffma2_rn(b, make_float2(-1.f, -1.f), a);
+}
+__device__ __forceinline__ float2 dup(float a) { return make_float2(a, a); }
 
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+// One complex value of two columns.
+struct cpair {
+  float2 re, im;
+};
+__device__ __forceinline__ cpair cadd(cpair a, cpair b) {
+  return {padd(a.re, b.re), padd(a.im, b.im)};
 }
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) {
-  return make_float2(a.x + b.x, a.y + b.y);
+__device__ __forceinline__ cpair csub(cpair a, cpair b) {
+  return {psub(a.re, b.re), psub(a.im, b.im)};
 }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) {
-  return make_float2(a.x - b.x, a.y - b.y);
-}
-__device__ __forceinline__ float2 cconj(float2 a) { return make_float2(a.x, -a.y); }
-// Multiply by +i (kSign = +1) or -i (kSign = -1).
+// a + i kSign b and a - i kSign b: a quarter turn is a choice of operands.
 template <int kSign>
-__device__ __forceinline__ float2 cmul_i(float2 a) {
-  return kSign > 0 ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
+__device__ __forceinline__ cpair cadd_i(cpair a, cpair b) {
+  return kSign > 0 ? cpair{psub(a.re, b.im), padd(a.im, b.re)}
+                   : cpair{padd(a.re, b.im), psub(a.im, b.re)};
+}
+template <int kSign>
+__device__ __forceinline__ cpair csub_i(cpair a, cpair b) {
+  return cadd_i<-kSign>(a, b);
+}
+// a (wr + i wi), the same factor for both columns; nwi = -wi.
+__device__ __forceinline__ cpair cmul_w(cpair a, float2 wr, float2 wi, float2 nwi) {
+  return {pfma(a.re, wr, pmul(a.im, nwi)), pfma(a.re, wi, pmul(a.im, wr))};
 }
 
-// exp(2 pi i k / 16), k = 0..7 (the 16th roots of unity used by the
-// register DFTs; cos/sin of multiples of pi/8).
-__device__ __forceinline__ float2 root16(int k) {
+// Multiplies by exp(kSign 2 pi i K / 16) for a compile-time K in [0, 9].
+template <int K, int kSign>
+__device__ __forceinline__ cpair twiddle16(cpair a) {
   constexpr float c1 = 0.92387953251128674f, s1 = 0.38268343236508977f;
   constexpr float h = 0.70710678118654757f;
-  switch (k & 7) {
-    case 0: return make_float2(1.f, 0.f);
-    case 1: return make_float2(c1, s1);
-    case 2: return make_float2(h, h);
-    case 3: return make_float2(s1, c1);
-    case 4: return make_float2(0.f, 1.f);
-    case 5: return make_float2(-s1, c1);
-    case 6: return make_float2(-h, h);
-    default: return make_float2(-c1, s1);
-  }
-}
-
-// exp(kSign 2 pi i k / 16) for any k >= 0.
-template <int kSign>
-__device__ __forceinline__ float2 w16(int k) {
-  float2 w = root16(k & 7);
-  if (k & 8) w = make_float2(-w.x, -w.y);
-  return kSign < 0 ? cconj(w) : w;
-}
-
-// Multiplies by exp(kSign 2 pi i k / 16) for a compile-time k: multiples of
-// 4 are sign swaps (no multiply), the others one complex multiply.
-template <int K, int kSign>
-__device__ __forceinline__ float2 twiddle16(float2 a) {
-  constexpr int k = K & 15;
-  if constexpr (k == 0) {
+  constexpr float co[10] = {1.f, c1, h, s1, 0.f, -s1, -h, -c1, -1.f, -c1};
+  constexpr float si[10] = {0.f, s1, h, c1, 1.f, c1, h, s1, 0.f, -s1};
+  if constexpr (K == 0) {
     return a;
-  } else if constexpr (k == 4) {
-    return cmul_i<kSign>(a);
-  } else if constexpr (k == 8) {
-    return make_float2(-a.x, -a.y);
-  } else if constexpr (k == 12) {
-    return cmul_i<-kSign>(a);
+  } else if constexpr (K == 4) {
+    const float2 z = make_float2(0.f, 0.f);
+    return kSign > 0 ? cpair{psub(z, a.im), a.re} : cpair{a.im, psub(z, a.re)};
   } else {
-    return cmul(a, w16<kSign>(k));
+    constexpr float wi = kSign * si[K];
+    return cmul_w(a, dup(co[K]), dup(wi), dup(-wi));
   }
 }
 
 // DFT of length 4: X_k = sum_q v_q exp(kSign 2 pi i q k / 4).
 template <int kSign>
-__device__ __forceinline__ void dft4(float2& a, float2& b, float2& c, float2& d) {
-  const float2 s0 = cadd(a, c), d0 = csub(a, c);
-  const float2 s1 = cadd(b, d), d1 = cmul_i<kSign>(csub(b, d));
+__device__ __forceinline__ void dft4(cpair& a, cpair& b, cpair& c, cpair& d) {
+  const cpair s0 = cadd(a, c), d0 = csub(a, c);
+  const cpair s1 = cadd(b, d), d1 = csub(b, d);
   a = cadd(s0, s1);
   c = csub(s0, s1);
-  b = cadd(d0, d1);
-  d = csub(d0, d1);
+  b = cadd_i<kSign>(d0, d1);
+  d = csub_i<kSign>(d0, d1);
 }
 
-// In-register DFT of length R (power of two <= 16), natural order in and
-// out: v_s <- sum_q v_q exp(kSign 2 pi i q s / R).  Lengths 4 and 16 use
-// DFT-4 butterflies (16 = 4 x 4 with the twiddles of multiples of 4 as sign
-// swaps); 2 and 8 split once more by two.
 template <int R, int kSign>
-__device__ __forceinline__ void dft_reg(float2* v) {
-  if constexpr (R == 1) {
-    return;
-  } else if constexpr (R == 2) {
-    float2 a = v[0], b = v[1];
+__device__ __forceinline__ void dft_reg(cpair* v);
+
+// In-register DFT of length A B with A and B coprime (Good 1958; Thomas
+// 1963): the inputs n = B n1 + A n2 (mod A B) make it an A x B
+// two-dimensional DFT without twiddles, whose entry (k mod A, k mod B) is X_k.
+template <int A, int B, int kSign>
+__device__ __forceinline__ void dft_coprime(cpair* v) {
+  constexpr int R = A * B;
+  cpair t[R];
+#pragma unroll
+  for (int n1 = 0; n1 < A; ++n1) {
+    cpair row[B];
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) row[n2] = v[(B * n1 + A * n2) % R];
+    dft_reg<B, kSign>(row);
+#pragma unroll
+    for (int k2 = 0; k2 < B; ++k2) t[n1 * B + k2] = row[k2];
+  }
+#pragma unroll
+  for (int k2 = 0; k2 < B; ++k2) {
+    cpair col[A];
+#pragma unroll
+    for (int n1 = 0; n1 < A; ++n1) col[n1] = t[n1 * B + k2];
+    dft_reg<A, kSign>(col);
+#pragma unroll
+    for (int k1 = 0; k1 < A; ++k1) t[k1 * B + k2] = col[k1];
+  }
+#pragma unroll
+  for (int k = 0; k < R; ++k) v[k] = t[(k % A) * B + k % B];
+}
+
+// In-register DFT of length R, natural order in and out:
+// v_s <- sum_q v_q exp(kSign 2 pi i q s / R).
+template <int R, int kSign>
+__device__ __forceinline__ void dft_reg(cpair* v) {
+  if constexpr (R == 2) {
+    const cpair a = v[0], b = v[1];
     v[0] = cadd(a, b);
     v[1] = csub(a, b);
+  } else if constexpr (R == 3) {
+    // X1,2 = (a - (b + c) / 2) +- i sin(pi/3) (b - c).
+    constexpr float s3 = 0.86602540378443865f;
+    const cpair t = cadd(v[1], v[2]), u = csub(v[1], v[2]);
+    const cpair m = {pfma(t.re, dup(-0.5f), v[0].re), pfma(t.im, dup(-0.5f), v[0].im)};
+    const float2 p = dup(kSign * s3), n = dup(-kSign * s3);
+    v[0] = cadd(v[0], t);
+    v[1] = {pfma(u.im, n, m.re), pfma(u.re, p, m.im)};
+    v[2] = {pfma(u.im, p, m.re), pfma(u.re, n, m.im)};
   } else if constexpr (R == 4) {
     dft4<kSign>(v[0], v[1], v[2], v[3]);
+  } else if constexpr (R == 5) {
+    constexpr float c1 = 0.30901699437494742f, c2 = -0.80901699437494742f;
+    constexpr float s1 = 0.95105651629515357f, s2 = 0.58778525229247313f;
+    const cpair t1 = cadd(v[1], v[4]), u1 = csub(v[1], v[4]);
+    const cpair t2 = cadd(v[2], v[3]), u2 = csub(v[2], v[3]);
+    const cpair m1 = {pfma(t2.re, dup(c2), pfma(t1.re, dup(c1), v[0].re)),
+                      pfma(t2.im, dup(c2), pfma(t1.im, dup(c1), v[0].im))};
+    const cpair m2 = {pfma(t2.re, dup(c1), pfma(t1.re, dup(c2), v[0].re)),
+                      pfma(t2.im, dup(c1), pfma(t1.im, dup(c2), v[0].im))};
+    const cpair w1 = {pfma(u2.re, dup(s2), pmul(u1.re, dup(s1))),
+                      pfma(u2.im, dup(s2), pmul(u1.im, dup(s1)))};
+    const cpair w2 = {pfma(u2.re, dup(-s1), pmul(u1.re, dup(s2))),
+                      pfma(u2.im, dup(-s1), pmul(u1.im, dup(s2)))};
+    v[0] = cadd(v[0], cadd(t1, t2));
+    v[1] = cadd_i<kSign>(m1, w1);
+    v[4] = csub_i<kSign>(m1, w1);
+    v[2] = cadd_i<kSign>(m2, w2);
+    v[3] = csub_i<kSign>(m2, w2);
+  } else if constexpr (R == 8) {
+    cpair e[4], o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      e[i] = v[2 * i];
+      o[i] = v[2 * i + 1];
+    }
+    dft_reg<4, kSign>(e);
+    dft_reg<4, kSign>(o);
+    o[1] = twiddle16<2, kSign>(o[1]);
+    o[3] = twiddle16<6, kSign>(o[3]);
+    v[0] = cadd(e[0], o[0]);
+    v[4] = csub(e[0], o[0]);
+    v[1] = cadd(e[1], o[1]);
+    v[5] = csub(e[1], o[1]);
+    v[2] = cadd_i<kSign>(e[2], o[2]);
+    v[6] = csub_i<kSign>(e[2], o[2]);
+    v[3] = cadd(e[3], o[3]);
+    v[7] = csub(e[3], o[3]);
   } else if constexpr (R == 16) {
     // q = 4 q1 + q2, s = s1 + 4 s2: DFT-4 over q1 for each q2, twiddle
     // W16^(q2 s1), DFT-4 over q2 for each s1.
-    float2 y[16];
+    cpair y[16];
 #pragma unroll
     for (int q2 = 0; q2 < 4; ++q2) {
-      float2 a = v[q2], b = v[4 + q2], c = v[8 + q2], d = v[12 + q2];
+      cpair a = v[q2], b = v[4 + q2], c = v[8 + q2], d = v[12 + q2];
       dft4<kSign>(a, b, c, d);
-      y[4 * q2] = a;      // s1 = 0
-      y[4 * q2 + 1] = b;  // s1 = 1
-      y[4 * q2 + 2] = c;  // s1 = 2
-      y[4 * q2 + 3] = d;  // s1 = 3
+      y[4 * q2] = a;
+      y[4 * q2 + 1] = b;
+      y[4 * q2 + 2] = c;
+      y[4 * q2 + 3] = d;
     }
     y[5] = twiddle16<1, kSign>(y[5]);
     y[6] = twiddle16<2, kSign>(y[6]);
@@ -494,357 +571,327 @@ __device__ __forceinline__ void dft_reg(float2* v) {
     y[15] = twiddle16<9, kSign>(y[15]);
 #pragma unroll
     for (int s1 = 0; s1 < 4; ++s1) {
-      float2 a = y[s1], b = y[4 + s1], c = y[8 + s1], d = y[12 + s1];
+      cpair a = y[s1], b = y[4 + s1], c = y[8 + s1], d = y[12 + s1];
       dft4<kSign>(a, b, c, d);
       v[s1] = a;
       v[s1 + 4] = b;
       v[s1 + 8] = c;
       v[s1 + 12] = d;
     }
+  } else if constexpr (R == 6) {
+    dft_coprime<2, 3, kSign>(v);
+  } else if constexpr (R == 10) {
+    dft_coprime<2, 5, kSign>(v);
+  } else if constexpr (R == 12) {
+    dft_coprime<3, 4, kSign>(v);
+  } else if constexpr (R == 15) {
+    dft_coprime<3, 5, kSign>(v);
   } else {
-    // R = 8: even / odd halves, then W8^k = W16^(2k) on the odd half.
-    constexpr int H = R / 2;
-    float2 e[H], o[H];
-#pragma unroll
-    for (int i = 0; i < H; ++i) {
-      e[i] = v[2 * i];
-      o[i] = v[2 * i + 1];
-    }
-    dft_reg<H, kSign>(e);
-    dft_reg<H, kSign>(o);
-    const float2 t0 = o[0];
-    const float2 t1 = twiddle16<2, kSign>(o[1]);
-    const float2 t2 = twiddle16<4, kSign>(o[2]);
-    const float2 t3 = twiddle16<6, kSign>(o[3]);
-    v[0] = cadd(e[0], t0);
-    v[4] = csub(e[0], t0);
-    v[1] = cadd(e[1], t1);
-    v[5] = csub(e[1], t1);
-    v[2] = cadd(e[2], t2);
-    v[6] = csub(e[2], t2);
-    v[3] = cadd(e[3], t3);
-    v[7] = csub(e[3], t3);
+    static_assert(R == 20, "radix");
+    dft_coprime<4, 5, kSign>(v);
   }
 }
 
-// One radix-R Stockham pass over N points for kFftJS columns.  load(n, c)
-// returns element n of column c; store(n, c, v) writes output element n.
-// Every thread issues all of its loads before its first store; kSync puts a
-// barrier between the two, so that the pass may run in place on one shared
-// buffer.
-template <int N, int R, int kSign, bool kSync, class Load, class Store>
-__device__ __forceinline__ void stockham_pass(int Ns, const float2* twn,
-                                              Load load, Store store) {
+// Radices (at most three passes), threads, the CTAs per SM that bound the
+// registers, and column pairs per CTA for each supported half length: every N
+// of the named grids.  Passes are few and wide (a pass costs a round trip
+// through shared memory and a barrier) and the thread count is near the widest
+// pass's N / R x pairs items.  16 pairs make a row segment a full 128-byte
+// line: TL255 (N = 256), 128 fields: 2 CTAs of 256 threads and 16 pairs 37.1 /
+// 31.1 us (inverse / forward), pair 146 us; 5 of 128 threads and 8 pairs 37.2 /
+// 35.0 us, 155 us; a register bound of 80 (6 CTAs) 43 / 45 us.  T42 (N = 64),
+// 900 fields: 16 pairs 12.4 / 10.6 us, 8 pairs 12.6 / 12.6 us.  Shorter rows
+// (N <= 48) and the lengths whose passes hold 60-80 registers (160 on) keep 8.
+template <int N> struct FftCfg;
+#define DINO_FFT_CFG(N, R1, R2, R3, THREADS, CTAS, PAIRS)                  \
+  template <> struct FftCfg<N> {                                           \
+    static constexpr int r1 = R1, r2 = R2, r3 = R3, threads = THREADS,     \
+                         ctas = CTAS, pairs = PAIRS;                       \
+    static_assert(R1 * R2 * R3 == N && THREADS % PAIRS == 0, "radices");    \
+  };
+DINO_FFT_CFG(8, 8, 1, 1, 32, 16, 8)
+DINO_FFT_CFG(16, 16, 1, 1, 32, 16, 8)
+DINO_FFT_CFG(32, 8, 4, 1, 64, 14, 8)
+DINO_FFT_CFG(48, 8, 6, 1, 64, 14, 8)
+DINO_FFT_CFG(64, 8, 8, 1, 128, 5, 16)
+DINO_FFT_CFG(96, 12, 8, 1, 192, 4, 16)
+DINO_FFT_CFG(128, 16, 8, 1, 128, 4, 16)
+DINO_FFT_CFG(160, 16, 10, 1, 128, 5, 8)
+DINO_FFT_CFG(180, 12, 15, 1, 128, 5, 8)
+DINO_FFT_CFG(256, 16, 16, 1, 256, 2, 16)
+DINO_FFT_CFG(320, 16, 20, 1, 160, 3, 8)
+DINO_FFT_CFG(512, 8, 8, 8, 256, 2, 8)
+DINO_FFT_CFG(640, 8, 8, 10, 320, 2, 8)
+DINO_FFT_CFG(1280, 16, 8, 10, 640, 1, 8)
+#undef DINO_FFT_CFG
+
+bool fft_supported(int n) {
+  switch (n) {
+    case 8: case 16: case 32: case 48: case 64: case 96: case 128: case 160:
+    case 180: case 256: case 320: case 512: case 640: case 1280:
+      return true;
+  }
+  return false;
+}
+
+// Shared memory of both kernels: N x pairs complex column pairs and the N
+// twiddles exp(kSign 2 pi i k / N) as (re, re, im, im).
+template <int N>
+constexpr size_t fft_smem_bytes() {
+  return sizeof(float4) * ((size_t)N * FftCfg<N>::pairs + N);
+}
+
+__device__ __forceinline__ cpair ld_cpair(const float4* s) {
+  const float4 t = *s;
+  return {make_float2(t.x, t.y), make_float2(t.z, t.w)};
+}
+__device__ __forceinline__ void st_cpair(float4* s, cpair v) {
+  *s = make_float4(v.re.x, v.re.y, v.im.x, v.im.y);
+}
+
+// One radix-R Stockham pass over N points for P column pairs.
+// load(n) returns element n of the thread's column pair (tid mod P in
+// every pass); store(n, v) writes output element n.  Every thread issues all
+// of its loads before its first store; kSync puts a barrier between the two,
+// so that the pass may run in place on one shared buffer.
+template <int N, int R, int Ns, int kSign, bool kSync, class Load, class Store>
+__device__ __forceinline__ void stockham_pass(const float4* tw, Load load, Store store) {
+  constexpr int T = FftCfg<N>::threads;
   constexpr int Q = N / R;
-  constexpr int kTotal = Q * kFftJS;
-  constexpr int kItems = (kTotal + kFftThreads - 1) / kFftThreads;
-  const int stride = N / (Ns * R);
-  float2 v[kItems][R];
+  constexpr int P = FftCfg<N>::pairs;
+  constexpr int kRows = T / P;  // items per column pair and round
+  constexpr int kItems = (Q + kRows - 1) / kRows;
+  constexpr int stride = N / (Ns * R);
+  const int j0 = threadIdx.x / P;
+  cpair v[kItems][R];
 #pragma unroll
   for (int it = 0; it < kItems; ++it) {
-    const int item = threadIdx.x + it * kFftThreads;
-    if (item < kTotal) {
-      const int c = item % kFftJS, j = item / kFftJS;
+    const int j = j0 + it * kRows;
+    if (j < Q) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[it][r] = load(j + r * Q, c);
+      for (int r = 0; r < R; ++r) v[it][r] = load(j + r * Q);
     }
   }
   if (kSync) __syncthreads();
 #pragma unroll
   for (int it = 0; it < kItems; ++it) {
-    const int item = threadIdx.x + it * kFftThreads;
-    if (item < kTotal) {
-      const int c = item % kFftJS, j = item / kFftJS;
+    const int j = j0 + it * kRows;
+    if (j < Q) {
       const int k = j % Ns;
-      if (k) {
+      if constexpr (Ns > 1) {
 #pragma unroll
         for (int r = 1; r < R; ++r) {
-          float2 w = twn[r * k * stride];
-          if (kSign < 0) w = cconj(w);
-          v[it][r] = cmul(v[it][r], w);
+          const float4 w = tw[r * k * stride];
+          const float2 wr = make_float2(w.x, w.y), wi = make_float2(w.z, w.w);
+          const cpair a = v[it][r];
+          v[it][r] = {psub(pmul(a.re, wr), pmul(a.im, wi)), pfma(a.re, wi, pmul(a.im, wr))};
         }
       }
       dft_reg<R, kSign>(v[it]);
       const int base = (j / Ns) * Ns * R + k;
 #pragma unroll
-      for (int r = 0; r < R; ++r) store(base + r * Ns, c, v[it][r]);
+      for (int r = 0; r < R; ++r) store(base + r * Ns, v[it][r]);
     }
   }
 }
 
-// Radix schedule (at most three passes) for each supported N.
-template <int N> struct FftRadix;
-template <> struct FftRadix<8> { static constexpr int r1 = 8, r2 = 1, r3 = 1; };
-template <> struct FftRadix<16> { static constexpr int r1 = 16, r2 = 1, r3 = 1; };
-template <> struct FftRadix<32> { static constexpr int r1 = 8, r2 = 4, r3 = 1; };
-template <> struct FftRadix<64> { static constexpr int r1 = 8, r2 = 8, r3 = 1; };
-template <> struct FftRadix<128> { static constexpr int r1 = 16, r2 = 8, r3 = 1; };
-template <> struct FftRadix<256> { static constexpr int r1 = 16, r2 = 16, r3 = 1; };
-template <> struct FftRadix<512> { static constexpr int r1 = 8, r2 = 8, r3 = 8; };
-
-// Shared memory of both kernels: one N x kFftJS complex buffer and the two
-// N-entry twiddle tables.
-template <int N>
-constexpr size_t fft_smem_bytes() {
-  return sizeof(float2) * ((size_t)N * kFftJS + 2 * N);
-}
-
-// Runs all passes on the one shared buffer S: the first pass reads via
-// `first` (in place when kFirstInS), the last writes via `last`; the passes
-// between run in place.
-// kLastInS: the last pass writes back into S (in place, so its loads finish
-// before its stores).
-template <int N, int kSign, bool kFirstInS, bool kLastInS = false, class First, class Last>
-__device__ __forceinline__ void fft_passes(float2* S, const float2* twn, First first,
+// Runs all passes; the first reads via `first` (in place on S when kFirstInS)
+// and the last writes via `last` (in place on S when kLastInS).
+template <int N, int kSign, bool kFirstInS, bool kLastInS, class First, class Last>
+__device__ __forceinline__ void fft_passes(float4* S, const float4* tw, First first,
                                            Last last) {
-  using Rd = FftRadix<N>;
-  auto s_load = [S](int n, int c) { return S[n * kFftJS + c]; };
-  auto s_store = [S](int n, int c, float2 v) { S[n * kFftJS + c] = v; };
-  if constexpr (Rd::r2 == 1) {
-    stockham_pass<N, Rd::r1, kSign, kFirstInS || kLastInS>(1, twn, first, last);
-  } else if constexpr (Rd::r3 == 1) {
-    stockham_pass<N, Rd::r1, kSign, kFirstInS>(1, twn, first, s_store);
+  using C = FftCfg<N>;
+  constexpr int P = C::pairs;
+  const int p = threadIdx.x % P;
+  auto s_load = [S, p](int n) { return ld_cpair(S + n * P + p); };
+  auto s_store = [S, p](int n, cpair v) { st_cpair(S + n * P + p, v); };
+  if constexpr (C::r2 == 1) {
+    stockham_pass<N, C::r1, 1, kSign, kFirstInS && kLastInS>(tw, first, last);
+  } else if constexpr (C::r3 == 1) {
+    stockham_pass<N, C::r1, 1, kSign, kFirstInS>(tw, first, s_store);
     __syncthreads();
-    stockham_pass<N, Rd::r2, kSign, kLastInS>(Rd::r1, twn, s_load, last);
+    stockham_pass<N, C::r2, C::r1, kSign, kLastInS>(tw, s_load, last);
   } else {
-    stockham_pass<N, Rd::r1, kSign, kFirstInS>(1, twn, first, s_store);
+    stockham_pass<N, C::r1, 1, kSign, kFirstInS>(tw, first, s_store);
     __syncthreads();
-    stockham_pass<N, Rd::r2, kSign, true>(Rd::r1, twn, s_load, s_store);
+    stockham_pass<N, C::r2, C::r1, kSign, true>(tw, s_load, s_store);
     __syncthreads();
-    stockham_pass<N, Rd::r3, kSign, kLastInS>(Rd::r1 * Rd::r2, twn, s_load, last);
+    stockham_pass<N, C::r3, C::r1 * C::r2, kSign, kLastInS>(tw, s_load, last);
   }
 }
 
-// Copies a rows x kFftJS tile (row stride J floats) into shared memory
-// (row stride kFftJS): 16-byte asynchronous copies when rows start 16-byte
-// aligned and the tile is full, else scalar loads with zero fill past ncol.
-template <int kMaxRows>
-__device__ __forceinline__ void stage_tile(const float* __restrict__ src, int rows,
-                                           int J, int ncol, float* dst) {
-  if ((J & 3) == 0 && ncol == kFftJS && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-    constexpr int kQ = kFftJS / 4;  // float4 per row
-    // 16-byte asynchronous copies (cp.async): every copy of the thread is in
-    // flight at once and none holds a register; the caller's barrier follows
-    // the wait below.
-    constexpr int kChunks = (kMaxRows * kQ + kFftThreads - 1) / kFftThreads;
-#pragma unroll
-    for (int i = 0; i < kChunks; ++i) {
-      const int t = threadIdx.x + i * kFftThreads;
-      const int r = t / kQ, q = t % kQ;
-      if (r < rows) {
-        const float* g = src + (size_t)r * J + 4 * q;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                         (uint32_t)__cvta_generic_to_shared(reinterpret_cast<float4*>(dst) + t)),
-                     "l"(g)
-                     : "memory");
-      }
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
+// The two columns of a row for one thread: one 8-byte access when kVec (even
+// J and 8-byte aligned bases, so `cols` is 0 or 2), else scalar ones.
+template <bool kVec>
+__device__ __forceinline__ float2 ld_cols(const float* __restrict__ g, int cols) {
+  if (kVec)
+    return cols ? *reinterpret_cast<const float2*>(g) : make_float2(0.f, 0.f);
+  return make_float2(cols > 0 ? g[0] : 0.f, cols > 1 ? g[1] : 0.f);
+}
+template <bool kVec>
+__device__ __forceinline__ void st_cols(float* g, float2 v, int cols) {
+  if (kVec) {
+    if (cols) *reinterpret_cast<float2*>(g) = v;
   } else {
-    for (int t = threadIdx.x; t < rows * kFftJS; t += kFftThreads) {
-      const int r = t / kFftJS, c = t % kFftJS;
-      dst[t] = (c < ncol) ? src[(size_t)r * J + c] : 0.f;
-    }
+    if (cols > 0) g[0] = v.x;
+    if (cols > 1) g[1] = v.y;
   }
 }
 
 // Fourier coefficients F[b][row][j] -> nodal[b][i][j] (optionally scaled by
 // wq[j], which gives the adjoint of the weighted forward transform).
-// Z[k] = (X[k] + conj X[N-k]) + i w_I^k (X[k] - conj X[N-k]), then
-// z = IDFT_N(Z) and x[2n] = Re z[n], x[2n+1] = Im z[n].  The coefficient tile
-// (at most 2N - 1 rows of kFftJS floats) is staged in the shared buffer, Z is
-// formed in registers in two halves and written back over it, the passes run
-// in place and a per-column copy writes the nodal rows.  Up to N = 256 the
-// kernel fits 48 registers, so five CTAs (36 KB of shared memory each) share
-// an SM.
-template <int N>
-__global__ void __launch_bounds__(kFftThreads, N <= 256 ? 5 : 3)
+// With A = X[k] + conj X[N-k], B = X[k] - conj X[N-k] and T = w_I^k B, the
+// half-length spectrum is Z[k] = A + i T and Z[N-k] = conj(A) + i conj(T)
+// (w_I^(N-k) = -conj w_I^k); then z = IDFT_N(Z) and x[2n] = Re z[n],
+// x[2n+1] = Im z[n].  Z is formed from the coefficients' global rows (four
+// 8-byte loads an item, eight items in flight a thread), the first passes run
+// in place in shared memory and the last writes the nodal rows.
+template <int N, bool kVec>
+__global__ void __launch_bounds__(FftCfg<N>::threads, FftCfg<N>::ctas)
 rfft_inverse_kernel(const float* __restrict__ F, float* __restrict__ out,
                     int M, int lw, int J, const float2* __restrict__ tw_n,
                     const float2* __restrict__ tw_i,
                     const float* __restrict__ wq) {
-  extern __shared__ float2 sm[];
-  float2* S = sm;
-  float2* twn = S + N * kFftJS;
-  float2* twi = twn + N;
-  const int tid = threadIdx.x;
+  constexpr int T = FftCfg<N>::threads, P = FftCfg<N>::pairs;
+  extern __shared__ float4 sm[];
+  float4* S = sm;
+  float4* tw = S + N * P;
+  const int tid = threadIdx.x, p = tid % P;
   const int b = blockIdx.y;
-  const int j0 = blockIdx.x * kFftJS;
-  const int ncol = min(kFftJS, J - j0);
-  for (int t = tid; t < N; t += kFftThreads) {
-    twn[t] = tw_n[t];
-    twi[t] = tw_i[t];
+  const int col = (blockIdx.x * P + p) * 2;
+  const int cols = max(0, min(2, J - col));
+  for (int t = tid; t < N; t += T) {
+    const float2 w = tw_n[t];
+    tw[t] = make_float4(w.x, w.x, w.y, w.y);
   }
-  const float* Fb = F + (size_t)b * M * J + j0;
-  const int rows = min(M, 2 * min(lw, N) - 1);  // rows X() reads; <= 2N - 1
-  const float* src = reinterpret_cast<const float*>(S);
-  stage_tile<2 * N>(Fb, rows, J, ncol, reinterpret_cast<float*>(S));
-  __syncthreads();
+  const float* Fb = F + (size_t)b * M * J + col;
   const float inv_sqrt_2pi = 0.3989422804014327f;
   const float half_inv_sqrt_pi = 0.28209479177387814f;
-  auto X = [&](int k, int c) -> float2 {
-    if (c >= ncol || k >= lw || k >= N) return make_float2(0.f, 0.f);
-    if (k == 0) return make_float2(src[c] * inv_sqrt_2pi, 0.f);
-    return make_float2(src[(2 * k - 1) * kFftJS + c] * half_inv_sqrt_pi,
-                       -src[(2 * k) * kFftJS + c] * half_inv_sqrt_pi);
-  };
-  // Pairs (k, N - k), k = 0..N/2; k = 0 pairs with the (zero) Nyquist term.
-  // A thread keeps one column (c = tid mod kFftJS) and takes
-  // k = tid / kFftJS + kRowsPerPass * it.  Z[k] overwrites the staged rows
-  // 2k and 2k + 1 and Z[N - k] the rows 2(N - k) and 2(N - k) + 1, so the
-  // items run in two halves (k < kSplit, then the rest), each loading all of
-  // its X before any of its Z is written: the first half's Z rows are ones
-  // that the second half no longer reads, except row 2 kSplit - 1 of
-  // Z[kSplit - 1], which is written after the second half's loads.  Half
-  // the X values are live at a time.
-  constexpr int kRowsPerPass = kFftThreads / kFftJS;
-  constexpr int kItems = (N / 2 + 1 + kRowsPerPass - 1) / kRowsPerPass;
-  constexpr int kItA = kItems / 2;
-  constexpr int kSplit = kItA * kRowsPerPass;
-  const int cz = tid % kFftJS, k0 = tid / kFftJS;
-  auto z_pair = [&](int k, float2 xk, float2 xn, bool write_k) {
-    const float2 xnc = cconj(xn), xkc = cconj(xk);
-    const float2 zk = cadd(cadd(xk, xnc), cmul_i<1>(cmul(twi[k], csub(xk, xnc))));
-    if (write_k) S[k * kFftJS + cz] = zk;
-    if (k > 0 && k < N / 2 + (N & 1)) {
-      const int kn = N - k;
-      S[kn * kFftJS + cz] =
-          cadd(cadd(xn, xkc), cmul_i<1>(cmul(twi[kn], csub(xn, xkc))));
-    }
-    return zk;
-  };
-  float2 held = make_float2(0.f, 0.f);  // Z[kSplit - 1], written last
-  bool hold = false;
-  if constexpr (kItA > 0) {
-    float2 xk[kItA], xn[kItA];
+  const float2 wc = wq ? ld_cols<false>(wq + col, cols) : make_float2(1.f, 1.f);
+  const float2 sc = pmul(wc, dup(half_inv_sqrt_pi));
+  // Items k = 0 .. N/2 - 1: the pair (k, N - k), and for k = 0 the two terms
+  // without a partner, Z[0] and Z[N/2].
+  constexpr int kRows = T / P;
+  constexpr int kAll = (N / 2 + kRows - 1) / kRows;
+  constexpr int kBatch = kAll < 8 ? kAll : 8;
+  const int k0 = tid / P;
 #pragma unroll
-    for (int it = 0; it < kItA; ++it) {
-      const int k = k0 + it * kRowsPerPass;
-      xk[it] = X(k, cz);
-      xn[it] = (k == 0) ? make_float2(0.f, 0.f) : X(N - k, cz);
-    }
-    __syncthreads();
+  for (int i0 = 0; i0 < kAll; i0 += kBatch) {
+    float2 ck[kBatch], sk[kBatch], cn[kBatch], sn[kBatch];
 #pragma unroll
-    for (int it = 0; it < kItA; ++it) {
-      const int k = k0 + it * kRowsPerPass;
-      const bool last_row = (k == kSplit - 1);
-      const float2 zk = z_pair(k, xk[it], xn[it], !last_row);
-      if (last_row) {
-        held = zk;
-        hold = true;
+    for (int i = 0; i < kBatch; ++i) {
+      const int k = k0 + (i0 + i) * kRows;
+      const int kn = k == 0 ? N / 2 : N - k;
+      const int nk = (k < N / 2 && k < lw) ? cols : 0;
+      const int nn = (k < N / 2 && kn < lw) ? cols : 0;
+      const float* fk = Fb + (size_t)(k == 0 ? 0 : 2 * k - 1) * J;
+      const float* fn = Fb + (size_t)(2 * kn - 1) * J;
+      ck[i] = ld_cols<kVec>(fk, nk);
+      sk[i] = ld_cols<kVec>(fk + J, k == 0 ? 0 : nk);
+      cn[i] = ld_cols<kVec>(fn, nn);
+      sn[i] = ld_cols<kVec>(fn + J, nn);
+    }
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      const int k = k0 + (i0 + i) * kRows;
+      if (k >= N / 2) continue;
+      if (k == 0) {
+        const float2 x0 = pmul(ck[i], pmul(wc, dup(inv_sqrt_2pi)));
+        st_cpair(S + p, {x0, x0});
+        const float2 two = padd(sc, sc);
+        st_cpair(S + (N / 2) * P + p, {pmul(cn[i], two), pmul(sn[i], two)});
+        continue;
       }
+      const float2 a = pmul(ck[i], sc), s = pmul(sk[i], sc);
+      const float2 c = pmul(cn[i], sc), d = pmul(sn[i], sc);
+      const float2 ar = padd(a, c), ai = psub(d, s);
+      const float2 br = psub(a, c), q = padd(s, d);  // B = br - i q
+      const float2 w = tw_i[k];
+      const float2 wr = dup(w.x), wi = dup(w.y);
+      const float2 tr = pfma(br, wr, pmul(q, wi));
+      const float2 ti = psub(pmul(br, wi), pmul(q, wr));
+      st_cpair(S + k * P + p, {psub(ar, ti), padd(ai, tr)});
+      st_cpair(S + (N - k) * P + p, {padd(ar, ti), psub(tr, ai)});
     }
-  }
-  {
-    constexpr int kItB = kItems - kItA;
-    float2 xk[kItB], xn[kItB];
-#pragma unroll
-    for (int it = 0; it < kItB; ++it) {
-      const int k = kSplit + k0 + it * kRowsPerPass;
-      if (k <= N / 2) {
-        xk[it] = X(k, cz);
-        xn[it] = (k == 0) ? make_float2(0.f, 0.f) : X(N - k, cz);
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int it = 0; it < kItB; ++it) {
-      const int k = kSplit + k0 + it * kRowsPerPass;
-      if (k <= N / 2) z_pair(k, xk[it], xn[it], true);
-    }
-    if (hold) S[(kSplit - 1) * kFftJS + cz] = held;
   }
   __syncthreads();
-  float* ob = out + (size_t)b * (2 * N) * J + j0;
-  auto first = [S](int n, int c) { return S[n * kFftJS + c]; };
-  // The last pass writes z back into S; then each thread copies its column
-  // (c = tid mod kFftJS, the same in every pass) out as rows 2n (Re z[n])
-  // and 2n + 1 (Im z[n]) with its weight read once.  Keeping the global
-  // stores out of the pass keeps its register count down.
-  auto last = [S](int n, int c, float2 v) { S[n * kFftJS + c] = v; };
-  fft_passes<N, 1, true, true>(S, twn, first, last);
-  __syncthreads();
-  const int cth = tid % kFftJS;
-  if (cth < ncol) {
-    const float sc = wq ? wq[j0 + cth] : 1.f;
-    float* oc = ob + cth;
-    for (int n = tid / kFftJS; n < N; n += kFftThreads / kFftJS) {
-      const float2 v = S[n * kFftJS + cth];
-      oc[2 * n * J] = v.x * sc;
-      oc[(2 * n + 1) * J] = v.y * sc;
-    }
-  }
+  float* ob = out + (size_t)b * (2 * N) * J + col;
+  auto first = [S, p](int n) { return ld_cpair(S + n * P + p); };
+  auto last = [ob, J, cols](int n, cpair v) {
+    float* o = ob + (size_t)(2 * n) * J;
+    st_cols<kVec>(o, v.re, cols);
+    st_cols<kVec>(o + J, v.im, cols);
+  };
+  fft_passes<N, 1, true, false>(S, tw, first, last);
 }
 
 // nodal[b][i][j] -> F[b][row][j] (times wq[j] when given: the forward SHT's
-// quadrature weights; without: the adjoint of the inverse transform).
-template <int N>
-__global__ void __launch_bounds__(kFftThreads)
+// quadrature weights; without: the adjoint of the inverse transform).  The
+// first pass reads the nodal rows, the last leaves Z in shared memory; with
+// s = (Z[k] + conj Z[N-k]) / 2, d = (Z[k] - conj Z[N-k]) / 2 and
+// U = -i conj(w_I^k) d, X[k] = s + U and X[N-k] = conj(s - U).
+template <int N, bool kVec>
+__global__ void __launch_bounds__(FftCfg<N>::threads, FftCfg<N>::ctas)
 rfft_forward_kernel(const float* __restrict__ x, float* __restrict__ F, int M,
                     int lw, int J, const float2* __restrict__ tw_n,
                     const float2* __restrict__ tw_i,
                     const float* __restrict__ wq) {
-  extern __shared__ float2 sm[];
-  float2* S = sm;
-  float2* twn = S + N * kFftJS;
-  float2* twi = twn + N;
-  const int tid = threadIdx.x;
+  constexpr int T = FftCfg<N>::threads, P = FftCfg<N>::pairs;
+  extern __shared__ float4 sm[];
+  float4* S = sm;
+  float4* tw = S + N * P;
+  const int tid = threadIdx.x, p = tid % P;
   const int b = blockIdx.y;
-  const int j0 = blockIdx.x * kFftJS;
-  const int ncol = min(kFftJS, J - j0);
-  for (int t = tid; t < N; t += kFftThreads) {
-    twn[t] = tw_n[t];
-    twi[t] = tw_i[t];
+  const int col = (blockIdx.x * P + p) * 2;
+  const int cols = max(0, min(2, J - col));
+  for (int t = tid; t < N; t += T) {
+    const float2 w = tw_n[t];
+    tw[t] = make_float4(w.x, w.x, -w.y, -w.y);
   }
-  const float* xb = x + (size_t)b * (2 * N) * J + j0;
-  // The nodal tile (2N rows of kFftJS floats) is staged by asynchronous
-  // copies; the first pass reads it in place.
-  stage_tile<2 * N>(xb, 2 * N, J, ncol, reinterpret_cast<float*>(S));
-  __syncthreads();
-  const float* Sf = reinterpret_cast<const float*>(S);
-  auto first = [Sf](int n, int c) {
-    return make_float2(Sf[2 * n * kFftJS + c], Sf[(2 * n + 1) * kFftJS + c]);
+  const float* xb = x + (size_t)b * (2 * N) * J + col;
+  auto first = [xb, J, cols](int n) -> cpair {
+    const float* g = xb + (size_t)(2 * n) * J;
+    return {ld_cols<kVec>(g, cols), ld_cols<kVec>(g + J, cols)};
   };
-  auto last = [S](int n, int c, float2 v) { S[n * kFftJS + c] = v; };
-  fft_passes<N, -1, true>(S, twn, first, last);
+  auto last = [S, p](int n, cpair v) { st_cpair(S + n * P + p, v); };
+  fft_passes<N, -1, false, true>(S, tw, first, last);
   __syncthreads();
-  float* Fb = F + (size_t)b * M * J + j0;
+  if (cols == 0) return;
+  float* Fb = F + (size_t)b * M * J + col;
   const float inv_sqrt_2pi = 0.3989422804014327f;
   const float inv_sqrt_pi = 0.5641895835477563f;
-  // X[k] and X[N - k] from the same two values of Z: with
-  // s = (Z[k] + conj Z[N-k]) / 2 and d = (Z[k] - conj Z[N-k]) / 2,
-  // X[k] = s + e^{-2 pi i k / I} (-i d), and X[N-k] likewise with Z[k] and
-  // Z[N-k] exchanged.  A thread keeps one column (c = tid mod kFftJS) and
-  // takes k = tid / kFftJS + kFftJS q for k <= N / 2.
-  const int c = tid % kFftJS;
-  if (c < ncol) {
-    const float w = wq ? wq[j0 + c] : 1.f;
-    const float a0 = w * inv_sqrt_2pi, a1 = w * inv_sqrt_pi;
-    float* Fc = Fb + c;
-    for (int k = tid / kFftJS; k <= N / 2; k += kFftThreads / kFftJS) {
-      const int kn = (N - k) & (N - 1);  // N - k; 0 for k = 0
-      const float2 zk = S[k * kFftJS + c];
-      const float2 zn = S[kn * kFftJS + c];
-      if (k < lw) {
-        const float2 zc = cconj(zn);
-        const float2 s2 = make_float2(0.5f * (zk.x + zc.x), 0.5f * (zk.y + zc.y));
-        const float2 d2 = make_float2(0.5f * (zk.x - zc.x), 0.5f * (zk.y - zc.y));
-        const float2 xk = cadd(s2, cmul(cconj(twi[k]), cmul_i<-1>(d2)));
-        if (k == 0) {
-          Fc[0] = xk.x * a0;
-        } else {
-          Fc[(2 * k - 1) * J] = xk.x * a1;
-          Fc[2 * k * J] = -xk.y * a1;
-        }
+  const float2 wc = wq ? ld_cols<false>(wq + col, cols) : make_float2(1.f, 1.f);
+  const float2 a0 = pmul(wc, dup(inv_sqrt_2pi)), a1 = pmul(wc, dup(inv_sqrt_pi));
+  const float2 ah = pmul(a1, dup(0.5f));
+  constexpr int kRows = T / P;
+#pragma unroll 4
+  for (int k = tid / P; k < N / 2; k += kRows) {
+    const int kn = k == 0 ? N / 2 : N - k;
+    const cpair zk = ld_cpair(S + k * P + p);
+    const cpair zn = ld_cpair(S + kn * P + p);
+    float* fk = Fb + (size_t)(k == 0 ? 0 : 2 * k - 1) * J;
+    float* fn = Fb + (size_t)(2 * kn - 1) * J;
+    if (k == 0) {
+      st_cols<kVec>(fk, pmul(padd(zk.re, zk.im), a0), cols);
+      if (kn < lw) {
+        st_cols<kVec>(fn, pmul(zn.re, a1), cols);
+        st_cols<kVec>(fn + J, pmul(zn.im, a1), cols);
       }
-      if (k > 0 && k < N / 2 && kn < lw) {
-        const float2 zc = cconj(zk);
-        const float2 s2 = make_float2(0.5f * (zn.x + zc.x), 0.5f * (zn.y + zc.y));
-        const float2 d2 = make_float2(0.5f * (zn.x - zc.x), 0.5f * (zn.y - zc.y));
-        const float2 xn = cadd(s2, cmul(cconj(twi[kn]), cmul_i<-1>(d2)));
-        Fc[(2 * kn - 1) * J] = xn.x * a1;
-        Fc[2 * kn * J] = -xn.y * a1;
-      }
+      continue;
+    }
+    const float2 w = tw_i[k];
+    const float2 wr = dup(w.x), wi = dup(w.y);
+    const float2 sr = padd(zk.re, zn.re), si = psub(zk.im, zn.im);  // 2 s
+    const float2 dr = psub(zk.re, zn.re), di = padd(zk.im, zn.im);  // 2 d
+    const float2 ur = psub(pmul(wr, di), pmul(wi, dr));
+    const float2 v = pfma(wi, di, pmul(wr, dr));  // -Im 2U
+    if (k < lw) {
+      st_cols<kVec>(fk, pmul(padd(sr, ur), ah), cols);
+      st_cols<kVec>(fk + J, pmul(psub(v, si), ah), cols);
+    }
+    if (kn < lw) {
+      st_cols<kVec>(fn, pmul(psub(sr, ur), ah), cols);
+      st_cols<kVec>(fn + J, pmul(padd(si, v), ah), cols);
     }
   }
 }
@@ -889,10 +936,11 @@ static int configure_rfft() {
   static PerDeviceOnce once;
   return once.run([] {
     const int smem = (int)fft_smem_bytes<N>();
-    DINO_CHECK_CUDA(cudaFuncSetAttribute(rfft_inverse_kernel<N>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    DINO_CHECK_CUDA(cudaFuncSetAttribute(rfft_forward_kernel<N>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    DINO_CHECK_CUDA(cudaFuncSetAttribute(rfft_inverse_kernel<N, true>, attr, smem));
+    DINO_CHECK_CUDA(cudaFuncSetAttribute(rfft_inverse_kernel<N, false>, attr, smem));
+    DINO_CHECK_CUDA(cudaFuncSetAttribute(rfft_forward_kernel<N, true>, attr, smem));
+    DINO_CHECK_CUDA(cudaFuncSetAttribute(rfft_forward_kernel<N, false>, attr, smem));
     return DINO_OK;
   });
 }
@@ -900,18 +948,18 @@ static int configure_rfft() {
 template <int N>
 static int launch_rfft(dino_plan* p, const float* in, float* out, int nf,
                        bool inverse, const float* wq, cudaStream_t st) {
+  constexpr int T = FftCfg<N>::threads;
   const size_t smem = fft_smem_bytes<N>();
   if (!p) return configure_rfft<N>();
   DINO_TRY(configure_rfft<N>());
-  dim3 grid(ceil_div(p->J, kFftJS), nf);
-  if (inverse) {
-    rfft_inverse_kernel<N><<<grid, kFftThreads, smem, st>>>(
-        in, out, p->M, p->lw, p->J, p->d_tw_n, p->d_tw_i, wq);
-    return check_launch("rfft_inverse");
-  }
-  rfft_forward_kernel<N><<<grid, kFftThreads, smem, st>>>(
-      in, out, p->M, p->lw, p->J, p->d_tw_n, p->d_tw_i, wq);
-  return check_launch("rfft_forward");
+  dim3 grid(ceil_div(p->J, 2 * FftCfg<N>::pairs), nf);
+  // Two columns per 8-byte access where every row starts 8-byte aligned.
+  const bool vec = p->J % 2 == 0 && (reinterpret_cast<uintptr_t>(in) & 7) == 0 &&
+                   (reinterpret_cast<uintptr_t>(out) & 7) == 0;
+  auto* kernel = inverse ? (vec ? rfft_inverse_kernel<N, true> : rfft_inverse_kernel<N, false>)
+                         : (vec ? rfft_forward_kernel<N, true> : rfft_forward_kernel<N, false>);
+  kernel<<<grid, T, smem, st>>>(in, out, p->M, p->lw, p->J, p->d_tw_n, p->d_tw_i, wq);
+  return check_launch(inverse ? "rfft_inverse" : "rfft_forward");
 }
 
 static int rfft_dispatch_n(int n, dino_plan* p, const float* in, float* out,
@@ -921,10 +969,17 @@ static int rfft_dispatch_n(int n, dino_plan* p, const float* in, float* out,
     case 8: return launch_rfft<8>(p, in, out, nf, inverse, wq, st);
     case 16: return launch_rfft<16>(p, in, out, nf, inverse, wq, st);
     case 32: return launch_rfft<32>(p, in, out, nf, inverse, wq, st);
+    case 48: return launch_rfft<48>(p, in, out, nf, inverse, wq, st);
     case 64: return launch_rfft<64>(p, in, out, nf, inverse, wq, st);
+    case 96: return launch_rfft<96>(p, in, out, nf, inverse, wq, st);
     case 128: return launch_rfft<128>(p, in, out, nf, inverse, wq, st);
+    case 160: return launch_rfft<160>(p, in, out, nf, inverse, wq, st);
+    case 180: return launch_rfft<180>(p, in, out, nf, inverse, wq, st);
     case 256: return launch_rfft<256>(p, in, out, nf, inverse, wq, st);
+    case 320: return launch_rfft<320>(p, in, out, nf, inverse, wq, st);
     case 512: return launch_rfft<512>(p, in, out, nf, inverse, wq, st);
+    case 640: return launch_rfft<640>(p, in, out, nf, inverse, wq, st);
+    case 1280: return launch_rfft<1280>(p, in, out, nf, inverse, wq, st);
   }
   set_error("internal: unsupported FFT length");
   return DINO_ERR_UNSUPPORTED;
@@ -936,7 +991,7 @@ static int rfft_dispatch(dino_plan* p, const float* in, float* out, int nf,
 }
 
 int sht_prepare(dino_plan* p) {
-  if (!p->fft_pow2) return DINO_OK;
+  if (!p->fft) return DINO_OK;
   return rfft_dispatch_n(p->N, nullptr, nullptr, nullptr, 0, true, nullptr, 0);
 }
 
@@ -944,7 +999,7 @@ int fourier_inverse(dino_plan* p, const float* F, float* nodal, int nf,
                     bool weighted_adjoint, cudaStream_t st) {
   NvtxRange range("inv_fourier");
   const float* wq = weighted_adjoint ? p->d_wq : nullptr;
-  if (p->fft_pow2) return rfft_dispatch(p, F, nodal, nf, true, wq, st);
+  if (p->fft) return rfft_dispatch(p, F, nodal, nf, true, wq, st);
   dim3 grid(ceil_div(p->J, 32), ceil_div(p->I, 8), nf);
   dft_inverse_kernel<<<grid, dim3(32, 8), 0, st>>>(F, nodal, p->M, p->I, p->J,
                                                     p->d_fbasis, wq);
@@ -955,7 +1010,7 @@ int fourier_forward(dino_plan* p, const float* nodal, float* F, int nf,
                     bool weighted, cudaStream_t st) {
   NvtxRange range("fwd_fourier");
   const float* wq = weighted ? p->d_wq : nullptr;
-  if (p->fft_pow2) return rfft_dispatch(p, nodal, F, nf, false, wq, st);
+  if (p->fft) return rfft_dispatch(p, nodal, F, nf, false, wq, st);
   dim3 grid(ceil_div(p->J, 32), ceil_div(p->M, 8), nf);
   dft_forward_kernel<<<grid, dim3(32, 8), 0, st>>>(nodal, F, p->M, p->I, p->J,
                                                     p->d_fbasis, wq);
