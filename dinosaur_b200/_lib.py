@@ -154,6 +154,7 @@ SIGNATURES = {
     'dino_swe_implicit': (ctypes.c_int, [_vp, _vp, _vp, _vp]),
     'dino_swe_implicit_inverse': (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_double,
                                                  _vp]),
+    'dino_swe_step': (ctypes.c_int, [_vp, _vp, ctypes.c_double, _DP, _i32, _vp]),
     'dino_pe_explicit_vjp': (ctypes.c_int, [_vp, _vp, _vp, _vp, _vp]),
     'dino_pe_implicit_vjp': (ctypes.c_int, [_vp, _vp, _vp, _vp]),
     'dino_pe_implicit_inverse_vjp': (ctypes.c_int, [_vp, _vp, _vp,

@@ -8,8 +8,14 @@
 //   -> inverse SHT -> nodal products (u (zeta + f), u phi, kinetic energy)
 //   -> forward SHT -> modal post-pass (div/curl, Laplacian, the layer
 //   pressure coupling through the density ratios, clip of the top l).
+// A filtered SIL3 step is three of them, the post-pass of each fused with the
+// stage that follows (the implicit part is elementwise in (layer, m, l)): 21
+// kernels, replayed from one CUDA graph, in place of about 150 launches of the
+// generic tableau loop over tensors, which the host could not issue as fast as
+// the GPU ran them.
 
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "dino_internal.cuh"
@@ -28,6 +34,20 @@ struct dino_swe {
   float* d_fwd_out = nullptr;
   float* d_work = nullptr;
   int work_fields = 0;
+  // SIL3 step (allocated by the first one): the state it advances, the two
+  // stage states, f0 and f1, the uploaded filters and the captured step.
+  float* d_y = nullptr;
+  float* d_Y[2] = {nullptr, nullptr};
+  float* d_f[2] = {nullptr, nullptr};
+  struct Filter {
+    std::vector<double> host;
+    float* dev;
+  };
+  std::vector<Filter> filters;
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  double graph_dt = 0;
+  const float* graph_filter = nullptr;
 };
 
 namespace dino {
@@ -111,26 +131,18 @@ struct SwePostArgs {
   float inv_radius;
 };
 
-// shallow_water.py:186-205.  p = D phi + orography (the layers' pressure
-// coupling); vorticity -div_cos_lat(b); divergence -lap(p + e) +
-// curl_cos_lat(b); potential -div_cos_lat(g); every tendency clipped.
-__global__ void swe_post_kernel(SwePostArgs a) {
+// The tendencies of one (member, layer, row, l) (shallow_water.py:186-205).
+// p = D phi + orography (the layers' pressure coupling); vorticity
+// -div_cos_lat(b); divergence -lap(p + e) + curl_cos_lat(b); potential
+// -div_cos_lat(g); every tendency clipped.
+__device__ __forceinline__ void swe_tendency(const SwePostArgs& a, int mb, int k, size_t idx,
+                                             float& fz, float& fd, float& fp) {
   const size_t ML = (size_t)a.M * a.L;
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= ML) return;
-  const int l = idx % a.L, row = idx / a.L;
-  const int k = blockIdx.y, mb = blockIdx.z, K = a.K;
+  const int l = idx % a.L, row = idx / a.L, K = a.K;
+  fz = fd = fp = 0.f;
+  if (l == a.L - 1) return;
   const size_t mK = (size_t)a.mem * K;
   const size_t plane = (size_t)mb * K + k;
-  float* out_z = a.tend + plane * ML;
-  float* out_d = a.tend + (mK + plane) * ML;
-  float* out_p = a.tend + (2 * mK + plane) * ML;
-  if (l == a.L - 1) {
-    out_z[idx] = 0.f;
-    out_d[idx] = 0.f;
-    out_p[idx] = 0.f;
-    return;
-  }
   const float* bu = a.fm + plane * ML;
   const float* bv = a.fm + (mK + plane) * ML;
   const float* gu = a.fm + (2 * mK + plane) * ML;
@@ -146,9 +158,87 @@ __global__ void swe_post_kernel(SwePostArgs a) {
                         dlat_at(bu, nullptr, row, l, a.L, a.lw, a.deriv, 2)) * ir;
   const float div_g = (d_dlon_at(gu, row, l, a.L) +
                        dlat_at(gv, nullptr, row, l, a.L, a.lw, a.deriv, 2)) * ir;
-  out_z[idx] = -div_b;
-  out_d[idx] = -a.lap[l] * (p + e[idx]) + curl_b;
-  out_p[idx] = -div_g;
+  fz = -div_b;
+  fd = -a.lap[l] * (p + e[idx]) + curl_b;
+  fp = -div_g;
+}
+
+__global__ void swe_post_kernel(SwePostArgs a) {
+  const size_t ML = (size_t)a.M * a.L;
+  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= ML) return;
+  const int k = blockIdx.y, mb = blockIdx.z;
+  const size_t mK = (size_t)a.mem * a.K;
+  const size_t plane = (size_t)mb * a.K + k;
+  float fz, fd, fp;
+  swe_tendency(a, mb, k, idx, fz, fd, fp);
+  a.tend[plane * ML + idx] = fz;
+  a.tend[(mK + plane) * ML + idx] = fd;
+  a.tend[(2 * mK + plane) * ML + idx] = fp;
+}
+
+// Stage kStage (1, 2, 3) of a filtered SIL3 step (time_integration.py:329-405)
+// from the transform outputs of its explicit evaluation at a.state (y0, Y1 or
+// Y2): the tendency f, the combination with y0, the earlier f_j and the
+// implicit terms (elementwise in (layer, m, l), so they are formed here from
+// the states themselves), the implicit inverse, and in the last stage the
+// final implicit term and the filter.  a.tend (stages 1, 2): where f is kept.
+struct SweStageArgs {
+  const float* y0;
+  const float* f0;
+  const float* f1;
+  float* out;
+  const float* phiref;
+  const float* filter;  // per l, or null (last stage)
+  float c0, c1, cf;     // coefficients of f0, f1 and f
+  float cg, eta;        // of the implicit terms, and of the implicit inverse
+};
+
+template <int kStage>
+__global__ void swe_stage_kernel(SwePostArgs a, SweStageArgs s) {
+  const size_t ML = (size_t)a.M * a.L;
+  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= ML) return;
+  const int l = idx % a.L, k = blockIdx.y, mb = blockIdx.z;
+  const size_t mK = (size_t)a.mem * a.K;
+  const size_t plane = (size_t)mb * a.K + k;
+  const size_t oz = plane * ML + idx, od = (mK + plane) * ML + idx,
+               op = (2 * mK + plane) * ML + idx;
+  float fz, fd, fp;
+  swe_tendency(a, mb, k, idx, fz, fd, fp);
+  if (kStage < 3) {
+    a.tend[oz] = fz;
+    a.tend[od] = fd;
+    a.tend[op] = fp;
+  }
+  const float lam = a.lap[l], ref = s.phiref[k];
+  const float y0d = s.y0[od], y0p = s.y0[op];
+  float z = s.y0[oz], d = y0d, p = y0p;
+  auto add = [&](float c, float vz, float vd, float vp) {
+    z = fmaf(c, vz, z);
+    d = fmaf(c, vd, d);
+    p = fmaf(c, vp, p);
+  };
+  if (kStage > 1) add(s.c0, s.f0[oz], s.f0[od], s.f0[op]);
+  if (kStage > 2) add(s.c1, s.f1[oz], s.f1[od], s.f1[op]);
+  add(s.cf, fz, fd, fp);
+  // g0 (and g2 at Y2 = a.state).
+  add(s.cg, 0.f, -lam * y0p, -ref * y0d);
+  if (kStage == 3) add(s.cg, 0.f, -lam * a.state[op], -ref * a.state[od]);
+  const float eta = s.eta;
+  const float inv = 1.f / (1.f - eta * eta * ref * lam);
+  const float sd = inv * (d - eta * lam * p);
+  const float sp = inv * (p - eta * ref * d);
+  if (kStage < 3) {
+    s.out[oz] = z;
+    s.out[od] = sd;
+    s.out[op] = sp;
+  } else {
+    const float w = s.filter ? s.filter[l] : 1.f;
+    s.out[oz] = z * w;
+    s.out[od] = fmaf(eta, -lam * sp, d) * w;
+    s.out[op] = fmaf(eta, -ref * sd, p) * w;
+  }
 }
 
 struct SweImplicitArgs {
@@ -204,6 +294,12 @@ void swe_free(dino_swe* s) {
   cudaFree(s->d_fwd_in);
   cudaFree(s->d_fwd_out);
   cudaFree(s->d_work);
+  if (s->exec) cudaGraphExecDestroy(s->exec);
+  if (s->graph) cudaGraphDestroy(s->graph);
+  cudaFree(s->d_y);
+  for (float* b : s->d_Y) cudaFree(b);
+  for (float* b : s->d_f) cudaFree(b);
+  for (auto& f : s->filters) cudaFree(f.dev);
   delete s;
 }
 
@@ -242,7 +338,8 @@ int swe_build(dino_swe* s, const dino_swe_desc* d) {
   return DINO_OK;
 }
 
-int swe_explicit_impl(dino_swe* s, const float* state, float* tend, cudaStream_t st) {
+// The explicit terms of `state` up to the forward transform (s->d_fwd_out).
+int swe_products(dino_swe* s, const float* state, cudaStream_t st) {
   dino_plan* p = s->plan;
   const int K = s->K, mem = s->mem;
   const int mK = mem * K;
@@ -261,15 +358,105 @@ int swe_explicit_impl(dino_swe* s, const float* state, float* tend, cudaStream_t
     swe_nodal_kernel<<<grid, 256, 0, st>>>(a);
     DINO_TRY(check_launch("swe_nodal"));
   }
-  DINO_TRY(sht_forward_to(p, s->d_fwd_in, s->d_fwd_out, 5 * mK, s->d_work,
-                          s->work_fields, st));
-  {
-    SwePostArgs a{s->d_fwd_out, state, tend, s->d_dens, s->d_orog, K, mem, s->M, s->L,
-                  p->lw, p->d_deriv, p->d_lap, (float)(1.0 / p->radius)};
-    dim3 grid(ceil_div((int)s->ML, 256), K, mem);
-    swe_post_kernel<<<grid, 256, 0, st>>>(a);
-    DINO_TRY(check_launch("swe_post"));
+  return sht_forward_to(p, s->d_fwd_in, s->d_fwd_out, 5 * mK, s->d_work, s->work_fields, st);
+}
+
+SwePostArgs post_args(dino_swe* s, const float* state, float* tend) {
+  return {s->d_fwd_out, state, tend, s->d_dens, s->d_orog, s->K, s->mem, s->M, s->L,
+          s->plan->lw, s->plan->d_deriv, s->plan->d_lap, (float)(1.0 / s->plan->radius)};
+}
+
+int swe_explicit_impl(dino_swe* s, const float* state, float* tend, cudaStream_t st) {
+  DINO_TRY(swe_products(s, state, st));
+  dim3 grid(ceil_div((int)s->ML, 256), s->K, s->mem);
+  swe_post_kernel<<<grid, 256, 0, st>>>(post_args(s, state, tend));
+  return check_launch("swe_post");
+}
+
+// One filtered SIL3 step of s->d_y in place.
+int swe_step_once(dino_swe* s, double dt, const float* filter, cudaStream_t st) {
+  dim3 grid(ceil_div((int)s->ML, 256), s->K, s->mem);
+  SweStageArgs a{};
+  a.y0 = s->d_y;
+  a.f0 = s->d_f[0];
+  a.f1 = s->d_f[1];
+  a.phiref = s->d_phiref;
+  DINO_TRY(swe_products(s, s->d_y, st));
+  a.out = s->d_Y[0];
+  a.cf = (float)(dt / 3);
+  a.cg = a.eta = (float)(dt / 6);
+  swe_stage_kernel<1><<<grid, 256, 0, st>>>(post_args(s, s->d_y, s->d_f[0]), a);
+  DINO_TRY(check_launch("swe_stage"));
+  DINO_TRY(swe_products(s, s->d_Y[0], st));
+  a.out = s->d_Y[1];
+  a.c0 = (float)(dt / 6);
+  a.cf = (float)(dt / 2);
+  a.cg = a.eta = (float)(dt / 3);
+  swe_stage_kernel<2><<<grid, 256, 0, st>>>(post_args(s, s->d_Y[0], s->d_f[1]), a);
+  DINO_TRY(check_launch("swe_stage"));
+  DINO_TRY(swe_products(s, s->d_Y[1], st));
+  a.out = s->d_y;
+  a.filter = filter;
+  a.c0 = (float)(dt / 2);
+  a.c1 = (float)(-dt / 2);
+  a.cf = (float)dt;
+  a.cg = (float)(3 * dt / 8);
+  a.eta = (float)(dt / 4);
+  swe_stage_kernel<3><<<grid, 256, 0, st>>>(post_args(s, s->d_Y[1], nullptr), a);
+  return check_launch("swe_stage");
+}
+
+int swe_step_impl(dino_swe* s, float* state, double dt, const double* host_filter, int n_steps,
+                  cudaStream_t st) {
+  const size_t bytes = sizeof(float) * 3 * (size_t)s->mem * s->K * s->ML;
+  for (float** b : {&s->d_y, &s->d_Y[0], &s->d_Y[1], &s->d_f[0], &s->d_f[1]})
+    if (!*b) DINO_CHECK_CUDA(cudaMalloc(b, bytes));
+  const float* filter = nullptr;
+  if (host_filter) {
+    for (auto& f : s->filters)
+      if (std::memcmp(f.host.data(), host_filter, sizeof(double) * s->L) == 0) filter = f.dev;
+    if (!filter) {
+      std::vector<float> w(s->L);
+      for (int l = 0; l < s->L; ++l) w[l] = (float)host_filter[l];
+      float* dev = nullptr;
+      DINO_TRY(upload(&dev, w));
+      s->filters.push_back({std::vector<double>(host_filter, host_filter + s->L), dev});
+      filter = dev;
+    }
   }
+  if (!(s->exec && s->graph_dt == dt && s->graph_filter == filter)) {
+    if (s->exec) cudaGraphExecDestroy(s->exec);
+    if (s->graph) cudaGraphDestroy(s->graph);
+    s->exec = nullptr;
+    s->graph = nullptr;
+    DINO_TRY(sht_prepare(s->plan));
+    // Captured on a private stream, so that the caller's stream (possibly the
+    // legacy default one) never enters capture mode.
+    cudaStream_t cap;
+    DINO_CHECK_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
+    cudaError_t ce = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
+    int rc = DINO_OK;
+    cudaGraph_t graph = nullptr;
+    if (ce == cudaSuccess) {
+      rc = swe_step_once(s, dt, filter, cap);
+      ce = cudaStreamEndCapture(cap, &graph);
+    }
+    cudaStreamDestroy(cap);
+    if (rc != DINO_OK || ce != cudaSuccess) {
+      if (graph) cudaGraphDestroy(graph);
+      if (rc != DINO_OK) return rc;
+      DINO_CHECK_CUDA(ce);
+    }
+    s->graph = graph;
+    DINO_CHECK_CUDA(cudaGraphInstantiate(&s->exec, graph, 0));
+    s->graph_dt = dt;
+    s->graph_filter = filter;
+  }
+  // The captured step works on the object's own buffer, so one capture serves
+  // every caller's state; two copies a call.
+  DINO_CHECK_CUDA(cudaMemcpyAsync(s->d_y, state, bytes, cudaMemcpyDeviceToDevice, st));
+  for (int i = 0; i < n_steps; ++i) DINO_CHECK_CUDA(cudaGraphLaunch(s->exec, st));
+  DINO_CHECK_CUDA(cudaMemcpyAsync(state, s->d_y, bytes, cudaMemcpyDeviceToDevice, st));
   return DINO_OK;
 }
 
@@ -343,6 +530,14 @@ int dino_swe_implicit_inverse(dino_swe* s, const float* state, float* out, doubl
   DINO_REQUIRE(s && state && out, DINO_ERR_ARG, "dino_swe_implicit_inverse: null argument");
   DINO_REQUIRE(std::isfinite(eta), DINO_ERR_ARG, "step_size must be finite");
   return swe_implicit_impl(s, state, out, 1, eta, (cudaStream_t)stream);
+}
+
+int dino_swe_step(dino_swe* s, float* state, double dt, const double* host_filter,
+                  int32_t n_steps, void* stream) {
+  DINO_REQUIRE(s && state, DINO_ERR_ARG, "dino_swe_step: null argument");
+  DINO_REQUIRE(n_steps >= 0, DINO_ERR_ARG, "n_steps must be >= 0");
+  if (n_steps == 0) return DINO_OK;
+  return swe_step_impl(s, state, dt, host_filter, n_steps, (cudaStream_t)stream);
 }
 
 }  // extern "C"

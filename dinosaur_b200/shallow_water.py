@@ -4,8 +4,8 @@
 ``ImplicitExplicitODE`` methods; each call runs the CUDA kernels of
 ``csrc/swe.cu`` through the C ABI on a packed
 [vorticity][divergence][potential] buffer.  The steppers of
-``dinosaur_b200.time_integration`` (``imex_rk_sil3``, ``step_with_filters``,
-``repeated``) apply unchanged.
+``dinosaur_b200.time_integration`` apply unchanged; ``imex_rk_sil3`` with
+spectral filters runs as one fused CUDA step (``dino_swe_step``).
 """
 
 from __future__ import annotations
@@ -144,6 +144,15 @@ class _Engine:
                name)
     return out
 
+  def step_(self, buf, dt, filt, n_steps):
+    """Advances the packed buffer in place by n filtered SIL3 steps."""
+    if filt is not None:
+      filt = np.ascontiguousarray(filt, np.float64)
+    _lib.check(_lib.lib().dino_swe_step(
+        self.handle, sh.ptr(buf), float(dt), None if filt is None else _lib.dptr(filt),
+        int(n_steps), sh.stream_handle()), 'dino_swe_step')
+    return buf
+
 
 @dataclasses.dataclass(eq=False)
 class ShallowWaterEquations(time_integration.ImplicitExplicitODE):
@@ -186,6 +195,22 @@ class ShallowWaterEquations(time_integration.ImplicitExplicitODE):
       eng = _Engine(self, members)
       self._engines[members] = eng
     return eng
+
+  def _fused_engine(self, state: State):
+    """The engine of `state` if the fused step takes it: Real-layout float32
+    CUDA tensors of one device without gradients, outside stream capture (the
+    generic stepper takes everything else)."""
+    leaves = (state.vorticity, state.divergence, state.potential)
+    plan = self.coords.horizontal.plan
+    if not all(isinstance(x, torch.Tensor) and x.is_cuda and x.dtype == torch.float32
+               and x.device.index == plan.device
+               and x.shape == state.vorticity.shape for x in leaves):
+      return None
+    if torch.is_grad_enabled() and any(x.requires_grad for x in leaves):
+      return None
+    if sh.is_fast_layout(self.coords.horizontal) or torch.cuda.is_current_stream_capturing():
+      return None
+    return self._engine(state)
 
   def explicit_terms(self, state: State) -> State:
     """shallow_water.py:158-205."""

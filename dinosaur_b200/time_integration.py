@@ -187,6 +187,39 @@ class FusedSIL3Step:
 
 
 @dataclasses.dataclass
+class FusedShallowWaterStep:
+  """One or more filtered SIL3 steps of the shallow-water equations.
+
+  Calling it is ``repeated(step_with_filters(imex_rk_sil3(eq, dt), filters),
+  n_steps)`` of the reference: on float32 CUDA states one fused CUDA step
+  (``dino_swe_step``), on any other state the generic tableau loop.
+  """
+
+  equation: Any
+  dt: float
+  filters: tuple = ()
+  n_steps: int = 1
+
+  def __call__(self, state):
+    eq = self.equation
+    eng = eq._fused_engine(state)  # pylint: disable=protected-access
+    if eng is not None:
+      scaling = None
+      for f in self.filters:
+        s = np.asarray(f.scaling, np.float64)
+        scaling = s if scaling is None else scaling * s
+      buf = eng.pack(state)  # a fresh buffer: the input state is not modified
+      return eng.unpack(eng.step_(buf, self.dt, scaling, self.n_steps), state)
+    step = imex_runge_kutta(SIL3_TABLEAU, eq, self.dt)
+    for _ in range(self.n_steps):
+      nxt = step(state)
+      for f in self.filters:
+        nxt = f(state, nxt)
+      state = nxt
+    return state
+
+
+@dataclasses.dataclass
 class TimeReversedImExODE(ImplicitExplicitODE):
   """An ImplicitExplicitODE reversed in time (time_integration.py:117-138):
   dx/dt = -explicit_terms(x) - implicit_terms(x)."""
@@ -216,8 +249,12 @@ def imex_rk_sil3(equation, time_step: float):
   is the same step with -dt (negated explicit and implicit terms, implicit
   inverse at -eta)."""
   from dinosaur_b200 import primitive_equations as pe  # pylint: disable=g-import-not-at-top
+  from dinosaur_b200 import shallow_water  # pylint: disable=g-import-not-at-top
   if isinstance(equation, pe.PrimitiveEquationsSigma):
     return FusedSIL3Step(equation, float(time_step))
+  if (type(equation) is shallow_water.ShallowWaterEquations  # pylint: disable=unidiomatic-typecheck
+      and isinstance(time_step, (int, float))):
+    return FusedShallowWaterStep(equation, float(time_step))
   if (isinstance(equation, TimeReversedImExODE) and
       isinstance(equation.forward_eq, pe.PrimitiveEquationsSigma)):
     return FusedSIL3Step(equation.forward_eq, -float(time_step))
@@ -280,6 +317,10 @@ def step_with_filters(step_fn, filters: Sequence[Callable]):
       s = np.asarray(f.scaling, np.float64)
       scaling = s if scaling is None else scaling * s
     return dataclasses.replace(step_fn, filter_scaling=scaling)
+  if (isinstance(step_fn, FusedShallowWaterStep) and step_fn.n_steps == 1 and all(
+      isinstance(f, SpectralStepFilter) and np.shape(f.scaling) ==
+      (step_fn.equation.coords.horizontal.total_wavenumbers,) for f in filters)):
+    return dataclasses.replace(step_fn, filters=step_fn.filters + tuple(filters))
 
   def _step_fn(u):
     u_next = step_fn(u)
@@ -295,7 +336,7 @@ def repeated(fn, steps: int, scan_fn=None):
   del scan_fn
   if steps == 1:
     return fn
-  if isinstance(fn, FusedSIL3Step):
+  if isinstance(fn, (FusedSIL3Step, FusedShallowWaterStep)):
     return dataclasses.replace(fn, n_steps=fn.n_steps * steps)
 
   def f_repeated(x):

@@ -310,6 +310,14 @@ DINO_API int dino_swe_implicit(dino_swe* swe, const float* d_state,
  * allowed. */
 DINO_API int dino_swe_implicit_inverse(dino_swe* swe, const float* d_state,
                                        float* d_out, double eta, void* stream);
+/* Advances d_state in place by n_steps of imex_rk_sil3 with time step dt
+ * (time_integration.py:375-405), each followed by multiplication with the
+ * per-l filter scaling (host array of length L; NULL = none), from one
+ * captured CUDA graph per (dt, filter).  The first call allocates the step's
+ * work buffers; calls on one object must not overlap in time. */
+DINO_API int dino_swe_step(dino_swe* swe, float* d_state, double dt,
+                           const double* host_filter, int32_t n_steps,
+                           void* stream);
 
 /* ---- Reverse mode (vector-Jacobian products) ----------------------------
  * The reference differentiates its step with jax.vjp / jax.grad through the

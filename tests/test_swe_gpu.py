@@ -130,3 +130,53 @@ def test_reference_steady_geostrophic_flow(params):
     mean = np.mean(w * pot / np.sum(w), axis=(-1, -2))
     assert np.all(np.abs(mean) < 1e-8), mean
     assert np.sqrt(np.square(pot - init).sum()) / init_l2 < params['tol']
+
+
+@pytest.mark.parametrize('layers,members,wavenumbers', [(1, 1, 5), (3, 1, 21), (2, 3, 12)])
+def test_fused_step_matches_generic_stepper(layers, members, wavenumbers):
+  # The fused CUDA step against the tableau loop over the same kernels' terms:
+  # both FP32, so they differ by the rounding of a few sums per stage (bound:
+  # 16 roundings of 6e-8 relative to each field's maximum, three steps).
+  grid = sh.Grid.with_wavenumbers(wavenumbers)
+  coords = coordinate_systems.CoordinateSystem(
+      grid, layer_coordinates.LayerCoordinates(layers))
+  rng = np.random.default_rng(3)
+  shape = (members, layers) if members > 1 else (layers,)
+  _, l = np.meshgrid(*grid.modal_axes, indexing='ij')
+  field = lambda a: torch.as_tensor(
+      a * rng.standard_normal(shape + l.shape) * grid.mask / (l + 1.0), device='cuda',
+      dtype=torch.float32)
+  state = sw.State(field(0.05), field(0.005), field(0.005))
+  orography = rng.standard_normal(l.shape) * grid.mask * 1e-3
+  eq = sw.ShallowWaterEquations(coords, units.SimUnits(), orography,
+                                np.linspace(0.04, 0.06, layers),
+                                densities=np.linspace(1.0, 1.5, layers))
+  dt = 0.05
+  filt = ti.exponential_step_filter(grid, dt)
+  fused = ti.repeated(ti.step_with_filters(ti.imex_rk_sil3(eq, dt), [filt]), 3)
+  assert isinstance(fused, ti.FusedShallowWaterStep)
+  generic = ti.repeated(ti.step_with_filters(
+      ti.imex_runge_kutta(ti.SIL3_TABLEAU, eq, dt), [filt]), 3)
+  before = state.vorticity.clone()
+  got, want = fused(state), generic(state)
+  assert torch.equal(state.vorticity, before)
+  assert_close(got, {k: getattr(want, k).double().cpu().numpy() for k in KEYS}, 1e-6)
+  # Another time step, no filter, and the first again: one capture per case.
+  other = ti.imex_rk_sil3(eq, 2 * dt)(state)
+  assert_close(other, {k: v.double().cpu().numpy() for k, v in vars(
+      ti.imex_runge_kutta(ti.SIL3_TABLEAU, eq, 2 * dt)(state)).items()}, 1e-6)
+  assert torch.equal(fused(state).potential, got.potential)
+
+
+def test_fused_step_leaves_other_states_to_the_generic_stepper():
+  _, _, grid, eq, _, st = case()
+  step = ti.imex_rk_sil3(eq, 0.05)
+  s = to_state(st)
+  assert eq._fused_engine(s) is not None
+  s64 = sw.State(s.vorticity.double(), s.divergence.double(), s.potential.double())
+  assert eq._fused_engine(s64) is None
+  assert step(s64).vorticity.dtype == torch.float64
+  leaf = s.vorticity.clone().requires_grad_(True)
+  assert eq._fused_engine(sw.State(leaf, s.divergence, s.potential)) is None
+  with pytest.raises(ValueError):
+    step(sw.State(s.vorticity[:, :-1], s.divergence[:, :-1], s.potential[:, :-1]))
