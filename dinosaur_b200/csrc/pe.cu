@@ -300,16 +300,16 @@ __device__ __forceinline__ void st_vec(float* p, const float (&x)[V]) {
 
 // One thread per (V adjacent columns, chunk of levels): blockDim =
 // (kNodalCols, C), chunk c holding levels [c K / C, (c + 1) K / C).  The
-// column totals and the prefix sums that sigma-dot needs come from partial
-// sums exchanged through shared memory, so a thread walks K / C levels.  The
-// partial sums are always those of the kNodalMaxChunks parts [s K / 4,
-// (s + 1) K / 4), of which a chunk holds 4 / C: every chunk count adds in the
-// same order and gives the same bits.  A part's running sums are its partial
-// sum formed in the same order, so the sigma-dot of a half level shared by two
-// parts is the same in both.  V columns share each address computation and level coefficient (the
+// column totals and the prefix sums that sigma-dot needs come from per-chunk
+// partial sums exchanged through shared memory, so a thread walks K / C
+// levels.  A chunk's running sums are its partial sum formed in the same
+// order, so the sigma-dot of a half level shared by two chunks is the same in
+// both.  V columns share each address computation and level coefficient (the
 // latitude count J is a multiple of V, so they lie on one meridian).
 // kTracers = false compiles out the tracer windows (dry states).
-constexpr int kNodalCols = 32, kNodalMaxChunks = 4;
+// Every field of the next level is loaded while a level is computed (moist
+// TL255 / 32 x 4: 570 -> 541 us a launch; T21 / 12: 10.0 -> 9.3 us).
+constexpr int kNodalCols = 32, kNodalMaxChunks = 2;
 
 template <bool kTracers, int V>
 __global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
@@ -329,9 +329,7 @@ __global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
   const unsigned col = (blockIdx.x * kNodalCols + tx) * V;
   const bool active = col < IJ;
   const int mb = blockIdx.y;
-  constexpr int S = kNodalMaxChunks;  // parts of the column
-  const int s0 = c * S / C, s1 = (c + 1) * S / C;
-  const int k0 = (s0 * K) / S;
+  const int k0 = (c * K) / C, k1 = ((c + 1) * K) / C;
   const int nT = kTracers ? a.nT : 0;
   const int hum = kTracers ? a.hum : -1;
   const int j = active ? (int)(col % (unsigned)a.J) : 0;
@@ -353,20 +351,17 @@ __global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
   const float rv1 = a.Rv_over_R - 1.f;
   float gx[V], gy[V];
 
-  // Pass 1: the chunk's parts' shares of the column totals of u.grad(ln ps) and of
+  // Pass 1: this chunk's share of the column totals of u.grad(ln ps) and of
   // (div + u.grad ln ps), both weighted by the layer thickness
   // (cumulative_sigma_integral, last level), and (moist) of the geopotential
   // suffix sum of the virtual-temperature difference.
+  float pe_[V], pf_[V], pg_[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) pe_[i] = pf_[i] = pg_[i] = 0.f;
   if (active) {
     ld_vec(gx, a.nod + ((size_t)a.p_gx + mb) * IJ + col);
     ld_vec(gy, a.nod + ((size_t)a.p_gy + mb) * IJ + col);
-  }
-  for (int s = s0; s < s1; ++s) {
-    const int ka = (s * K) / S, kb = active ? ((s + 1) * K) / S : 0;
-    float pe_[V], pf_[V], pg_[V];
-#pragma unroll
-    for (int i = 0; i < V; ++i) pe_[i] = pf_[i] = pg_[i] = 0.f;
-    for (int k = ka; k < kb; ++k) {
+    for (int k = k0; k < k1; ++k) {
       const unsigned o = (unsigned)k * IJ;
       const float ds = s_lev[4 * k].x;
       float u[V], v[V], d[V];
@@ -381,7 +376,7 @@ __global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
       }
     }
     if (hum >= 0) {
-      for (int k = max(ka, 1); k < kb; ++k) {
+      for (int k = max(k0, 1); k < k1; ++k) {
         const unsigned o = (unsigned)k * IJ;
         const float4 c1 = s_lev[4 * k + 1];
         const float tr = s_lev[4 * k].w;
@@ -392,12 +387,12 @@ __global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
         for (int i = 0; i < V; ++i) pg_[i] += (c1.z + c1.w) * (h[i] * (T[i] + tr) * rv1);
       }
     }
+  }
 #pragma unroll
-    for (int i = 0; i < V; ++i) {
-      s_e[s][tx * V + i] = pe_[i];
-      s_f[s][tx * V + i] = pf_[i];
-      if (kTracers) s_g[s][tx * V + i] = pg_[i];
-    }
+  for (int i = 0; i < V; ++i) {
+    s_e[c][tx * V + i] = pe_[i];
+    s_f[c][tx * V + i] = pf_[i];
+    if (kTracers) s_g[c][tx * V + i] = pg_[i];
   }
   __syncthreads();
   if (!active) return;
@@ -405,14 +400,13 @@ __global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
 #pragma unroll
   for (int i = 0; i < V; ++i) {
     Fe[i] = Ff[i] = pre_e[i] = pre_f[i] = 0.f;
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-      if (s == s0) {
+    for (int cc = 0; cc < C; ++cc) {
+      if (cc == c) {
         pre_e[i] = Fe[i];
         pre_f[i] = Ff[i];
       }
-      Fe[i] += s_e[s][tx * V + i];
-      Ff[i] += s_f[s][tx * V + i];
+      Fe[i] += s_e[cc][tx * V + i];
+      Ff[i] += s_f[cc][tx * V + i];
     }
   }
 
@@ -420,29 +414,27 @@ __global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
   // G[k][h] = R alpha_k (h = k), R (alpha_h + alpha_{h-1}) (h > k): a suffix
   // sum evaluated bottom-up (get_geopotential_weights_sigma, :306-338).
   if (hum >= 0) {
+    float suffix[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      suffix[i] = 0.f;
+      for (int cc = C - 1; cc > c; --cc) suffix[i] += s_g[cc][tx * V + i];
+    }
     float* Ogh = out(a.o_gh);
-    for (int s = s1 - 1; s >= s0; --s) {
-      float suffix[V];
+    for (int k = k1 - 1; k >= k0; --k) {
+      const unsigned o = (unsigned)k * IJ;
+      const float4 c1 = s_lev[4 * k + 1];
+      const float tr = s_lev[4 * k].w;
+      float h[V], T[V], g[V];
+      ld_vec(h, Ph + o);
+      ld_vec(T, PT + o);
 #pragma unroll
       for (int i = 0; i < V; ++i) {
-        suffix[i] = 0.f;
-        for (int ss = S - 1; ss > s; --ss) suffix[i] += s_g[ss][tx * V + i];
+        const float td = h[i] * (T[i] + tr) * rv1;
+        g[i] = a.R * (c1.z * td + suffix[i]);
+        suffix[i] += (c1.z + c1.w) * td;
       }
-      for (int k = ((s + 1) * K) / S - 1; k >= (s * K) / S; --k) {
-        const unsigned o = (unsigned)k * IJ;
-        const float4 c1 = s_lev[4 * k + 1];
-        const float tr = s_lev[4 * k].w;
-        float h[V], T[V], g[V];
-        ld_vec(h, Ph + o);
-        ld_vec(T, PT + o);
-#pragma unroll
-        for (int i = 0; i < V; ++i) {
-          const float td = h[i] * (T[i] + tr) * rv1;
-          g[i] = a.R * (c1.z * td + suffix[i]);
-          suffix[i] += (c1.z + c1.w) * td;
-        }
-        st_vec(Ogh + o, g);
-      }
+      st_vec(Ogh + o, g);
     }
   }
 
@@ -511,17 +503,10 @@ __global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
     }
   }
 
-  for (int k = k0, s = s0, kn = ((s0 + 1) * K) / S; k < (s1 * K) / S; ++k) {
-    while (k == kn) {  // the next part begins
-#pragma unroll
-      for (int i = 0; i < V; ++i) {
-        pre_e[i] += s_e[s][tx * V + i];
-        pre_f[i] += s_f[s][tx * V + i];
-        loc_e[i] = loc_f[i] = 0.f;
-      }
-      ++s;
-      kn = ((s + 1) * K) / S;
-    }
+  float zeta_n[V], div_n[V];
+  ld_vec(zeta_n, Pz + o0);
+  ld_vec(div_n, Pd + o0);
+  for (int k = k0; k < k1; ++k) {
     const unsigned o = (unsigned)k * IJ;
     const unsigned on = (k + 1 < K) ? o + IJ : o;
     const float4 c0 = s_lev[4 * k], c1 = s_lev[4 * k + 1];
@@ -532,8 +517,13 @@ __global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
     ld_vec(u_n, Pu + on);
     ld_vec(v_n, Pv + on);
     ld_vec(T_n, PT + on);
-    ld_vec(zeta, Pz + o);
-    ld_vec(div, Pd + o);
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      zeta[i] = zeta_n[i];
+      div[i] = div_n[i];
+    }
+    ld_vec(zeta_n, Pz + on);
+    ld_vec(div_n, Pd + on);
     float q_n[kTracers ? kMaxTracers : 1][V];
     if (kTracers) {
 #pragma unroll
@@ -2187,14 +2177,13 @@ static int pe_nodal_inputs(dino_pe* pe, const float* state, cudaStream_t st) {
   return DINO_OK;
 }
 
-// Level chunks per column for pe_nodal_kernel: the fewest (1, 2 or 4) that
-// give about two waves of 16 warps per SM, keeping four or more levels a chunk.
-static int nodal_chunks(const dino_pe* pe, int V) {
-  const int64_t warps = (int64_t)ceil_div((int)(pe->IJ / V), kNodalCols) * pe->mem;
-  int C = 1;
-  while (2 * C <= kNodalMaxChunks && warps * C < 16LL * pe->sms && pe->K >= 8 * C) C *= 2;
-  return C;
-}
+// Level chunks per column for pe_nodal_kernel: two from eight levels on.  The
+// count depends on the levels alone, so that a state's sums are formed in the
+// same order, and its tendencies have the same bits, in any batch.  Measured
+// with one, two and four chunks (us a launch): T21 / 12 14.0, 9.3, 7.9; T42 / 24
+// x 16 37.2, 37.7, 43.4; TL255 / 32 45.0, 45.2, 48.5; TL95 / 19 moist x 3 38.7,
+// 40.9, 39.6; TL255 / 32 moist x 4 547, 541, 561.
+static int nodal_chunks(const dino_pe* pe) { return pe->K >= 8 ? kNodalMaxChunks : 1; }
 
 // Adjacent columns per thread for pe_nodal_kernel: two for dry states where
 // the latitude count is even (122 registers; four need 188 and run slower),
@@ -2276,7 +2265,7 @@ static int launch_nodal(dino_pe* pe, const float* state, cudaStream_t st) {
   const NodalArgs a = make_nodal_args(pe);
   const int V = nodal_vec(pe);
   const dim3 grid(ceil_div((int)(pe->IJ / V), kNodalCols), pe->mem);
-  const dim3 block(kNodalCols, nodal_chunks(pe, V));
+  const dim3 block(kNodalCols, nodal_chunks(pe));
   const size_t smem = nodal_smem(pe->K);
   if (pe->nT > 0)
     pe_nodal_kernel<true, 1><<<grid, block, smem, st>>>(a);

@@ -225,9 +225,8 @@ def test_level_chunks_agree_across_batch_sizes():
 
 @pytest.mark.parametrize('layers,moist', [(2, False), (9, False), (19, True), (24, False)])
 def test_level_chunks_give_the_same_bits(layers, moist):
-  # The column sums are added in the same four parts whatever the chunk count
-  # (one, two or four chunks for these sizes), so batch sizes agree exactly in
-  # the temperature tendency of every member.
+  # The chunk count (one below eight levels, else two) does not depend on the
+  # batch, so every member's tendencies have the bits of the state alone.
   kw = dict(tracers=_tracers, humidity='specific_humidity') if moist else {}
   og, oeq, st, g, eq = make('T42', layers=layers, **kw)
   s1 = to_state(st)
