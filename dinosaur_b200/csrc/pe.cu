@@ -92,13 +92,14 @@ struct dino_pe {
   float* d_work = nullptr;
   int work_fields = 0;
   float* d_f[3] = {nullptr, nullptr, nullptr};
-  float* d_g[2] = {nullptr, nullptr};
   float* d_Y = nullptr;
-  float* d_ystar = nullptr;  // Y* of the current stage (implicit planes)
-  // l-major operands of the per-l implicit products: [L][2n][Cp].
+  // l-major operands of the per-l implicit products, [L][rows][Cp]: the input
+  // (Y* of a stage, or gathered planes; up to 2n rows), the output (up to 2n
+  // rows) and the implicit terms of a step's first state (n rows).
   int Cp = 0;
   float* d_lm_in = nullptr;
   float* d_lm_out = nullptr;
+  float* d_lm_g0 = nullptr;
   // Adjoint work (allocated by the first VJP call).
   float* d_xbar_n = nullptr;  // nodal cotangents, n_inv planes
   float* d_xbar_m = nullptr;  // their modal adjoint, n_inv planes
@@ -160,96 +161,133 @@ struct PrepArgs {
   float inv_radius;
 };
 
-// The modal-point geometry of (row, l), loaded once and reused for every
-// level: the d/dlon partner row and factor, and the cos_lat_d_dlat (tab 0) or
-// sec_lat_d_dlat_cos2 (tab 2) recurrence coefficients at l + 1 and l - 1
-// (optionally times a per-l scaling s, folded in).
-struct ModalNbr {
-  int row, l, L;
-  int dl_row;
-  float dl_fac;
-  float a1, b1;  // coefficients of x[l + 1] and x[l - 1] (0 when out of range)
+// The adjoint passes: threads cover (row, l) with l fastest; each walks `ppt`
+// of the (member, level) planes, reusing its operator coefficients.
+constexpr int kModalTX = 32, kModalTY = 8;
 
-  __device__ ModalNbr(int row_, int l_, int L_, int lw, const float* deriv, int tab,
-                      const float* s)
-      : row(row_), l(l_), L(L_) {
+// The forward passes (pe_prep_kernel, pe_post_kernel): a CTA of 32 x 8 threads
+// covers a tile of 32 rows x 32 l, four rows a thread, and walks `ppt` planes.
+constexpr int kTile = 32;
+constexpr int kTileRows = kTile / kModalTY;  // rows per thread
+
+// Planes per CTA of a modal pass with `tiles` (row, l) tiles: a CTA loads its
+// operator coefficients once for all of them, but small grids need the planes
+// spread to fill the chip (T21 / 12 levels, 2 tiles: eight planes a CTA left 4
+// CTAs and 19.6 us for the post-pass).  Eight where that still gives eight
+// CTAs per SM.
+static int planes_per_cta(int tiles, int planes, int sms) {
+  int ppt = 8;
+  while (ppt > 1 && (int64_t)tiles * ceil_div(planes, ppt) < 8LL * sms) ppt /= 2;
+  return ppt;
+}
+
+// Tile (row0, l0) holds only entries l < m, the structural zeros below the
+// triangular truncation: transforms neither read nor fill them.
+__device__ __forceinline__ bool below_triangle(int row0, int l0) {
+  return l0 + kTile - 1 < ((row0 + 1) >> 1);
+}
+
+// A modal plane x around (row, l): its d/dlon partner row and l + 1, l - 1.
+struct Nbr3 {
+  float p, up, dn;
+};
+
+// Indices and coefficients of one (row, l) for all planes: x_p times dlon,
+// x_{l+1} times a1 and x_{l-1} times b1 (0 where out of range, and then the
+// load is of the entry itself).
+struct ModalPoint {
+  unsigned idx, ip, iu, id;
+  float dlon, a1, b1;
+
+  __device__ __forceinline__ ModalPoint(int row, int l, int L, int lw, const float* deriv,
+                                        int tab) {
     const int m = (row + 1) >> 1;
-    if (row == 0) {
-      dl_row = 0;
-      dl_fac = 0.f;
-    } else if (row & 1) {
-      dl_row = row + 1;
-      dl_fac = (float)m;
-    } else {
-      dl_row = row - 1;
-      dl_fac = -(float)m;
-    }
+    const int prow = row == 0 ? 0 : (row & 1) ? row + 1 : row - 1;
+    dlon = row == 0 ? 0.f : (row & 1) ? (float)m : -(float)m;
+    idx = (unsigned)(row * L + l);
+    ip = (unsigned)(prow * L + l);
+    iu = l + 1 < L ? idx + 1 : idx;
+    id = l >= 1 ? idx - 1 : idx;
     const float* ta = deriv + (size_t)tab * lw * L + (size_t)m * L;
-    const float* tb = ta + (size_t)lw * L;
-    a1 = (l + 1 < L) ? ta[l + 1] * (s ? s[l + 1] : 1.f) : 0.f;
-    b1 = (l >= 1) ? tb[l - 1] * (s ? s[l - 1] : 1.f) : 0.f;
+    a1 = l + 1 < L ? ta[l + 1] : 0.f;
+    b1 = l >= 1 ? ta[(size_t)lw * L + l - 1] : 0.f;
   }
-  __device__ float dlon(const float* x) const {
-    return dl_fac * x[(size_t)dl_row * L + l];
-  }
-  __device__ float dlat(const float* x) const {
-    const float* xr = x + (size_t)row * L + l;
-    float v = 0.f;
-    if (l + 1 < L) v += a1 * xr[1];
-    if (l >= 1) v += b1 * xr[-1];
-    return v;
+  __device__ __forceinline__ Nbr3 load(const float* x) const {
+    return {x[ip], x[iu], x[id]};
   }
 };
 
-// Threads cover (row, l) with l fastest; each walks kPlanesPerThread of the
-// (member, level) planes, reusing its operator coefficients.
-constexpr int kModalTX = 32, kModalTY = 8, kPlanesPerThread = 8;
-
-__global__ void __launch_bounds__(kModalTX * kModalTY) pe_prep_kernel(PrepArgs a) {
-  const int l = blockIdx.x * kModalTX + threadIdx.x;
-  const int row = blockIdx.y * kModalTY + threadIdx.y;
-  if (l >= a.L || row >= a.M) return;
+// u cos and v cos of the vorticity and divergence, and the gradients of ln ps
+// (and humidity): reads the state planes once, writes the aux planes once.
+// Every load of a plane's four rows is issued before its first store (24 in
+// flight a thread), because a store that might alias stops the loads behind it.
+__global__ void __launch_bounds__(kModalTX * kModalTY, 3) pe_prep_kernel(PrepArgs a, int ppt) {
+  const int l0 = blockIdx.x * kTile, row0 = blockIdx.y * kTile;
+  // The inverse transform does not read the aux planes below the triangle
+  // (they keep the zeros of their allocation).
+  if (below_triangle(row0, l0)) return;
+  const int l = l0 + threadIdx.x;
+  if (l >= a.L) return;
   const size_t ML = (size_t)a.M * a.L;
-  const size_t idx = (size_t)row * a.L + l;
   const float ir = a.inv_radius;
-  // u, v from vorticity / divergence through the inverse Laplacian (scaled
-  // coefficients); unscaled ones for the humidity and ln ps gradients.
-  const ModalNbr ns(row, l, a.L, a.lw, a.deriv, 0, a.invlap);
-  const ModalNbr nu(row, l, a.L, a.lw, a.deriv, 0, nullptr);
   const float il = a.invlap[l];
-  const int q0 = blockIdx.z * kPlanesPerThread;
-  const int q1 = min(q0 + kPlanesPerThread, a.K * a.mem);
+  const float ilu = a.invlap[min(l + 1, a.L - 1)], ild = a.invlap[max(l - 1, 0)];
+  ModalPoint pt[kTileRows] = {
+      {min(row0 + (int)threadIdx.y, a.M - 1), l, a.L, a.lw, a.deriv, 0},
+      {min(row0 + (int)threadIdx.y + kModalTY, a.M - 1), l, a.L, a.lw, a.deriv, 0},
+      {min(row0 + (int)threadIdx.y + 2 * kModalTY, a.M - 1), l, a.L, a.lw, a.deriv, 0},
+      {min(row0 + (int)threadIdx.y + 3 * kModalTY, a.M - 1), l, a.L, a.lw, a.deriv, 0}};
+  // Rows past the last are clamped to it and write its value again.
+  const int q0 = blockIdx.z * ppt;
+  const int q1 = min(q0 + ppt, a.K * a.mem);
   for (int q = q0; q < q1; ++q) {
     const int mb = q / a.K, k = q - mb * a.K;
     const float* vort = a.state + pl(a.p_vort, mb, a.K, k) * ML;
     const float* div = a.state + pl(a.p_div, mb, a.K, k) * ML;
-    // psi = lap^-1 vort, chi = lap^-1 div (l = 0 -> 0)
-    const float dchi = ns.dlon(div) * il;
-    const float dpsi = ns.dlon(vort) * il;
-    const float cchi = ns.dlat(div);
-    const float cpsi = ns.dlat(vort);
-    a.aux[pl(a.a_u, mb, a.K, k) * ML + idx] = (dchi - cpsi) * ir;
-    a.aux[pl(a.a_v, mb, a.K, k) * ML + idx] = (cchi + dpsi) * ir;
+    Nbr3 z[kTileRows], d[kTileRows];
+#pragma unroll
+    for (int i = 0; i < kTileRows; ++i) {
+      z[i] = pt[i].load(vort);
+      d[i] = pt[i].load(div);
+    }
+    float* au = a.aux + pl(a.a_u, mb, a.K, k) * ML;
+    float* av = a.aux + pl(a.a_v, mb, a.K, k) * ML;
+#pragma unroll
+    for (int i = 0; i < kTileRows; ++i) {
+      // psi = lap^-1 vort, chi = lap^-1 div (l = 0 -> 0)
+      const float cu = pt[i].a1 * ilu, cd = pt[i].b1 * ild;
+      const float dchi = pt[i].dlon * d[i].p * il, dpsi = pt[i].dlon * z[i].p * il;
+      const float cchi = cu * d[i].up + cd * d[i].dn;
+      const float cpsi = cu * z[i].up + cd * z[i].dn;
+      au[pt[i].idx] = (dchi - cpsi) * ir;
+      av[pt[i].idx] = (cchi + dpsi) * ir;
+    }
     if (a.hum >= 0) {
       const float* qh = a.state + pl(a.p_hum, mb, a.K, k) * ML;
-      a.aux[pl(a.a_gqx, mb, a.K, k) * ML + idx] = nu.dlon(qh) * ir;
-      a.aux[pl(a.a_gqy, mb, a.K, k) * ML + idx] = nu.dlat(qh) * ir;
+      float* gx = a.aux + pl(a.a_gqx, mb, a.K, k) * ML;
+      float* gy = a.aux + pl(a.a_gqy, mb, a.K, k) * ML;
+#pragma unroll
+      for (int i = 0; i < kTileRows; ++i) z[i] = pt[i].load(qh);
+#pragma unroll
+      for (int i = 0; i < kTileRows; ++i) {
+        gx[pt[i].idx] = pt[i].dlon * z[i].p * ir;
+        gy[pt[i].idx] = (pt[i].a1 * z[i].up + pt[i].b1 * z[i].dn) * ir;
+      }
     }
     if (k == 0) {
       const float* lnps = a.state + ((size_t)a.p_lnps + mb) * ML;
-      a.aux[((size_t)a.a_gx + mb) * ML + idx] = nu.dlon(lnps) * ir;
-      a.aux[((size_t)a.a_gy + mb) * ML + idx] = nu.dlat(lnps) * ir;
-      if (a.hum >= 0)
-        a.aux[((size_t)a.a_laplnps + mb) * ML + idx] = lnps[idx] * a.lap[l];
-      if (a.a_lnpsdev >= 0)
-        a.aux[((size_t)a.a_lnpsdev + mb) * ML + idx] = idx == 0 ? 0.f : lnps[idx];
+#pragma unroll
+      for (int i = 0; i < kTileRows; ++i) {
+        const unsigned e = pt[i].idx;
+        const Nbr3 x = pt[i].load(lnps);
+        const float v = lnps[e];
+        a.aux[((size_t)a.a_gx + mb) * ML + e] = pt[i].dlon * x.p * ir;
+        a.aux[((size_t)a.a_gy + mb) * ML + e] = (pt[i].a1 * x.up + pt[i].b1 * x.dn) * ir;
+        if (a.hum >= 0) a.aux[((size_t)a.a_laplnps + mb) * ML + e] = v * a.lap[l];
+        if (a.a_lnpsdev >= 0) a.aux[((size_t)a.a_lnpsdev + mb) * ML + e] = e == 0 ? 0.f : v;
+      }
     }
   }
-}
-
-static dim3 modal_grid(int M, int L, int planes) {
-  return dim3(ceil_div(L, kModalTX), ceil_div(M, kModalTY),
-              ceil_div(planes, kPlanesPerThread));
 }
 
 // ---------------------------------------------------------------------------
@@ -969,12 +1007,13 @@ __global__ void __launch_bounds__(kHybThreads) pe_nodal_hybrid_kernel(HybridArgs
 
 // ---------------------------------------------------------------------------
 // Modal post-pass: curl/div, Laplacians, horizontal advection divergence,
-// orography, humidity corrections, clip of the top wavenumber.
+// orography, humidity corrections, clip of the top wavenumber; in a SIL3 step
+// together with the stage that follows it.
 // ---------------------------------------------------------------------------
 
 struct PostArgs {
   const float* fm;  // forward outputs (modal)
-  float* tend;      // packed state layout
+  float* tend;      // packed state layout (a stage: null when f is not kept)
   const float* orog;
   int K, mem, nT, hum, hs;
   int M, L, lw;
@@ -986,55 +1025,226 @@ struct PostArgs {
   float inv_radius, gravity;
 };
 
-__global__ void __launch_bounds__(kModalTX * kModalTY) pe_post_kernel(PostArgs a) {
-  const int l = blockIdx.x * kModalTX + threadIdx.x;
-  const int row = blockIdx.y * kModalTY + threadIdx.y;
-  if (l >= a.L || row >= a.M) return;
-  const size_t ML = (size_t)a.M * a.L;
-  const size_t idx = (size_t)row * a.L + l;
+// The IMEX stage Y* = y0 + sum_j fc_j f_j + fself f + sum_j gc_j g_j, f being
+// the tendency the post-pass forms.  Planes without an implicit part
+// (vorticity, tracers) are final: they go to `out`, times the per-l filter
+// when given.  The implicit planes (n = 2K + 1 rows: div, T', ln ps) go to
+// `lm` in the l-major layout of the per-l operator product; the g_j are rows
+// of l-major arrays as well.
+struct StageArgs {
+  const float* y0;
+  const float* f[2];
+  float fc[2];
+  int nf;
+  float fself;
+  const float* g[2];
+  float gc[2];
+  int g_nk[2], g_row[2];  // rows per l of g_j, and the first of its n rows
+  int ng;
+  const float* filter;
+  float* out;
+  float* lm;
+  int Cp;
+};
+
+// Bound by memory: a stage reads the forward outputs, y0 and the earlier f_j
+// once and writes each result once.  Stage and post-pass are one kernel
+// because f is then combined from registers (the last stage's f never reaches
+// memory), and the implicit planes leave through a shared-memory transpose, so
+// that neither Y* nor the g_j pass through the row-major layout.  A tile below
+// the triangle has f = 0 but for the orography term of div, so its forward
+// outputs and f_j are not read (nearly half of the tiles).  All loads of two
+// rows (and the plane's g) are issued before the stores that follow them.
+// kNf: -1 for the plain post-pass, else the number of earlier f_j.
+template <int kNf>
+__global__ void __launch_bounds__(kModalTX * kModalTY, 3)
+    pe_post_kernel(PostArgs a, StageArgs s, int ppt) {
+  constexpr bool kStage = kNf >= 0;
+  constexpr int kF = kNf > 0 ? kNf : 1;  // array sizes
+  constexpr int kPair = 2;               // rows whose loads are in flight together
+  __shared__ float tile[kStage ? 2 : 1][kStage ? 3 : 1][kTile][kTile + 1];
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int l0 = blockIdx.x * kTile, row0 = blockIdx.y * kTile;
+  const int l = l0 + tx, lc = min(l, a.L - 1);
+  const bool zero = below_triangle(row0, l0);
   const int K = a.K;
+  const size_t ML = (size_t)a.M * a.L;
   const bool clip = (l == a.L - 1);
-  const float lam = a.lap[l];
+  const float lam = a.lap[lc];
+  const float filt = (kStage && s.filter) ? s.filter[lc] : 1.f;
   const float ir = a.inv_radius;
-  const float orog = a.gravity * lam * a.orog[idx];
-  const ModalNbr nb(row, l, a.L, a.lw, a.deriv, 2, nullptr);
-  const int q0 = blockIdx.z * kPlanesPerThread;
-  const int q1 = min(q0 + kPlanesPerThread, K * a.mem);
+  const int n = 2 * K + 1;
+  const int q0 = blockIdx.z * ppt;
+  const int q1 = min(q0 + ppt, K * a.mem);
   for (int q = q0; q < q1; ++q) {
     const int mb = q / K, k = q - mb * K;
+    float(*tl)[kTile][kTile + 1] = tile[kStage ? (q & 1) : 0];
+    // Entry of y0 + sum_j fc_j f_j + fself f; f_j = f below the triangle.
+    struct Old {
+      float y, f[kF];
+    };
+    auto old = [&](size_t e) {
+      Old o{};
+      o.y = s.y0[e];
+#pragma unroll
+      for (int j = 0; j < kNf; ++j) o.f[j] = zero ? 0.f : s.f[j][e];
+      return o;
+    };
+    auto staged = [&](const Old& o, float f) {
+      float v = o.y;
+#pragma unroll
+      for (int j = 0; j < kNf; ++j) v = fmaf(s.fc[j], zero ? f : o.f[j], v);
+      return fmaf(s.fself, f, v);
+    };
+    const bool keep = kStage ? (a.tend != nullptr && !zero) : true;
+    // The implicit terms at this thread's entries of the transposed tiles.
+    float gd[kTileRows], gt[kTileRows];
+    const int trow = row0 + tx;
+    const size_t c = (size_t)mb * a.M + trow;
+    if (kStage) {
+#pragma unroll
+      for (int i = 0; i < kTileRows; ++i) {
+        const size_t gl = (size_t)(l0 + ty + kModalTY * i);
+        gd[i] = gt[i] = 0.f;
+        if (trow < a.M && gl < (size_t)a.L) {
+          const float* g0 = s.g[0] + (gl * s.g_nk[0] + s.g_row[0] + k) * s.Cp + c;
+          gd[i] = s.gc[0] * g0[0];
+          gt[i] = s.gc[0] * g0[(size_t)K * s.Cp];
+          if (kNf == 2) {
+            const float* g1 = s.g[1] + (gl * s.g_nk[1] + s.g_row[1] + k) * s.Cp + c;
+            gd[i] = fmaf(s.gc[1], g1[0], gd[i]);
+            gt[i] = fmaf(s.gc[1], g1[(size_t)K * s.Cp], gt[i]);
+          }
+        }
+      }
+    }
 #define FM(p) (a.fm + pl(p, mb, K, k) * ML)
-#define OUT(p) a.tend[pl(p, mb, K, k) * ML + idx]
-    const float* Au = FM(a.o_Au);
-    const float* Av = FM(a.o_Av);
-    float vort = -(nb.dlon(Av) - nb.dlat(Au)) * ir;
-    float div = -(nb.dlon(Au) + nb.dlat(Av)) * ir;
-    div += -lam * FM(a.o_KE)[idx] - orog;
-    if (a.hum >= 0) {
-      vort += FM(a.o_vh)[idx];
-      div += -lam * FM(a.o_gh)[idx] - FM(a.o_dh)[idx];
+    const size_t pv = pl(a.p_vort, mb, K, k) * ML, pd = pl(a.p_div, mb, K, k) * ML,
+                 pt_ = pl(a.p_temp, mb, K, k) * ML;
+#pragma unroll
+    for (int i0 = 0; i0 < kTileRows; i0 += kPair) {
+      Nbr3 Au[kPair], Av[kPair], uT[kPair], vT[kPair];
+      float KE[kPair], Tn[kPair], og[kPair], vh[kPair], gh[kPair], dh[kPair], hs[kPair];
+      Old oz[kPair], od[kPair], ot[kPair];
+#pragma unroll
+      for (int i = 0; i < kPair; ++i) {
+        const int row = min(row0 + ty + kModalTY * (i0 + i), a.M - 1);
+        const ModalPoint p(row, lc, a.L, a.lw, a.deriv, 2);
+        Au[i] = Av[i] = uT[i] = vT[i] = {0.f, 0.f, 0.f};
+        KE[i] = Tn[i] = vh[i] = gh[i] = dh[i] = hs[i] = 0.f;
+        og[i] = a.orog[p.idx];
+        if (!zero) {
+          Au[i] = p.load(FM(a.o_Au));
+          Av[i] = p.load(FM(a.o_Av));
+          uT[i].p = FM(a.o_uT)[p.ip];
+          vT[i].up = FM(a.o_vT)[p.iu];
+          vT[i].dn = FM(a.o_vT)[p.id];
+          KE[i] = FM(a.o_KE)[p.idx];
+          Tn[i] = FM(a.o_Tn)[p.idx];
+          if (a.hum >= 0) {
+            vh[i] = FM(a.o_vh)[p.idx];
+            gh[i] = FM(a.o_gh)[p.idx];
+            dh[i] = FM(a.o_dh)[p.idx];
+          }
+          if (a.hs) hs[i] = FM(a.o_hsT)[p.idx];
+        }
+        if (kStage) {
+          oz[i] = old(pv + p.idx);
+          od[i] = old(pd + p.idx);
+          ot[i] = old(pt_ + p.idx);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kPair; ++i) {
+        const int rr = ty + kModalTY * (i0 + i);
+        if (l >= a.L || row0 + rr >= a.M) continue;
+        const ModalPoint p(row0 + rr, lc, a.L, a.lw, a.deriv, 2);
+        float vort = -(p.dlon * Av[i].p - (p.a1 * Au[i].up + p.b1 * Au[i].dn)) * ir + vh[i];
+        float div = -(p.dlon * Au[i].p + (p.a1 * Av[i].up + p.b1 * Av[i].dn)) * ir;
+        div += -lam * KE[i] - a.gravity * lam * og[i];
+        div += -lam * gh[i] - dh[i];
+        float temp = Tn[i] - (p.dlon * uT[i].p + (p.a1 * vT[i].up + p.b1 * vT[i].dn)) * ir;
+        if (clip) vort = div = temp = 0.f;
+        temp += hs[i];
+        if (keep) {
+          a.tend[pv + p.idx] = vort;
+          a.tend[pd + p.idx] = div;
+          a.tend[pt_ + p.idx] = temp;
+        }
+        if (kStage) {
+          s.out[pv + p.idx] = staged(oz[i], vort) * filt;
+          tl[0][rr][tx] = staged(od[i], div);
+          tl[1][rr][tx] = staged(ot[i], temp);
+        }
+      }
     }
-    float temp = FM(a.o_Tn)[idx] - (nb.dlon(FM(a.o_uT)) + nb.dlat(FM(a.o_vT))) * ir;
-    if (clip) {
-      vort = 0.f;
-      div = 0.f;
-      temp = 0.f;
-    }
-    if (a.hs) temp += FM(a.o_hsT)[idx];
-    OUT(a.p_vort) = vort;
-    OUT(a.p_div) = div;
-    OUT(a.p_temp) = temp;
     for (int t = 0; t < a.nT; ++t) {
       const int ob = a.o_tr + 3 * t * a.mem * K;
-      float qv = FM(ob + 2 * a.mem * K)[idx] -
-                 (nb.dlon(FM(ob)) + nb.dlat(FM(ob + a.mem * K))) * ir;
-      OUT(a.p_tr + t * a.mem * K) = clip ? 0.f : qv;
+      const size_t pq = pl(a.p_tr + t * a.mem * K, mb, K, k) * ML;
+      float fq[kTileRows];
+      Old oq[kTileRows];
+#pragma unroll
+      for (int i = 0; i < kTileRows; ++i) {
+        const int row = min(row0 + ty + kModalTY * i, a.M - 1);
+        const ModalPoint p(row, lc, a.L, a.lw, a.deriv, 2);
+        fq[i] = 0.f;
+        if (!zero)
+          fq[i] = FM(ob + 2 * a.mem * K)[p.idx] -
+                  (p.dlon * FM(ob)[p.ip] + (p.a1 * FM(ob + a.mem * K)[p.iu] +
+                                            p.b1 * FM(ob + a.mem * K)[p.id])) * ir;
+        if (clip) fq[i] = 0.f;
+        if (kStage) oq[i] = old(pq + p.idx);
+      }
+#pragma unroll
+      for (int i = 0; i < kTileRows; ++i) {
+        const int row = row0 + ty + kModalTY * i;
+        if (l >= a.L || row >= a.M) continue;
+        const size_t e = pq + (size_t)row * a.L + l;
+        if (keep) a.tend[e] = fq[i];
+        if (kStage) s.out[e] = staged(oq[i], fq[i]) * filt;
+      }
     }
     if (k == 0) {
-      const float lnps = a.fm[((size_t)a.o_lnps + mb) * ML + idx];
-      a.tend[((size_t)a.p_lnps + mb) * ML + idx] = clip ? 0.f : lnps;
+#pragma unroll
+      for (int i = 0; i < kTileRows; ++i) {
+        const int rr = ty + kModalTY * i, row = row0 + rr;
+        if (l >= a.L || row >= a.M) continue;
+        const size_t idx = (size_t)row * a.L + l;
+        const float f = (zero || clip) ? 0.f : a.fm[((size_t)a.o_lnps + mb) * ML + idx];
+        const size_t e = ((size_t)a.p_lnps + mb) * ML + idx;
+        if (kStage) tl[2][rr][tx] = staged(old(e), f);
+        if (keep) a.tend[e] = f;
+      }
     }
 #undef FM
-#undef OUT
+    if (!kStage) continue;
+    // One barrier a plane: the next plane uses the other tile buffer, which
+    // everyone has finished reading before passing this plane's barrier.
+    __syncthreads();
+    if (trow < a.M) {
+#pragma unroll
+      for (int i = 0; i < kTileRows; ++i) {
+        const int ll = ty + kModalTY * i;
+        if (l0 + ll >= a.L) continue;
+        float* o = s.lm + ((size_t)(l0 + ll) * n + k) * s.Cp + c;
+        o[0] = tl[0][tx][ll] + gd[i];
+        o[(size_t)K * s.Cp] = tl[1][tx][ll] + gt[i];
+      }
+      if (k == 0) {
+#pragma unroll
+        for (int i = 0; i < kTileRows; ++i) {
+          const int ll = ty + kModalTY * i;
+          const size_t gl = (size_t)(l0 + ll);
+          if (l0 + ll >= a.L) continue;
+          float v = tl[2][tx][ll];
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            if (j < s.ng)
+              v = fmaf(s.gc[j], s.g[j][(gl * s.g_nk[j] + s.g_row[j] + 2 * K) * s.Cp + c], v);
+          s.lm[(gl * n + 2 * K) * s.Cp + c] = v;
+        }
+      }
+    }
   }
 }
 
@@ -1103,7 +1313,7 @@ struct ModalNbrT {
   }
 };
 
-__global__ void __launch_bounds__(kModalTX * kModalTY) pe_post_adjoint_kernel(PostAdjArgs a) {
+__global__ void __launch_bounds__(kModalTX * kModalTY) pe_post_adjoint_kernel(PostAdjArgs a, int ppt) {
   const int l = blockIdx.x * kModalTX + threadIdx.x;
   const int row = blockIdx.y * kModalTY + threadIdx.y;
   if (l >= a.L || row >= a.M) return;
@@ -1115,8 +1325,8 @@ __global__ void __launch_bounds__(kModalTX * kModalTY) pe_post_adjoint_kernel(Po
   const float ir = a.inv_radius;
   const float lam = a.lap[l];
   const ModalNbrT nb(row, l, a.L, a.lw, a.deriv, 2, Lc);
-  const int q0 = blockIdx.z * kPlanesPerThread;
-  const int q1 = min(q0 + kPlanesPerThread, K * a.mem);
+  const int q0 = blockIdx.z * ppt;
+  const int q1 = min(q0 + ppt, K * a.mem);
   for (int q = q0; q < q1; ++q) {
     const int mb = q / K, k = q - mb * K;
 #define TB(p) (a.tbar + pl(p, mb, K, k) * ML)
@@ -1454,7 +1664,7 @@ struct PrepAdjArgs {
   float inv_radius;
 };
 
-__global__ void __launch_bounds__(kModalTX * kModalTY) pe_prep_adjoint_kernel(PrepAdjArgs a) {
+__global__ void __launch_bounds__(kModalTX * kModalTY) pe_prep_adjoint_kernel(PrepAdjArgs a, int ppt) {
   const int l = blockIdx.x * kModalTX + threadIdx.x;
   const int row = blockIdx.y * kModalTY + threadIdx.y;
   if (l >= a.L || row >= a.M) return;
@@ -1465,8 +1675,8 @@ __global__ void __launch_bounds__(kModalTX * kModalTY) pe_prep_adjoint_kernel(Pr
   const float ir = a.inv_radius;
   const float s = a.invlap[l] * ir;
   const ModalNbrT nb(row, l, a.L, a.lw, a.deriv, 0, a.L);
-  const int q0 = blockIdx.z * kPlanesPerThread;
-  const int q1 = min(q0 + kPlanesPerThread, K * a.mem);
+  const int q0 = blockIdx.z * ppt;
+  const int q1 = min(q0 + ppt, K * a.mem);
   for (int q = q0; q < q1; ++q) {
     const int mb = q / K, k = q - mb * K;
     const float* ub = a.xbar + pl(a.p_u, mb, K, k) * ML;
@@ -1669,50 +1879,8 @@ __global__ void pe_matrix_build_kernel(MatBuildArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// IMEX stage: an elementwise combine and a per-(m, l) implicit solve
+// Per-l products of the implicit planes
 // ---------------------------------------------------------------------------
-
-// Y* = y0 + sum_t fc_t f_t + sum_t gc_t g_t over every plane of the packed
-// state (g terms exist on the divergence, temperature and ln ps planes only).
-// Planes without an implicit part (vorticity, tracers) are final after the
-// combine: they go to `out` (times the per-l filter when given); the
-// implicit planes go to `ystar` for the solve.
-struct CombineArgs {
-  const float* y0;
-  const float* f[3];
-  float fc[3];
-  int nf;
-  const float* g[2];
-  float gc[2];
-  int ng;
-  const float* filter;
-  float* out;
-  float* ystar;
-  int mK, nT, L;
-  size_t ML;
-};
-
-__global__ void pe_combine_kernel(CombineArgs a) {
-  const int plane = blockIdx.y;
-  size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= a.ML) return;
-  const bool implicit_plane =
-      (plane >= a.mK && plane < 3 * a.mK) || plane >= (3 + a.nT) * a.mK;
-  const size_t p = (size_t)plane * a.ML + idx;
-  float v = a.y0[p];
-#pragma unroll
-  for (int t = 0; t < 3; ++t)
-    if (t < a.nf) v = fmaf(a.fc[t], a.f[t][p], v);
-  if (implicit_plane) {
-#pragma unroll
-    for (int t = 0; t < 2; ++t)
-      if (t < a.ng) v = fmaf(a.gc[t], a.g[t][p], v);
-    a.ystar[p] = v;
-  } else {
-    if (a.filter) v *= a.filter[idx % a.L];
-    a.out[p] = v;
-  }
-}
 
 // Per-(l, column) application of an implicit operator: for every total
 // wavenumber l, Out[R x C] = A_l[R x nin] Ys[nin x C], where the C = members * M
@@ -1730,7 +1898,6 @@ struct LmArgs {
   const float* src2;  // gather: stacked planes [n, 2n), scaled by s2
   float s1, s2;
   float* out;         // scatter: rows [0, n)
-  float* out2;        // scatter: rows [n, 2n)
   float* lm;          // gather output / scatter input: [L][nk][Cp]
   int nk, n, K, M, L, C, Cp;
   int p_div, p_temp, p_lnps;
@@ -1774,8 +1941,8 @@ __global__ void __launch_bounds__(256) pe_lm_gather_kernel(LmArgs a) {
   }
 }
 
-// Row r of the l-major product back into the state layout (rows [0, n) to
-// out, [n, 2n) to out2), tiled like the gather.
+// Row r < n of the l-major product back into the state layout, tiled like the
+// gather.
 __global__ void __launch_bounds__(256) pe_lm_scatter_kernel(LmArgs a) {
   __shared__ float tile[32][33];
   const int r = blockIdx.z;
@@ -1794,8 +1961,7 @@ __global__ void __launch_bounds__(256) pe_lm_scatter_kernel(LmArgs a) {
     }
   }
   __syncthreads();
-  float* dst = (r < a.n ? a.out : a.out2) +
-               stacked_plane(a, r < a.n ? r : r - a.n, mb) * a.ML;
+  float* dst = a.out + stacked_plane(a, r, mb) * a.ML;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int rr = ty + 8 * i, row = row0 + rr, l = l0 + tx;
@@ -1925,16 +2091,9 @@ static void apply_launch(dim3 grid, size_t smem, cudaStream_t st, const ApplyArg
   pe_apply_kernel<TR><<<grid, 256, smem, st>>>(a);
 }
 
-static int launch_apply(dino_pe* pe, const MatEntry* m, const float* src,
-                        float* out, float* out2, cudaStream_t st,
-                        const float* src2 = nullptr, float s1 = 1.f, float s2 = 1.f) {
+static LmArgs lm_args(dino_pe* pe) {
   LmArgs g{};
-  g.src = src;
-  g.src2 = src2;
-  g.s1 = s1;
-  g.s2 = s2;
-  g.out = out;
-  g.out2 = out2;
+  g.s1 = g.s2 = 1.f;
   g.n = 2 * pe->K + 1;
   g.K = pe->K;
   g.M = pe->M;
@@ -1945,22 +2104,38 @@ static int launch_apply(dino_pe* pe, const MatEntry* m, const float* src,
   g.p_temp = 2 * pe->mem * pe->K;
   g.p_lnps = (3 + pe->nT) * pe->mem * pe->K;
   g.ML = pe->ML;
-  const dim3 tiles(ceil_div(pe->L, 32), ceil_div(pe->M, 32) * pe->mem);
+  return g;
+}
+
+// The implicit planes of src (and, for nk = 2n rows, of src2, scaled by s1 and
+// s2) into the l-major operand pe->d_lm_in.
+static int lm_gather(dino_pe* pe, int nk, const float* src, cudaStream_t st,
+                     const float* src2 = nullptr, float s1 = 1.f, float s2 = 1.f) {
+  LmArgs g = lm_args(pe);
+  g.src = src;
+  g.src2 = src2;
+  g.s1 = s1;
+  g.s2 = s2;
   g.lm = pe->d_lm_in;
-  g.nk = m->nin;
-  pe_lm_gather_kernel<<<dim3(tiles.x, tiles.y, m->nin), 256, 0, st>>>(g);
-  DINO_TRY(check_launch("pe_lm_gather"));
+  g.nk = nk;
+  const dim3 grid(ceil_div(pe->L, 32), ceil_div(pe->M, 32) * pe->mem, nk);
+  pe_lm_gather_kernel<<<grid, 256, 0, st>>>(g);
+  return check_launch("pe_lm_gather");
+}
+
+// The first `rows` rows of the per-l products of m with pe->d_lm_in.
+static int lm_apply(dino_pe* pe, const MatEntry* m, int rows, float* olm, cudaStream_t st) {
   ApplyArgs a{};
   a.A = m->d;
   a.ylm = pe->d_lm_in;
-  a.olm = pe->d_lm_out;
-  a.R = m->R;
+  a.olm = olm;
+  a.R = rows;
   a.nin = m->nin;
   a.RP = m->RP;
   a.Cp = pe->Cp;
-  const int tr = apply_tr(m->R);
+  const int tr = apply_tr(rows);
   const int rpt = 16 * tr;
-  dim3 grid(pe->Cp / kApplyCols, pe->L, ceil_div(m->R, rpt));
+  dim3 grid(pe->Cp / kApplyCols, pe->L, ceil_div(rows, rpt));
   const size_t smem = apply_smem(a.nin, tr);
   switch (tr) {
     case 1: apply_launch<1>(grid, smem, st, a); break;
@@ -1973,42 +2148,28 @@ static int launch_apply(dino_pe* pe, const MatEntry* m, const float* src,
     case 8: apply_launch<8>(grid, smem, st, a); break;
     default: apply_launch<9>(grid, smem, st, a); break;
   }
-  DINO_TRY(check_launch("pe_apply"));
+  return check_launch("pe_apply");
+}
+
+// The first n of the nk rows per l of pe->d_lm_out into out's implicit planes.
+static int lm_scatter(dino_pe* pe, int nk, float* out, cudaStream_t st) {
+  LmArgs g = lm_args(pe);
+  g.out = out;
   g.lm = pe->d_lm_out;
-  g.nk = m->R;
-  pe_lm_scatter_kernel<<<dim3(tiles.x, tiles.y, m->R), 256, 0, st>>>(g);
+  g.nk = nk;
+  const dim3 grid(ceil_div(pe->L, 32), ceil_div(pe->M, 32) * pe->mem, g.n);
+  pe_lm_scatter_kernel<<<grid, 256, 0, st>>>(g);
   return check_launch("pe_lm_scatter");
 }
 
-struct Term {
-  float c;
-  const float* x;
-};
-
-static int launch_combine(dino_pe* pe, const float* y0,
-                          std::initializer_list<Term> f,
-                          std::initializer_list<Term> g, const float* filter,
-                          float* out, cudaStream_t st) {
-  CombineArgs a{};
-  a.y0 = y0;
-  for (const Term& t : f) {
-    a.fc[a.nf] = t.c;
-    a.f[a.nf++] = t.x;
-  }
-  for (const Term& t : g) {
-    a.gc[a.ng] = t.c;
-    a.g[a.ng++] = t.x;
-  }
-  a.filter = filter;
-  a.out = out;
-  a.ystar = pe->d_ystar;
-  a.mK = pe->mem * pe->K;
-  a.nT = pe->nT;
-  a.L = pe->L;
-  a.ML = pe->ML;
-  dim3 grid(ceil_div((int)pe->ML, 256), pe->n_state);
-  pe_combine_kernel<<<grid, 256, 0, st>>>(a);
-  return check_launch("pe_combine");
+// out's implicit planes = the product of m with those of src (and src2).
+static int launch_apply(dino_pe* pe, const MatEntry* m, const float* src, float* out,
+                        cudaStream_t st, const float* src2 = nullptr, float s1 = 1.f,
+                        float s2 = 1.f) {
+  const int n = 2 * pe->K + 1;
+  DINO_TRY(lm_gather(pe, m->nin, src, st, src2, s1, s2));
+  DINO_TRY(lm_apply(pe, m, n, pe->d_lm_out, st));
+  return lm_scatter(pe, n, out, st);
 }
 
 static int get_matrix(dino_pe* pe, int kind, double eta, const double* host_filter,
@@ -2110,6 +2271,20 @@ static int get_filter(dino_pe* pe, const double* host, float** out) {
   return DINO_OK;
 }
 
+// Launch shapes of the modal passes and their planes per CTA (thread).
+static dim3 tile_grid(const dino_pe* pe, int* ppt) {
+  const int tl = ceil_div(pe->L, kTile), tr = ceil_div(pe->M, kTile);
+  const int planes = pe->K * pe->mem;
+  *ppt = planes_per_cta(tl * tr, planes, pe->sms);
+  return dim3(tl, tr, ceil_div(planes, *ppt));
+}
+static dim3 modal_grid(const dino_pe* pe, int* ppt) {
+  const int tl = ceil_div(pe->L, kModalTX), tr = ceil_div(pe->M, kModalTY);
+  const int planes = pe->K * pe->mem;
+  *ppt = planes_per_cta(tl * tr, planes, pe->sms);
+  return dim3(tl, tr, ceil_div(planes, *ppt));
+}
+
 // Modal pre-pass and inverse transforms: the nodal inputs of the column
 // kernel in pe->d_nodal.
 static int pe_nodal_inputs(dino_pe* pe, const float* state, cudaStream_t st) {
@@ -2151,7 +2326,9 @@ static int pe_nodal_inputs(dino_pe* pe, const float* state, cudaStream_t st) {
     a.lap = p->d_lap;
     a.invlap = p->d_invlap;
     a.inv_radius = (float)(1.0 / p->radius);
-    pe_prep_kernel<<<modal_grid(pe->M, pe->L, K * mem), dim3(kModalTX, kModalTY), 0, st>>>(a);
+    int ppt = 0;
+    const dim3 grid = tile_grid(pe, &ppt);
+    pe_prep_kernel<<<grid, dim3(kModalTX, kModalTY), 0, st>>>(a, ppt);
     DINO_TRY(check_launch("pe_prep"));
   }
   // 2. inverse SHT of [state kinds][aux][ln ps (Held-Suarez)]
@@ -2335,58 +2512,107 @@ static NodalArgs make_nodal_args(dino_pe* pe) {
   return a;
 }
 
-static int pe_explicit_impl(dino_pe* pe, const float* state, float* tend,
-                            cudaStream_t st) {
-  dino_plan* p = pe->plan;
-  const int K = pe->K, mem = pe->mem;
-  const int mK = mem * K;
+// The explicit terms of `state` up to the forward transform: the modal
+// products in pe->d_fwd_out, which the post-pass turns into tendencies.
+static int pe_explicit_products(dino_pe* pe, const float* state, cudaStream_t st) {
   DINO_TRY(pe_nodal_inputs(pe, state, st));
-  // 3. fused nodal column kernel
-  {
-    DINO_TRY(launch_nodal(pe, state, st));
+  DINO_TRY(launch_nodal(pe, state, st));
+  return sht_forward_to(pe->plan, pe->d_fwd_in, pe->d_fwd_out, pe->n_fwd, pe->d_work,
+                        pe->work_fields, st);
+}
+
+static PostArgs make_post_args(dino_pe* pe, float* tend) {
+  const int mK = pe->mem * pe->K;
+  PostArgs a{};
+  a.fm = pe->d_fwd_out;
+  a.tend = tend;
+  a.orog = pe->d_orog;
+  a.K = pe->K;
+  a.mem = pe->mem;
+  a.nT = pe->nT;
+  a.hum = pe->hum;
+  a.hs = pe->hs;
+  a.M = pe->M;
+  a.L = pe->L;
+  a.lw = pe->plan->lw;
+  a.o_Au = pe->o_Au;
+  a.o_Av = pe->o_Av;
+  a.o_KE = pe->o_KE;
+  a.o_uT = pe->o_uT;
+  a.o_vT = pe->o_vT;
+  a.o_Tn = pe->o_Tn;
+  a.o_tr = pe->o_tr;
+  a.o_vh = pe->o_vh;
+  a.o_gh = pe->o_gh;
+  a.o_dh = pe->o_dh;
+  a.o_hsT = pe->o_hsT;
+  a.o_lnps = pe->o_lnps;
+  a.p_vort = 0;
+  a.p_div = mK;
+  a.p_temp = 2 * mK;
+  a.p_tr = 3 * mK;
+  a.p_lnps = (3 + pe->nT) * mK;
+  a.deriv = pe->plan->d_deriv;
+  a.lap = pe->plan->d_lap;
+  a.inv_radius = (float)(1.0 / pe->plan->radius);
+  a.gravity = (float)pe->g;
+  return a;
+}
+
+static int pe_explicit_impl(dino_pe* pe, const float* state, float* tend, cudaStream_t st) {
+  DINO_TRY(pe_explicit_products(pe, state, st));
+  int ppt = 0;
+  const dim3 grid = tile_grid(pe, &ppt);
+  pe_post_kernel<-1><<<grid, dim3(kModalTX, kModalTY), 0, st>>>(make_post_args(pe, tend),
+                                                                StageArgs{}, ppt);
+  return check_launch("pe_post");
+}
+
+struct Term {
+  float c;
+  const float* x;
+};
+struct GTerm {
+  float c;
+  const float* lm;
+  int nk, row;
+};
+
+// A SIL3 stage from the products of the last explicit evaluation (StageArgs):
+// Y* into pe->d_lm_in and the final planes into `out`; `keep_f`: where the
+// tendency itself goes, or null.
+static int launch_stage(dino_pe* pe, const float* y0, std::initializer_list<Term> f,
+                        float fself, float* keep_f, std::initializer_list<GTerm> g,
+                        const float* filter, float* out, cudaStream_t st) {
+  StageArgs s{};
+  s.y0 = y0;
+  for (const Term& t : f) {
+    s.fc[s.nf] = t.c;
+    s.f[s.nf++] = t.x;
   }
-  // 4. forward SHT
-  DINO_TRY(sht_forward_to(p, pe->d_fwd_in, pe->d_fwd_out, pe->n_fwd, pe->d_work,
-                          pe->work_fields, st));
-  // 5. modal post-pass
-  {
-    PostArgs a{};
-    a.fm = pe->d_fwd_out;
-    a.tend = tend;
-    a.orog = pe->d_orog;
-    a.K = K;
-    a.mem = mem;
-    a.nT = pe->nT;
-    a.hum = pe->hum;
-    a.hs = pe->hs;
-    a.M = pe->M;
-    a.L = pe->L;
-    a.lw = p->lw;
-    a.o_Au = pe->o_Au;
-    a.o_Av = pe->o_Av;
-    a.o_KE = pe->o_KE;
-    a.o_uT = pe->o_uT;
-    a.o_vT = pe->o_vT;
-    a.o_Tn = pe->o_Tn;
-    a.o_tr = pe->o_tr;
-    a.o_vh = pe->o_vh;
-    a.o_gh = pe->o_gh;
-    a.o_dh = pe->o_dh;
-    a.o_hsT = pe->o_hsT;
-    a.o_lnps = pe->o_lnps;
-    a.p_vort = 0;
-    a.p_div = mK;
-    a.p_temp = 2 * mK;
-    a.p_tr = 3 * mK;
-    a.p_lnps = (3 + pe->nT) * mK;
-    a.deriv = p->d_deriv;
-    a.lap = p->d_lap;
-    a.inv_radius = (float)(1.0 / p->radius);
-    a.gravity = (float)pe->g;
-    pe_post_kernel<<<modal_grid(pe->M, pe->L, K * mem), dim3(kModalTX, kModalTY), 0, st>>>(a);
-    DINO_TRY(check_launch("pe_post"));
+  s.fself = fself;
+  for (const GTerm& t : g) {
+    s.gc[s.ng] = t.c;
+    s.g_nk[s.ng] = t.nk;
+    s.g_row[s.ng] = t.row;
+    s.g[s.ng++] = t.lm;
   }
-  return DINO_OK;
+  s.filter = filter;
+  s.out = out;
+  s.lm = pe->d_lm_in;
+  s.Cp = pe->Cp;
+  int ppt = 0;
+  const dim3 grid = tile_grid(pe, &ppt);
+  const PostArgs a = make_post_args(pe, keep_f);
+  const dim3 block(kModalTX, kModalTY);
+  // The stage with two earlier f_j is also the one with two g_j.
+  if (s.nf == 0)
+    pe_post_kernel<0><<<grid, block, 0, st>>>(a, s, ppt);
+  else if (s.nf == 1)
+    pe_post_kernel<1><<<grid, block, 0, st>>>(a, s, ppt);
+  else
+    pe_post_kernel<2><<<grid, block, 0, st>>>(a, s, ppt);
+  return check_launch("pe_stage");
 }
 
 // One filtered imex_rk_sil3 step in place (time_integration.py:329-405 with
@@ -2397,7 +2623,9 @@ static int pe_explicit_impl(dino_pe* pe, const float* state, float* tend,
 //   Y2 = (1 - dt/3 G)^-1 (y + dt/6 f0 + dt/2 f1 + dt/3 g0),  f2 = F(Y2), g2 = G(Y2)
 //   Y3* = y + dt/2 f0 - dt/2 f1 + dt f2 + 3dt/8 g0 + 3dt/8 g2
 //   y_next = filter(Y3* + dt/4 G((1 - dt/4 G)^-1 Y3*))
-// Each stage is one elementwise combine plus one per-l operator product.
+// Each stage is the post-pass of its explicit evaluation and the combination
+// (one kernel), one per-l operator product and the scatter of its result; the
+// implicit terms g0 and g2 stay in the l-major layout of the products.
 struct StepMats {
   const MatEntry* L;      // G
   const MatEntry* inv1;   // (1 - dt/6 G)^-1
@@ -2414,29 +2642,40 @@ static int get_step_mats(dino_pe* pe, double dt, const double* host_filter,
   return DINO_OK;
 }
 
-static int pe_step_once(dino_pe* pe, float* y, double dt, const float* filt,
-                        const StepMats& m, cudaStream_t st) {
-  DINO_TRY(pe_explicit_impl(pe, y, pe->d_f[0], st));
-  DINO_TRY(launch_apply(pe, m.L, y, pe->d_g[0], nullptr, st));
-  DINO_TRY(launch_combine(pe, y, {{(float)(dt / 3.0), pe->d_f[0]}},
-                          {{(float)(dt / 6.0), pe->d_g[0]}}, nullptr, pe->d_Y, st));
-  DINO_TRY(launch_apply(pe, m.inv1, pe->d_ystar, pe->d_Y, nullptr, st));
-  DINO_TRY(pe_explicit_impl(pe, pe->d_Y, pe->d_f[1], st));
-  DINO_TRY(launch_combine(
-      pe, y, {{(float)(dt / 6.0), pe->d_f[0]}, {(float)(dt * 0.5), pe->d_f[1]}},
-      {{(float)(dt / 3.0), pe->d_g[0]}}, nullptr, pe->d_Y, st));
-  DINO_TRY(launch_apply(pe, m.invg2, pe->d_ystar, pe->d_Y, pe->d_g[1], st));
-  DINO_TRY(pe_explicit_impl(pe, pe->d_Y, pe->d_f[2], st));
-  DINO_TRY(launch_combine(
-      pe, y,
-      {{(float)(dt * 0.5), pe->d_f[0]}, {(float)(dt * -0.5), pe->d_f[1]},
-       {(float)dt, pe->d_f[2]}},
-      {{(float)(dt * 0.375), pe->d_g[0]}, {(float)(dt * 0.375), pe->d_g[1]}},
-      filt, y, st));
-  DINO_TRY(launch_apply(pe, m.fin3, pe->d_ystar, y, nullptr, st));
-  return DINO_OK;
+// The stage states Y1 and Y2 of a step from y: f0 (and f1 when keep_f1) in
+// pe->d_f, g0 in pe->d_lm_g0 and, when with_g2, g2 in the second n rows of
+// pe->d_lm_out.  Leaves Y2 in Y2 (which may be Y1).
+static int pe_step_stages(dino_pe* pe, const float* y, float* Y1, float* Y2, double dt,
+                          const StepMats& m, bool keep_f1, bool with_g2, cudaStream_t st) {
+  const int n = 2 * pe->K + 1;
+  DINO_TRY(lm_gather(pe, n, y, st));
+  DINO_TRY(lm_apply(pe, m.L, n, pe->d_lm_g0, st));
+  DINO_TRY(pe_explicit_products(pe, y, st));
+  DINO_TRY(launch_stage(pe, y, {}, (float)(dt / 3.0), pe->d_f[0],
+                        {{(float)(dt / 6.0), pe->d_lm_g0, n, 0}}, nullptr, Y1, st));
+  DINO_TRY(lm_apply(pe, m.inv1, n, pe->d_lm_out, st));
+  DINO_TRY(lm_scatter(pe, n, Y1, st));
+  DINO_TRY(pe_explicit_products(pe, Y1, st));
+  DINO_TRY(launch_stage(pe, y, {{(float)(dt / 6.0), pe->d_f[0]}}, (float)(dt * 0.5),
+                        keep_f1 ? pe->d_f[1] : nullptr,
+                        {{(float)(dt / 3.0), pe->d_lm_g0, n, 0}}, nullptr, Y2, st));
+  DINO_TRY(lm_apply(pe, m.invg2, with_g2 ? 2 * n : n, pe->d_lm_out, st));
+  return lm_scatter(pe, with_g2 ? 2 * n : n, Y2, st);
 }
 
+static int pe_step_once(dino_pe* pe, float* y, double dt, const float* filt,
+                        const StepMats& m, cudaStream_t st) {
+  const int n = 2 * pe->K + 1;
+  DINO_TRY(pe_step_stages(pe, y, pe->d_Y, pe->d_Y, dt, m, true, true, st));
+  DINO_TRY(pe_explicit_products(pe, pe->d_Y, st));
+  const float c = (float)(dt * 0.375);
+  DINO_TRY(launch_stage(pe, y,
+                        {{(float)(dt * 0.5), pe->d_f[0]}, {(float)(dt * -0.5), pe->d_f[1]}},
+                        (float)dt, nullptr,
+                        {{c, pe->d_lm_g0, n, 0}, {c, pe->d_lm_out, 2 * n, n}}, filt, y, st));
+  DINO_TRY(lm_apply(pe, m.fin3, n, pe->d_lm_out, st));
+  return lm_scatter(pe, n, y, st);
+}
 
 // ---------------------------------------------------------------------------
 // Reverse mode
@@ -2489,8 +2728,9 @@ static int pe_explicit_vjp_impl(dino_pe* pe, const float* state, const float* tb
     a.deriv = p->d_deriv;
     a.lap = p->d_lap;
     a.inv_radius = (float)(1.0 / p->radius);
-    pe_post_adjoint_kernel<<<modal_grid(pe->M, pe->L, K * mem), dim3(kModalTX, kModalTY), 0,
-                             st>>>(a);
+    int ppt = 0;
+    const dim3 grid = modal_grid(pe, &ppt);
+    pe_post_adjoint_kernel<<<grid, dim3(kModalTX, kModalTY), 0, st>>>(a, ppt);
     DINO_TRY(check_launch("pe_post_adjoint"));
   }
   DINO_TRY(sht_forward_adjoint_to(p, pe->d_fwd_out, pe->d_fwd_in, pe->n_fwd,
@@ -2531,8 +2771,9 @@ static int pe_explicit_vjp_impl(dino_pe* pe, const float* state, const float* tb
     a.lap = p->d_lap;
     a.invlap = p->d_invlap;
     a.inv_radius = (float)(1.0 / p->radius);
-    pe_prep_adjoint_kernel<<<modal_grid(pe->M, pe->L, K * mem), dim3(kModalTX, kModalTY), 0,
-                             st>>>(a);
+    int ppt = 0;
+    const dim3 grid = modal_grid(pe, &ppt);
+    pe_prep_adjoint_kernel<<<grid, dim3(kModalTX, kModalTY), 0, st>>>(a, ppt);
     DINO_TRY(check_launch("pe_prep_adjoint"));
   }
   return DINO_OK;
@@ -2600,29 +2841,20 @@ static int pe_step_vjp_impl(dino_pe* pe, const float* y, const float* out_ct,
   float* V = pe->d_adj[5];
   const float fdt = (float)dt;
   // Stage states.
-  DINO_TRY(pe_explicit_impl(pe, y, pe->d_f[0], st));
-  DINO_TRY(launch_apply(pe, m.L, y, pe->d_g[0], nullptr, st));
-  DINO_TRY(launch_combine(pe, y, {{(float)(dt / 3.0), pe->d_f[0]}},
-                          {{(float)(dt / 6.0), pe->d_g[0]}}, nullptr, Y1, st));
-  DINO_TRY(launch_apply(pe, m.inv1, pe->d_ystar, Y1, nullptr, st));
-  DINO_TRY(pe_explicit_impl(pe, Y1, pe->d_f[1], st));
-  DINO_TRY(launch_combine(
-      pe, y, {{(float)(dt / 6.0), pe->d_f[0]}, {(float)(dt * 0.5), pe->d_f[1]}},
-      {{(float)(dt / 3.0), pe->d_g[0]}}, nullptr, Y2, st));
-  DINO_TRY(launch_apply(pe, m.invg2, pe->d_ystar, Y2, pe->d_g[1], st));
+  DINO_TRY(pe_step_stages(pe, y, Y1, Y2, dt, m, false, false, st));
   // Reverse sweep.
   float* C = pe->d_f[0];
-  DINO_TRY(launch_apply(pe, mt.fin3, out_ct, Z3, nullptr, st));
+  DINO_TRY(launch_apply(pe, mt.fin3, out_ct, Z3, st));
   DINO_TRY(launch_lincomb(pe, {{out_ct, 0.f, 1.f}}, filt, Z3, 2, st));
   DINO_TRY(launch_lincomb(pe, {{Z3, fdt, fdt}}, nullptr, C, 0, st));
   DINO_TRY(pe_explicit_vjp_impl(pe, Y2, C, V, st));
-  DINO_TRY(launch_apply(pe, mt.invg2, V, Z2, nullptr, st, Z3, 1.f,
+  DINO_TRY(launch_apply(pe, mt.invg2, V, Z2, st, Z3, 1.f,
                         (float)(dt * 0.375)));
   DINO_TRY(launch_lincomb(pe, {{V, 0.f, 1.f}}, nullptr, Z2, 2, st));
   const float h = (float)(dt * 0.5);
   DINO_TRY(launch_lincomb(pe, {{Z3, -h, -h}, {Z2, h, h}}, nullptr, C, 0, st));
   DINO_TRY(pe_explicit_vjp_impl(pe, Y1, C, V, st));
-  DINO_TRY(launch_apply(pe, mt.inv1, V, Z1, nullptr, st));
+  DINO_TRY(launch_apply(pe, mt.inv1, V, Z1, st));
   DINO_TRY(launch_lincomb(pe, {{V, 0.f, 1.f}}, nullptr, Z1, 2, st));
   const float c3 = (float)(dt * 0.5), c2 = (float)(dt / 6.0), c1 = (float)(dt / 3.0);
   DINO_TRY(launch_lincomb(pe, {{Z3, c3, c3}, {Z2, c2, c2}, {Z1, c1, c1}}, nullptr, C,
@@ -2635,7 +2867,7 @@ static int pe_step_vjp_impl(dino_pe* pe, const float* y, const float* out_ct,
                            {Z2, (float)(dt / 3.0), 0.f},
                            {Z1, (float)(dt / 6.0), 0.f}},
                           nullptr, Gb, 1, st));
-  DINO_TRY(launch_apply(pe, mt.L, Gb, Tt, nullptr, st));
+  DINO_TRY(launch_apply(pe, mt.L, Gb, Tt, st));
   DINO_TRY(launch_lincomb(pe,
                           {{Z1, 1.f, 1.f}, {Z2, 1.f, 1.f}, {Z3, 1.f, 1.f},
                            {V, 1.f, 1.f}, {Tt, 1.f, 0.f}},
@@ -2667,11 +2899,10 @@ static void pe_free(dino_pe* pe) {
   cudaFree(pe->d_fwd_out);
   cudaFree(pe->d_work);
   for (auto* f : pe->d_f) cudaFree(f);
-  for (auto* g : pe->d_g) cudaFree(g);
   cudaFree(pe->d_Y);
-  cudaFree(pe->d_ystar);
   cudaFree(pe->d_lm_in);
   cudaFree(pe->d_lm_out);
+  cudaFree(pe->d_lm_g0);
   cudaFree(pe->d_xbar_n);
   cudaFree(pe->d_xbar_m);
   for (auto* b : pe->d_adj) cudaFree(b);
@@ -2862,15 +3093,14 @@ static int pe_build(dino_pe* pe, const dino_pe_desc* d) {
   DINO_REQUIRE((uint64_t)pe->n_inv * IJ < (1ull << 32) && (uint64_t)pe->n_fwd * IJ < (1ull << 32),
                DINO_ERR_UNSUPPORTED, "nodal buffers must hold fewer than 2^32 values");
   DINO_CHECK_CUDA(cudaMalloc(&pe->d_aux, sizeof(float) * pe->n_aux * ML));
+  DINO_CHECK_CUDA(cudaMemset(pe->d_aux, 0, sizeof(float) * pe->n_aux * ML));
   DINO_CHECK_CUDA(cudaMalloc(&pe->d_nodal, sizeof(float) * pe->n_inv * IJ));
   DINO_CHECK_CUDA(cudaMalloc(&pe->d_fwd_in, sizeof(float) * pe->n_fwd * IJ));
   DINO_CHECK_CUDA(cudaMalloc(&pe->d_fwd_out, sizeof(float) * pe->n_fwd * ML));
   pe->work_fields = pe->n_inv > pe->n_fwd ? pe->n_inv : pe->n_fwd;
   DINO_CHECK_CUDA(cudaMalloc(&pe->d_work, sizeof(float) * (size_t)pe->work_fields * p->M * p->J));
   for (auto*& f : pe->d_f) DINO_CHECK_CUDA(cudaMalloc(&f, sizeof(float) * pe->n_state * ML));
-  for (auto*& g : pe->d_g) DINO_CHECK_CUDA(cudaMalloc(&g, sizeof(float) * pe->n_state * ML));
   DINO_CHECK_CUDA(cudaMalloc(&pe->d_Y, sizeof(float) * pe->n_state * ML));
-  DINO_CHECK_CUDA(cudaMalloc(&pe->d_ystar, sizeof(float) * pe->n_state * ML));
   pe->Cp = ceil_div(pe->mem * pe->M, kApplyCols) * kApplyCols;
   {
     const size_t lm = (size_t)pe->L * 2 * (2 * K + 1) * pe->Cp;
@@ -2878,6 +3108,8 @@ static int pe_build(dino_pe* pe, const dino_pe_desc* d) {
     DINO_CHECK_CUDA(cudaMalloc(&pe->d_lm_out, sizeof(float) * lm));
     DINO_CHECK_CUDA(cudaMemset(pe->d_lm_in, 0, sizeof(float) * lm));
     DINO_CHECK_CUDA(cudaMemset(pe->d_lm_out, 0, sizeof(float) * lm));
+    DINO_CHECK_CUDA(cudaMalloc(&pe->d_lm_g0, sizeof(float) * (lm / 2)));
+    DINO_CHECK_CUDA(cudaMemset(pe->d_lm_g0, 0, sizeof(float) * (lm / 2)));
   }
   DINO_CHECK_CUDA(cudaMalloc(&pe->d_flag, sizeof(int)));
   DINO_CHECK_CUDA(cudaDeviceSynchronize());
@@ -2999,7 +3231,7 @@ int dino_pe_implicit(dino_pe* pe, const float* state, float* out, void* stream) 
   DINO_CHECK_CUDA(cudaMemsetAsync(out, 0, sizeof(float) * pe->n_state * pe->ML, st));
   const MatEntry* m = nullptr;
   DINO_TRY(get_matrix(pe, kMatL, 0.0, nullptr, &m));
-  return launch_apply(pe, m, state, out, nullptr, st);
+  return launch_apply(pe, m, state, out, st);
 }
 
 int dino_pe_implicit_inverse(dino_pe* pe, const float* state, float* out,
@@ -3019,7 +3251,7 @@ int dino_pe_implicit_inverse(dino_pe* pe, const float* state, float* out,
                                       sizeof(float) * pe->nT * mK * pe->ML,
                                       cudaMemcpyDeviceToDevice, st));
   }
-  return launch_apply(pe, m, state, out, nullptr, st);
+  return launch_apply(pe, m, state, out, st);
 }
 
 int dino_pe_step(dino_pe* pe, float* state, double dt, const double* host_filter,
@@ -3124,7 +3356,7 @@ int dino_pe_implicit_vjp(dino_pe* pe, const float* out_ct, float* in_ct, void* s
   DINO_CHECK_CUDA(cudaMemsetAsync(in_ct, 0, sizeof(float) * pe->n_state * pe->ML, st));
   const MatEntry* m = nullptr;
   DINO_TRY(get_matrix(pe, kMatL, 0.0, nullptr, &m, true));
-  return launch_apply(pe, m, out_ct, in_ct, nullptr, st);
+  return launch_apply(pe, m, out_ct, in_ct, st);
 }
 
 int dino_pe_implicit_inverse_vjp(dino_pe* pe, const float* out_ct, float* in_ct,
@@ -3137,7 +3369,7 @@ int dino_pe_implicit_inverse_vjp(dino_pe* pe, const float* out_ct, float* in_ct,
   cudaStream_t st = (cudaStream_t)stream;
   if (out_ct != in_ct)
     DINO_TRY(launch_lincomb(pe, {{out_ct, 0.f, 1.f}}, nullptr, in_ct, 2, st));
-  return launch_apply(pe, m, out_ct, in_ct, nullptr, st);
+  return launch_apply(pe, m, out_ct, in_ct, st);
 }
 
 int dino_pe_step_vjp(dino_pe* pe, const float* state, const float* out_ct,

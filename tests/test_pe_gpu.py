@@ -389,3 +389,44 @@ def test_time_reversed_step_and_digital_filter_initialization():
   odfi = od.digital_filter_initialization(oeq, od.imex_rk_sil3, oflt, 8 * dt,
                                           8 * dt, dt)
   assert_state(dfi(to_state(st)), odfi(st), 5e-5)
+
+
+@pytest.mark.parametrize('wavenumbers,layers,members,moist,below', [
+    (5, 1, 1, False, False), (16, 9, 3, False, True), (21, 2, 1, True, True),
+    (43, 5, 2, True, False), (85, 3, 1, False, True), (85, 3, 1, False, False)])
+def test_fused_step_matches_tableau_loop(wavenumbers, layers, members, moist, below):
+  # The fused step (stage kernel, l-major implicit terms, zero column blocks
+  # skipped) against the tableau loop over explicit_terms, implicit_terms and
+  # implicit_inverse, at sizes around its 32 x 32 tiles and 128-column blocks;
+  # `below` puts values below the triangle (l < m), which transforms ignore and
+  # the other parts carry along.  Both are FP32 on the same kernels' terms:
+  # they differ by the rounding of the stage sums (at most seven terms, whose
+  # implicit part is up to ~10x the state's divergence): 5e-6 of each maximum.
+  rng = np.random.default_rng(wavenumbers)
+  g = sh.Grid.with_wavenumbers(wavenumbers)
+  coords = coordinate_systems.CoordinateSystem(
+      g, sigma_coordinates.SigmaCoordinates.equidistant(layers))
+  _, l = np.meshgrid(*g.modal_axes, indexing='ij')
+  def field(amplitude, k, mean=0.0):
+    x = amplitude * rng.standard_normal((members, k) + l.shape) / (l + 1.0) ** 1.5
+    x = x * (1.0 if below else g.mask)
+    x[..., 0, 0] += 2 * np.sqrt(np.pi) * mean
+    x = torch.as_tensor(x, device='cuda', dtype=torch.float32)
+    return x if members > 1 else x[0]
+  tr = {}
+  if moist:
+    tr = {'specific_humidity': field(1e-3, layers, 5e-3), 'tracer': field(0.3, layers, 1.0)}
+  state = pe.State(field(0.05, layers), field(0.005, layers), field(5.0, layers),
+                   field(0.01, 1, 45.0), tracers=tr)
+  orography = (rng.standard_normal(l.shape) * g.mask * 1e-5).astype(np.float32)
+  eq = pe.PrimitiveEquationsSigma(
+      np.linspace(220.0, 290.0, layers), orography, coords, units.SimUnits(),
+      humidity_key='specific_humidity' if moist else None)
+  dt = 0.05
+  filt = ti.exponential_step_filter(g, dt)
+  got = ti.step_with_filters(ti.imex_rk_sil3(eq, dt), [filt])(state)
+  want = ti.step_with_filters(ti.imex_runge_kutta(ti.SIL3_TABLEAU, eq, dt), [filt])(state)
+  leaves = lambda s: [getattr(s, k) for k in KEYS] + [s.tracers[k] for k in tr]
+  for a, b in zip(leaves(got), leaves(want)):
+    a, b = a.double(), b.double()
+    assert float((a - b).abs().max() / b.abs().max()) < 5e-6
