@@ -1974,16 +1974,28 @@ struct ApplyArgs {
   const float* ylm;   // [L][nin][Cp]
   float* olm;         // [L][R][Cp]
   int R, nin, RP, Cp;
+  int C, M;           // valid columns (member * M + row)
 };
 
 constexpr int kApplyCols = 128;
 constexpr int kApplyMaxTR = 9;
 
+// Whether the 128 columns from c0 lie below the triangle at l: all of one
+// member's rows m > l, where valid coefficients are zero.
+__device__ __forceinline__ bool cols_below_triangle(int c0, int C, int M, int l) {
+  const int last = min(c0 + kApplyCols, C) - 1;
+  return c0 / M == last / M && ((c0 % M + 1) >> 1) > l;
+}
+
 // A CTA takes one l, 128 columns and 16*TR rows of A_l: it stages A_l^T and
 // the operand rows in shared memory and each thread accumulates a TR x 8
 // register tile, columns 4 cg .. 4 cg + 3 and 64 + 4 cg .. 64 + 4 cg + 3
 // (two conflict-free float4 operand reads per k, broadcast A reads, float4
-// stores).
+// stores).  Adjacent columns share an f32x2 FMA, which halves the issue slots
+// of a kernel that filled 68 % of them with its FMA pipe 52 % busy.  Columns
+// below the triangle are zero in any state the transforms made; where such a
+// block's operand really is zero, its product is written without being formed
+// (3 of 8 blocks at TL255 with one member).
 template <int TR>
 __global__ void __launch_bounds__(256) pe_apply_kernel(ApplyArgs a) {
   constexpr int RPT = 16 * TR;
@@ -1996,45 +2008,58 @@ __global__ void __launch_bounds__(256) pe_apply_kernel(ApplyArgs a) {
   const int c0 = blockIdx.x * kApplyCols;
   const int l = blockIdx.y;
   const int r0 = blockIdx.z * RPT;
+  bool some = true;
   {
-    const float* Ag = a.A + (size_t)l * nin * a.RP + r0;
-    constexpr int Q = RPT / 4;
-    for (int e = tid; e < nin * Q; e += 256) {
-      const int k = e / Q, q = e - k * Q;
-      reinterpret_cast<float4*>(At)[e] =
-          reinterpret_cast<const float4*>(Ag + (size_t)k * a.RP)[q];
-    }
     const float* Yg = a.ylm + (size_t)l * nin * a.Cp + c0;
-    for (int e = tid; e < nin * Q4; e += 256) {
-      const int k = e / Q4, q = e - k * Q4;
-      reinterpret_cast<float4*>(Ys)[e] =
-          reinterpret_cast<const float4*>(Yg + (size_t)k * a.Cp)[q];
+    if (cols_below_triangle(c0, a.C, a.M, l)) {
+      bool mine = false;
+      for (int e = tid; e < nin * Q4; e += 256) {
+        const int k = e / Q4, q = e - k * Q4;
+        const float4 v = reinterpret_cast<const float4*>(Yg + (size_t)k * a.Cp)[q];
+        reinterpret_cast<float4*>(Ys)[e] = v;
+        mine |= v.x != 0.f || v.y != 0.f || v.z != 0.f || v.w != 0.f;
+      }
+      some = __syncthreads_or(mine);
+    } else {
+      for (int e = tid; e < nin * Q4; e += 256) {
+        const int k = e / Q4, q = e - k * Q4;
+        reinterpret_cast<float4*>(Ys)[e] =
+            reinterpret_cast<const float4*>(Yg + (size_t)k * a.Cp)[q];
+      }
+    }
+    if (some) {
+      const float* Ag = a.A + (size_t)l * nin * a.RP + r0;
+      constexpr int Q = RPT / 4;
+      for (int e = tid; e < nin * Q; e += 256) {
+        const int k = e / Q, q = e - k * Q;
+        reinterpret_cast<float4*>(At)[e] =
+            reinterpret_cast<const float4*>(Ag + (size_t)k * a.RP)[q];
+      }
     }
   }
-  __syncthreads();
   const int cg = tid & 15, rg = tid >> 4;
-  float acc[TR][8];
+  float2 acc[TR][4];
 #pragma unroll
   for (int i = 0; i < TR; ++i)
 #pragma unroll
-    for (int c = 0; c < 8; ++c) acc[i][c] = 0.f;
-  const float* ar = At + rg * TR;
-  const float4* yr = reinterpret_cast<const float4*>(Ys) + cg;
+    for (int c = 0; c < 4; ++c) acc[i][c] = make_float2(0.f, 0.f);
+  if (some) {
+    __syncthreads();
+    const float* ar = At + rg * TR;
+    const float4* yr = reinterpret_cast<const float4*>(Ys) + cg;
 #pragma unroll 2
-  for (int k = 0; k < nin; ++k) {
-    const float4 y0 = yr[k * Q4];
-    const float4 y1 = yr[k * Q4 + 16];
+    for (int k = 0; k < nin; ++k) {
+      const float4 y0 = yr[k * Q4];
+      const float4 y1 = yr[k * Q4 + 16];
+      const float2 y[4] = {make_float2(y0.x, y0.y), make_float2(y0.z, y0.w),
+                           make_float2(y1.x, y1.y), make_float2(y1.z, y1.w)};
 #pragma unroll
-    for (int i = 0; i < TR; ++i) {
-      const float av = ar[k * RPT + i];
-      acc[i][0] = fmaf(av, y0.x, acc[i][0]);
-      acc[i][1] = fmaf(av, y0.y, acc[i][1]);
-      acc[i][2] = fmaf(av, y0.z, acc[i][2]);
-      acc[i][3] = fmaf(av, y0.w, acc[i][3]);
-      acc[i][4] = fmaf(av, y1.x, acc[i][4]);
-      acc[i][5] = fmaf(av, y1.y, acc[i][5]);
-      acc[i][6] = fmaf(av, y1.z, acc[i][6]);
-      acc[i][7] = fmaf(av, y1.w, acc[i][7]);
+      for (int i = 0; i < TR; ++i) {
+        const float av = ar[k * RPT + i];
+        const float2 aa = make_float2(av, av);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[i][c] = __ffma2_rn(aa, y[c], acc[i][c]);
+      }
     }
   }
   float* og = a.olm + (size_t)l * a.R * a.Cp + c0 + cg * 4;
@@ -2043,9 +2068,10 @@ __global__ void __launch_bounds__(256) pe_apply_kernel(ApplyArgs a) {
     const int r = r0 + rg * TR + i;
     if (r < a.R) {
       float* o = og + (size_t)r * a.Cp;
-      *reinterpret_cast<float4*>(o) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+      *reinterpret_cast<float4*>(o) =
+          make_float4(acc[i][0].x, acc[i][0].y, acc[i][1].x, acc[i][1].y);
       *reinterpret_cast<float4*>(o + 64) =
-          make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
+          make_float4(acc[i][2].x, acc[i][2].y, acc[i][3].x, acc[i][3].y);
     }
   }
 }
@@ -2133,6 +2159,8 @@ static int lm_apply(dino_pe* pe, const MatEntry* m, int rows, float* olm, cudaSt
   a.nin = m->nin;
   a.RP = m->RP;
   a.Cp = pe->Cp;
+  a.C = pe->mem * pe->M;
+  a.M = pe->M;
   const int tr = apply_tr(rows);
   const int rpt = 16 * tr;
   dim3 grid(pe->Cp / kApplyCols, pe->L, ceil_div(rows, rpt));
