@@ -9,6 +9,8 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/dino_b200.h"
@@ -51,6 +53,56 @@ struct Status {
 
 // Checks the launch status of the last kernel (does not synchronize).
 int check_launch(const char* what);
+
+// Launches a kernel that may start while the one before it on the stream is
+// finishing (programmatic dependent launch): its CTAs are brought up, and do
+// what needs no earlier result, during the predecessor's last wave, which a
+// plain launch would wait out.  Every kernel launched so calls pdl_wait() on
+// every path before it touches memory that an earlier kernel writes or reads,
+// so each still sees the whole of its predecessor (and, by the predecessor's
+// own wait, of everything before it).  Grids below kPdlMinCtas launch plainly:
+// in a captured graph a programmatic edge between two short kernels costs more
+// than the tail it hides (T21 / 12 steps 517 us plainly, 551 with every launch
+// overlapped and 498 from 250 CTAs on; T85 shallow water 496, 620 and 497; T42 /
+// 24 x 16 745, 725 and 725; TL159 pair of 75 fields 96.6, 89.0 and 88.9; moist
+// TL255 / 32 x 4 11320, 11220 and 11180).
+constexpr int64_t kPdlMinCtas = 250;
+template <class... P, class... A>
+int launch_pdl(const char* what, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+               cudaStream_t st, const A&... args) {
+  static_assert(sizeof...(P) == sizeof...(A), "kernel arguments");
+  std::tuple<std::remove_cv_t<P>...> values(args...);
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = (int64_t)grid.x * grid.y * grid.z >= kPdlMinCtas ? 1 : 0;
+  const cudaError_t err = std::apply(
+      [&](auto&... v) {
+        void* ptrs[] = {static_cast<void*>(&v)...};
+        return cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(kernel), ptrs);
+      },
+      values);
+  if (err == cudaSuccess) return DINO_OK;
+  cudaGetLastError();
+  set_error(std::string("kernel launch failed (") + what + "): " + cudaGetErrorString(err));
+  return DINO_ERR_CUDA;
+}
+
+// The kernel side of launch_pdl: lets the next kernel's CTAs come up (its own
+// pdl_wait holds them until this grid has finished), and waits for the
+// previous grid's end and memory.  Both are no-ops after a plain launch.
+__device__ __forceinline__ void pdl_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 // An NVTX range over the enclosing scope, so that profilers group the
 // kernels a phase launches under the reference's names for its phases

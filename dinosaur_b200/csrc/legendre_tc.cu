@@ -804,7 +804,11 @@ legendre_tc_kernel(const __grid_constant__ CUtensorMap tBh,
   const int m = a.m0 + blockIdx.y;
   const int tile = blockIdx.x;
   const int rows = (m == 0) ? a.nf : 2 * a.nf;
-  if (tile * 128 >= rows) return;  // uniform for the CTA
+  pdl_trigger();
+  if (tile * 128 >= rows) {  // uniform for the CTA
+    pdl_wait();
+    return;
+  }
 
   const int Lm = a.L - m;
   const int n_par[2] = {(Lm + 1) >> 1, Lm >> 1};
@@ -826,8 +830,10 @@ legendre_tc_kernel(const __grid_constant__ CUtensorMap tBh,
     }
   }
   // Uniform early exits: no output column in this range.
-  if (kForward && cnt[0] == 0) return;
-  if (!kForward && lo >= a.Jh) return;
+  if ((kForward && cnt[0] == 0) || (!kForward && lo >= a.Jh)) {
+    pdl_wait();
+    return;
+  }
   const int nblocks = kblk[0] + kblk[1];
   const uint32_t tile_a = 128u * Op::kRowBytes;             // 128 rows x one K block
   const uint32_t tile_b = (uint32_t)a.Nsub * Op::kRowBytes;  // Nsub rows x one K block
@@ -857,8 +863,6 @@ legendre_tc_kernel(const __grid_constant__ CUtensorMap tBh,
       tma_load_2d(st + 2 * tile_a, &tBh, &full_bar[i], k * Op::kKB, yb);
       tma_load_2d(st + 2 * tile_a + tile_b, &tBl, &full_bar[i], k * Op::kKB, yb);
     }
-  } else if (warp >= 2) {
-    tc_prefetch_block<kForward, Op>(a, m, tile, rows, 0, threadIdx.x - 64);
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -867,6 +871,10 @@ legendre_tc_kernel(const __grid_constant__ CUtensorMap tBh,
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  // The set-up above (barriers, table tiles, TMEM) needs nothing that an
+  // earlier kernel wrote; the rows do.
+  pdl_wait();
+  if (warp >= 2) tc_prefetch_block<kForward, Op>(a, m, tile, rows, 0, threadIdx.x - 64);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -1072,9 +1080,9 @@ legendre_tc_kernel(const __grid_constant__ CUtensorMap tBh,
         }
         __syncwarp();
       }
-      // The stores have read their shared-memory source before the CTA (and
-      // its shared memory) ends; their global writes complete with the grid.
-      if (lane == 0 && nb > 0) bulk_wait_read<0>();
+      // The stores have read their source and written their rows before the
+      // CTA (and its shared memory) ends.
+      if (lane == 0 && nb > 0) bulk_wait_all();
       __syncwarp();
     } else {
       const int nchunks = (max(cnt[0], cnt[1]) + 15) / 16;
@@ -1247,13 +1255,13 @@ static void tc_set_shape(const TcTables* t, int m0, int nsub, int stages, TcArgs
 
 // One launch of the contraction in the plan's operand format.
 template <bool kForward>
-static void tc_launch(const TcTables* t, dim3 grid, size_t smem, cudaStream_t st,
-                      const CUtensorMap& bh, const CUtensorMap& bl, const CUtensorMap& o2,
-                      const CUtensorMap& o1, const TcArgs& a) {
-  if (t->tf32)
-    legendre_tc_kernel<kForward, OpTf32><<<grid, kTcThreads, smem, st>>>(bh, bl, o2, o1, a);
-  else
-    legendre_tc_kernel<kForward, OpBf16><<<grid, kTcThreads, smem, st>>>(bh, bl, o2, o1, a);
+static int tc_launch(const TcTables* t, dim3 grid, size_t smem, cudaStream_t st,
+                     const CUtensorMap& bh, const CUtensorMap& bl, const CUtensorMap& o2,
+                     const CUtensorMap& o1, const TcArgs& a) {
+  auto* kernel = t->tf32 ? legendre_tc_kernel<kForward, OpTf32>
+                         : legendre_tc_kernel<kForward, OpBf16>;
+  return launch_pdl(kForward ? "legendre_tc_forward" : "legendre_tc_inverse", kernel, grid,
+                    kTcThreads, smem, st, bh, bl, o2, o1, a);
 }
 
 template <bool kForward>
@@ -1286,8 +1294,7 @@ static int tc_time_shape(dino_plan* p, TcTables* t, const TcShape& c, int m0, in
   constexpr int kReps = 10;
   for (int r = 0; r <= kReps; ++r) {
     if (r == 1) DINO_CHECK_CUDA(cudaEventRecord(e0, 0));
-    tc_launch<kForward>(t, grid, c.smem, 0, bh, bl, o2, o1, a);
-    DINO_TRY(check_launch("legendre_tc (autotune)"));
+    DINO_TRY(tc_launch<kForward>(t, grid, c.smem, 0, bh, bl, o2, o1, a));
   }
   DINO_CHECK_CUDA(cudaEventRecord(e1, 0));
   DINO_CHECK_CUDA(cudaEventSynchronize(e1));
@@ -1563,8 +1570,7 @@ int tc_legendre_inverse(dino_plan* p, const Segs& in, float* out, int nf,
     const TcTables::Shape& sh = t->inv[gi];
     tc_set_shape(t, sh.m0, sh.Nsub, sh.stages, &a);
     dim3 grid(ceil_div(2 * nf, 128), sh.m1 - sh.m0, sh.nsplit);
-    tc_launch<false>(t, grid, sh.smem, st, sh.bh, sh.bl, o2, o1, a);
-    DINO_TRY(check_launch("legendre_tc_inverse"));
+    DINO_TRY(tc_launch<false>(t, grid, sh.smem, st, sh.bh, sh.bl, o2, o1, a));
   }
   return DINO_OK;
 }
@@ -1583,8 +1589,7 @@ int tc_legendre_forward(dino_plan* p, const float* G, float* out, int nf,
     const TcTables::Shape& sh = t->fwd[gi];
     tc_set_shape(t, sh.m0, sh.Nsub, sh.stages, &a);
     dim3 grid(ceil_div(2 * nf, 128), sh.m1 - sh.m0, sh.nsplit);
-    tc_launch<true>(t, grid, sh.smem, st, sh.bh, sh.bl, unused, unused, a);
-    DINO_TRY(check_launch("legendre_tc_forward"));
+    DINO_TRY(tc_launch<true>(t, grid, sh.smem, st, sh.bh, sh.bl, unused, unused, a));
   }
   return DINO_OK;
 }

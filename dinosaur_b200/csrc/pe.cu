@@ -222,6 +222,8 @@ struct ModalPoint {
 // Every load of a plane's four rows is issued before its first store (24 in
 // flight a thread), because a store that might alias stops the loads behind it.
 __global__ void __launch_bounds__(kModalTX * kModalTY, 3) pe_prep_kernel(PrepArgs a, int ppt) {
+  pdl_trigger();
+  pdl_wait();
   const int l0 = blockIdx.x * kTile, row0 = blockIdx.y * kTile;
   // The inverse transform does not read the aux planes below the triangle
   // (they keep the zeros of their allocation).
@@ -352,6 +354,8 @@ constexpr int kNodalCols = 32, kNodalMaxChunks = 2;
 template <bool kTracers, int V>
 __global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
     pe_nodal_kernel(NodalArgs a) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ float4 s_lev[];  // [K][kLevPack / 4]
   __shared__ float s_e[kNodalMaxChunks][kNodalCols * V];
   __shared__ float s_f[kNodalMaxChunks][kNodalCols * V];
@@ -769,6 +773,8 @@ struct HybridArgs {
 //     terms (:2124-2224, whose integrands are the same D_k) and the tracers.
 // Outputs use the planes of pe_nodal_kernel, so the modal post-pass is shared.
 __global__ void __launch_bounds__(kHybThreads) pe_nodal_hybrid_kernel(HybridArgs a) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ float s_hyb[];
   const int K = a.K;
   for (int i = threadIdx.x; i < K * kHybPack + kHybTail; i += blockDim.x) s_hyb[i] = a.lev[i];
@@ -1059,6 +1065,8 @@ struct StageArgs {
 template <int kNf>
 __global__ void __launch_bounds__(kModalTX * kModalTY, 3)
     pe_post_kernel(PostArgs a, StageArgs s, int ppt) {
+  pdl_trigger();
+  pdl_wait();
   constexpr bool kStage = kNf >= 0;
   constexpr int kF = kNf > 0 ? kNf : 1;  // array sizes
   constexpr int kPair = 2;               // rows whose loads are in flight together
@@ -1314,6 +1322,8 @@ struct ModalNbrT {
 };
 
 __global__ void __launch_bounds__(kModalTX * kModalTY) pe_post_adjoint_kernel(PostAdjArgs a, int ppt) {
+  pdl_trigger();
+  pdl_wait();
   const int l = blockIdx.x * kModalTX + threadIdx.x;
   const int row = blockIdx.y * kModalTY + threadIdx.y;
   if (l >= a.L || row >= a.M) return;
@@ -1384,6 +1394,8 @@ struct NodalAdjArgs {
 // pe_nodal_kernel); plane offsets are 32-bit (the nodal and forward-input
 // buffers hold fewer than 2^32 floats, checked on the host).
 __global__ void __launch_bounds__(128, 5) pe_nodal_adjoint_kernel(NodalAdjArgs A) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ float4 s_lev[];  // [K][kLevPack / 4]
   const NodalArgs& a = A.f;
   const int K = a.K;
@@ -1665,6 +1677,8 @@ struct PrepAdjArgs {
 };
 
 __global__ void __launch_bounds__(kModalTX * kModalTY) pe_prep_adjoint_kernel(PrepAdjArgs a, int ppt) {
+  pdl_trigger();
+  pdl_wait();
   const int l = blockIdx.x * kModalTX + threadIdx.x;
   const int row = blockIdx.y * kModalTY + threadIdx.y;
   if (l >= a.L || row >= a.M) return;
@@ -1723,6 +1737,8 @@ struct LinCombArgs {
 };
 
 __global__ void pe_lincomb_kernel(LinCombArgs a) {
+  pdl_trigger();
+  pdl_wait();
   const int plane = blockIdx.y;
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= a.ML) return;
@@ -1914,6 +1930,8 @@ __device__ __forceinline__ size_t stacked_plane(const LmArgs& a, int i, int mb) 
 // threads): blockIdx.y enumerates (member, row tile), so a tile never spans
 // two members and the column c = member * M + row needs no division.
 __global__ void __launch_bounds__(256) pe_lm_gather_kernel(LmArgs a) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float tile[32][33];
   const int k = blockIdx.z;
   const int row_tiles = (a.M + 31) / 32;
@@ -1944,6 +1962,8 @@ __global__ void __launch_bounds__(256) pe_lm_gather_kernel(LmArgs a) {
 // Row r < n of the l-major product back into the state layout, tiled like the
 // gather.
 __global__ void __launch_bounds__(256) pe_lm_scatter_kernel(LmArgs a) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float tile[32][33];
   const int r = blockIdx.z;
   const int row_tiles = (a.M + 31) / 32;
@@ -1998,6 +2018,8 @@ __device__ __forceinline__ bool cols_below_triangle(int c0, int C, int M, int l)
 // (3 of 8 blocks at TL255 with one member).
 template <int TR>
 __global__ void __launch_bounds__(256) pe_apply_kernel(ApplyArgs a) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int RPT = 16 * TR;
   constexpr int Q4 = kApplyCols / 4;  // float4 per operand row
   extern __shared__ __align__(16) float smem[];
@@ -2113,8 +2135,8 @@ static int prepare_apply() {
 }
 
 template <int TR>
-static void apply_launch(dim3 grid, size_t smem, cudaStream_t st, const ApplyArgs& a) {
-  pe_apply_kernel<TR><<<grid, 256, smem, st>>>(a);
+static int apply_launch(dim3 grid, size_t smem, cudaStream_t st, const ApplyArgs& a) {
+  return launch_pdl("pe_apply", pe_apply_kernel<TR>, grid, 256, smem, st, a);
 }
 
 static LmArgs lm_args(dino_pe* pe) {
@@ -2145,8 +2167,7 @@ static int lm_gather(dino_pe* pe, int nk, const float* src, cudaStream_t st,
   g.lm = pe->d_lm_in;
   g.nk = nk;
   const dim3 grid(ceil_div(pe->L, 32), ceil_div(pe->M, 32) * pe->mem, nk);
-  pe_lm_gather_kernel<<<grid, 256, 0, st>>>(g);
-  return check_launch("pe_lm_gather");
+  return launch_pdl("pe_lm_gather", pe_lm_gather_kernel, grid, 256, 0, st, g);
 }
 
 // The first `rows` rows of the per-l products of m with pe->d_lm_in.
@@ -2166,17 +2187,16 @@ static int lm_apply(dino_pe* pe, const MatEntry* m, int rows, float* olm, cudaSt
   dim3 grid(pe->Cp / kApplyCols, pe->L, ceil_div(rows, rpt));
   const size_t smem = apply_smem(a.nin, tr);
   switch (tr) {
-    case 1: apply_launch<1>(grid, smem, st, a); break;
-    case 2: apply_launch<2>(grid, smem, st, a); break;
-    case 3: apply_launch<3>(grid, smem, st, a); break;
-    case 4: apply_launch<4>(grid, smem, st, a); break;
-    case 5: apply_launch<5>(grid, smem, st, a); break;
-    case 6: apply_launch<6>(grid, smem, st, a); break;
-    case 7: apply_launch<7>(grid, smem, st, a); break;
-    case 8: apply_launch<8>(grid, smem, st, a); break;
-    default: apply_launch<9>(grid, smem, st, a); break;
+    case 1: return apply_launch<1>(grid, smem, st, a);
+    case 2: return apply_launch<2>(grid, smem, st, a);
+    case 3: return apply_launch<3>(grid, smem, st, a);
+    case 4: return apply_launch<4>(grid, smem, st, a);
+    case 5: return apply_launch<5>(grid, smem, st, a);
+    case 6: return apply_launch<6>(grid, smem, st, a);
+    case 7: return apply_launch<7>(grid, smem, st, a);
+    case 8: return apply_launch<8>(grid, smem, st, a);
+    default: return apply_launch<9>(grid, smem, st, a);
   }
-  return check_launch("pe_apply");
 }
 
 // The first n of the nk rows per l of pe->d_lm_out into out's implicit planes.
@@ -2186,8 +2206,7 @@ static int lm_scatter(dino_pe* pe, int nk, float* out, cudaStream_t st) {
   g.lm = pe->d_lm_out;
   g.nk = nk;
   const dim3 grid(ceil_div(pe->L, 32), ceil_div(pe->M, 32) * pe->mem, g.n);
-  pe_lm_scatter_kernel<<<grid, 256, 0, st>>>(g);
-  return check_launch("pe_lm_scatter");
+  return launch_pdl("pe_lm_scatter", pe_lm_scatter_kernel, grid, 256, 0, st, g);
 }
 
 // out's implicit planes = the product of m with those of src (and src2).
@@ -2356,8 +2375,7 @@ static int pe_nodal_inputs(dino_pe* pe, const float* state, cudaStream_t st) {
     a.inv_radius = (float)(1.0 / p->radius);
     int ppt = 0;
     const dim3 grid = tile_grid(pe, &ppt);
-    pe_prep_kernel<<<grid, dim3(kModalTX, kModalTY), 0, st>>>(a, ppt);
-    DINO_TRY(check_launch("pe_prep"));
+    DINO_TRY(launch_pdl("pe_prep", pe_prep_kernel, grid, dim3(kModalTX, kModalTY), 0, st, a, ppt));
   }
   // 2. inverse SHT of [state kinds][aux][ln ps (Held-Suarez)]
   {
@@ -2462,8 +2480,7 @@ static int launch_nodal_hybrid(dino_pe* pe, const float* state, cudaStream_t st)
   const dim3 grid(ceil_div((int)pe->IJ, kHybThreads), pe->mem);
   const size_t smem = sizeof(float) * ((size_t)K * kHybPack + kHybTail +
                                        (size_t)(K + 1) * kHybThreads);
-  pe_nodal_hybrid_kernel<<<grid, kHybThreads, smem, st>>>(a);
-  return check_launch("pe_nodal_hybrid");
+  return launch_pdl("pe_nodal_hybrid", pe_nodal_hybrid_kernel, grid, kHybThreads, smem, st, a);
 }
 static int launch_nodal(dino_pe* pe, const float* state, cudaStream_t st) {
   if (pe->hybrid) return launch_nodal_hybrid(pe, state, st);
@@ -2472,13 +2489,9 @@ static int launch_nodal(dino_pe* pe, const float* state, cudaStream_t st) {
   const dim3 grid(ceil_div((int)(pe->IJ / V), kNodalCols), pe->mem);
   const dim3 block(kNodalCols, nodal_chunks(pe));
   const size_t smem = nodal_smem(pe->K);
-  if (pe->nT > 0)
-    pe_nodal_kernel<true, 1><<<grid, block, smem, st>>>(a);
-  else if (V == 2)
-    pe_nodal_kernel<false, 2><<<grid, block, smem, st>>>(a);
-  else
-    pe_nodal_kernel<false, 1><<<grid, block, smem, st>>>(a);
-  return check_launch("pe_nodal");
+  auto* kernel = pe->nT > 0 ? pe_nodal_kernel<true, 1>
+                            : V == 2 ? pe_nodal_kernel<false, 2> : pe_nodal_kernel<false, 1>;
+  return launch_pdl("pe_nodal", kernel, grid, block, smem, st, a);
 }
 
 static NodalArgs make_nodal_args(dino_pe* pe) {
@@ -2591,9 +2604,8 @@ static int pe_explicit_impl(dino_pe* pe, const float* state, float* tend, cudaSt
   DINO_TRY(pe_explicit_products(pe, state, st));
   int ppt = 0;
   const dim3 grid = tile_grid(pe, &ppt);
-  pe_post_kernel<-1><<<grid, dim3(kModalTX, kModalTY), 0, st>>>(make_post_args(pe, tend),
-                                                                StageArgs{}, ppt);
-  return check_launch("pe_post");
+  return launch_pdl("pe_post", pe_post_kernel<-1>, grid, dim3(kModalTX, kModalTY), 0, st,
+                    make_post_args(pe, tend), StageArgs{}, ppt);
 }
 
 struct Term {
@@ -2634,13 +2646,8 @@ static int launch_stage(dino_pe* pe, const float* y0, std::initializer_list<Term
   const PostArgs a = make_post_args(pe, keep_f);
   const dim3 block(kModalTX, kModalTY);
   // The stage with two earlier f_j is also the one with two g_j.
-  if (s.nf == 0)
-    pe_post_kernel<0><<<grid, block, 0, st>>>(a, s, ppt);
-  else if (s.nf == 1)
-    pe_post_kernel<1><<<grid, block, 0, st>>>(a, s, ppt);
-  else
-    pe_post_kernel<2><<<grid, block, 0, st>>>(a, s, ppt);
-  return check_launch("pe_stage");
+  auto* kernel = s.nf == 0 ? pe_post_kernel<0> : s.nf == 1 ? pe_post_kernel<1> : pe_post_kernel<2>;
+  return launch_pdl("pe_stage", kernel, grid, block, 0, st, a, s, ppt);
 }
 
 // One filtered imex_rk_sil3 step in place (time_integration.py:329-405 with
@@ -2758,8 +2765,8 @@ static int pe_explicit_vjp_impl(dino_pe* pe, const float* state, const float* tb
     a.inv_radius = (float)(1.0 / p->radius);
     int ppt = 0;
     const dim3 grid = modal_grid(pe, &ppt);
-    pe_post_adjoint_kernel<<<grid, dim3(kModalTX, kModalTY), 0, st>>>(a, ppt);
-    DINO_TRY(check_launch("pe_post_adjoint"));
+    DINO_TRY(launch_pdl("pe_post_adjoint", pe_post_adjoint_kernel, grid,
+                        dim3(kModalTX, kModalTY), 0, st, a, ppt));
   }
   DINO_TRY(sht_forward_adjoint_to(p, pe->d_fwd_out, pe->d_fwd_in, pe->n_fwd,
                                   pe->d_work, pe->work_fields, st));
@@ -2769,8 +2776,8 @@ static int pe_explicit_vjp_impl(dino_pe* pe, const float* state, const float* tb
     a.fbar = pe->d_fwd_in;
     a.xbar = pe->d_xbar_n;
     dim3 grid(ceil_div((int)pe->IJ, 128), mem);
-    pe_nodal_adjoint_kernel<<<grid, 128, nodal_smem(K), st>>>(a);
-    DINO_TRY(check_launch("pe_nodal_adjoint"));
+    DINO_TRY(launch_pdl("pe_nodal_adjoint", pe_nodal_adjoint_kernel, grid, 128, nodal_smem(K), st,
+                        a));
   }
   DINO_TRY(sht_inverse_adjoint_to(p, pe->d_xbar_n, pe->d_xbar_m, pe->n_inv,
                                   pe->d_work, pe->work_fields, st));
@@ -2801,8 +2808,8 @@ static int pe_explicit_vjp_impl(dino_pe* pe, const float* state, const float* tb
     a.inv_radius = (float)(1.0 / p->radius);
     int ppt = 0;
     const dim3 grid = modal_grid(pe, &ppt);
-    pe_prep_adjoint_kernel<<<grid, dim3(kModalTX, kModalTY), 0, st>>>(a, ppt);
-    DINO_TRY(check_launch("pe_prep_adjoint"));
+    DINO_TRY(launch_pdl("pe_prep_adjoint", pe_prep_adjoint_kernel, grid,
+                        dim3(kModalTX, kModalTY), 0, st, a, ppt));
   }
   return DINO_OK;
 }
@@ -2829,8 +2836,7 @@ static int launch_lincomb(dino_pe* pe, std::initializer_list<LinTerm> terms,
   a.only = only;
   a.ML = pe->ML;
   dim3 grid(ceil_div((int)pe->ML, 256), pe->n_state);
-  pe_lincomb_kernel<<<grid, 256, 0, st>>>(a);
-  return check_launch("pe_lincomb");
+  return launch_pdl("pe_lincomb", pe_lincomb_kernel, grid, 256, 0, st, a);
 }
 
 struct StepMatsT {

@@ -51,6 +51,8 @@ __global__ void __launch_bounds__(kLegThreads)
 legendre_inverse_simt(Segs in, float* __restrict__ out, int B, int M, int L,
                       int J, int Jh, const float* __restrict__ ptab,
                       const int64_t* __restrict__ ptab_off) {
+  pdl_trigger();
+  pdl_wait();
   const int m = blockIdx.z;
   const int rows = (m == 0) ? B : 2 * B;
   const int r0 = blockIdx.y * kLegTB;
@@ -184,6 +186,8 @@ legendre_forward_simt(const float* __restrict__ G, float* __restrict__ out,
                       int B, int M, int L, int J, int Jh,
                       const float* __restrict__ ptab,
                       const int64_t* __restrict__ ptab_off) {
+  pdl_trigger();
+  pdl_wait();
   const int m = blockIdx.z;
   const int rows = (m == 0) ? B : 2 * B;
   const int r0 = blockIdx.y * kLegTB;
@@ -338,9 +342,8 @@ int legendre_inverse_fp32(dino_plan* p, const Segs& in, float* out, int nf,
                           cudaStream_t st) {
   NvtxRange range("inv_legendre");
   dim3 grid(ceil_div(p->Jh, kLegTN), ceil_div(2 * nf, kLegTB), p->lw);
-  legendre_inverse_simt<<<grid, kLegThreads, 0, st>>>(
-      in, out, nf, p->M, p->L, p->J, p->Jh, p->d_ptab, p->d_ptab_off);
-  return check_launch("legendre_inverse_simt");
+  return launch_pdl("legendre_inverse_simt", legendre_inverse_simt, grid, kLegThreads, 0, st, in,
+                    out, nf, p->M, p->L, p->J, p->Jh, p->d_ptab, p->d_ptab_off);
 }
 
 int legendre_inverse(dino_plan* p, const Segs& in, float* out, int nf,
@@ -349,9 +352,8 @@ int legendre_inverse(dino_plan* p, const Segs& in, float* out, int nf,
   if (p->precision != DINO_PREC_FP32 && !tc_use_simt(p, false))
     return tc_legendre_inverse(p, in, out, nf, st);
   dim3 grid(ceil_div(p->Jh, kLegTN), ceil_div(2 * nf, kLegTB), p->lw);
-  legendre_inverse_simt<<<grid, kLegThreads, 0, st>>>(
-      in, out, nf, p->M, p->L, p->J, p->Jh, p->d_ptab, p->d_ptab_off);
-  return check_launch("legendre_inverse_simt");
+  return launch_pdl("legendre_inverse_simt", legendre_inverse_simt, grid, kLegThreads, 0, st, in,
+                    out, nf, p->M, p->L, p->J, p->Jh, p->d_ptab, p->d_ptab_off);
 }
 
 int legendre_forward(dino_plan* p, const float* G, float* out, int nf,
@@ -367,14 +369,13 @@ int legendre_forward_fp32(dino_plan* p, const float* G, float* out, int nf,
                           cudaStream_t st) {
   if (p->L > 64) {
     dim3 grid(ceil_div(p->L, 64), ceil_div(2 * nf, kLegTB), p->lw);
-    legendre_forward_simt<64><<<grid, kLegThreads, 0, st>>>(
-        G, out, nf, p->M, p->L, p->J, p->Jh, p->d_ptab, p->d_ptab_off);
+    return launch_pdl("legendre_forward_simt", legendre_forward_simt<64>, grid, kLegThreads, 0,
+                      st, G, out, nf, p->M, p->L, p->J, p->Jh, p->d_ptab, p->d_ptab_off);
   } else {
     dim3 grid(ceil_div(p->L, 32), ceil_div(2 * nf, kLegTB), p->lw);
-    legendre_forward_simt<32><<<grid, kLegThreads, 0, st>>>(
-        G, out, nf, p->M, p->L, p->J, p->Jh, p->d_ptab, p->d_ptab_off);
+    return launch_pdl("legendre_forward_simt", legendre_forward_simt<32>, grid, kLegThreads, 0,
+                      st, G, out, nf, p->M, p->L, p->J, p->Jh, p->d_ptab, p->d_ptab_off);
   }
-  return check_launch("legendre_forward_simt");
 }
 
 // ---------------------------------------------------------------------------
@@ -752,6 +753,7 @@ rfft_inverse_kernel(const float* __restrict__ F, float* __restrict__ out,
                     int M, int lw, int J, const float2* __restrict__ tw_n,
                     const float2* __restrict__ tw_i,
                     const float* __restrict__ wq) {
+  pdl_trigger();
   constexpr int T = FftCfg<N>::threads, P = FftCfg<N>::pairs;
   extern __shared__ float4 sm[];
   float4* S = sm;
@@ -764,6 +766,7 @@ rfft_inverse_kernel(const float* __restrict__ F, float* __restrict__ out,
     const float2 w = tw_n[t];
     tw[t] = make_float4(w.x, w.x, w.y, w.y);
   }
+  pdl_wait();
   const float* Fb = F + (size_t)b * M * J + col;
   const float inv_sqrt_2pi = 0.3989422804014327f;
   const float half_inv_sqrt_pi = 0.28209479177387814f;
@@ -836,6 +839,7 @@ rfft_forward_kernel(const float* __restrict__ x, float* __restrict__ F, int M,
                     int lw, int J, const float2* __restrict__ tw_n,
                     const float2* __restrict__ tw_i,
                     const float* __restrict__ wq) {
+  pdl_trigger();
   constexpr int T = FftCfg<N>::threads, P = FftCfg<N>::pairs;
   extern __shared__ float4 sm[];
   float4* S = sm;
@@ -848,6 +852,7 @@ rfft_forward_kernel(const float* __restrict__ x, float* __restrict__ F, int M,
     const float2 w = tw_n[t];
     tw[t] = make_float4(w.x, w.x, -w.y, -w.y);
   }
+  pdl_wait();
   const float* xb = x + (size_t)b * (2 * N) * J + col;
   auto first = [xb, J, cols](int n) -> cpair {
     const float* g = xb + (size_t)(2 * n) * J;
@@ -902,6 +907,8 @@ __global__ void dft_inverse_kernel(const float* __restrict__ F,
                                    float* __restrict__ out, int M, int I, int J,
                                    const float* __restrict__ f,
                                    const float* __restrict__ wq) {
+  pdl_trigger();
+  pdl_wait();
   int j = blockIdx.x * 32 + threadIdx.x;
   int i = blockIdx.y * 8 + threadIdx.y;
   int b = blockIdx.z;
@@ -918,6 +925,8 @@ __global__ void dft_forward_kernel(const float* __restrict__ x,
                                    float* __restrict__ F, int M, int I, int J,
                                    const float* __restrict__ f,
                                    const float* __restrict__ wq) {
+  pdl_trigger();
+  pdl_wait();
   int j = blockIdx.x * 32 + threadIdx.x;
   int r = blockIdx.y * 8 + threadIdx.y;
   int b = blockIdx.z;
@@ -958,8 +967,8 @@ static int launch_rfft(dino_plan* p, const float* in, float* out, int nf,
                    (reinterpret_cast<uintptr_t>(out) & 7) == 0;
   auto* kernel = inverse ? (vec ? rfft_inverse_kernel<N, true> : rfft_inverse_kernel<N, false>)
                          : (vec ? rfft_forward_kernel<N, true> : rfft_forward_kernel<N, false>);
-  kernel<<<grid, T, smem, st>>>(in, out, p->M, p->lw, p->J, p->d_tw_n, p->d_tw_i, wq);
-  return check_launch(inverse ? "rfft_inverse" : "rfft_forward");
+  return launch_pdl(inverse ? "rfft_inverse" : "rfft_forward", kernel, grid, T, smem, st, in, out,
+                    p->M, p->lw, p->J, p->d_tw_n, p->d_tw_i, wq);
 }
 
 static int rfft_dispatch_n(int n, dino_plan* p, const float* in, float* out,
@@ -1001,9 +1010,8 @@ int fourier_inverse(dino_plan* p, const float* F, float* nodal, int nf,
   const float* wq = weighted_adjoint ? p->d_wq : nullptr;
   if (p->fft) return rfft_dispatch(p, F, nodal, nf, true, wq, st);
   dim3 grid(ceil_div(p->J, 32), ceil_div(p->I, 8), nf);
-  dft_inverse_kernel<<<grid, dim3(32, 8), 0, st>>>(F, nodal, p->M, p->I, p->J,
-                                                    p->d_fbasis, wq);
-  return check_launch("dft_inverse");
+  return launch_pdl("dft_inverse", dft_inverse_kernel, grid, dim3(32, 8), 0, st, F, nodal, p->M,
+                    p->I, p->J, p->d_fbasis, wq);
 }
 
 int fourier_forward(dino_plan* p, const float* nodal, float* F, int nf,
@@ -1012,9 +1020,8 @@ int fourier_forward(dino_plan* p, const float* nodal, float* F, int nf,
   const float* wq = weighted ? p->d_wq : nullptr;
   if (p->fft) return rfft_dispatch(p, nodal, F, nf, false, wq, st);
   dim3 grid(ceil_div(p->J, 32), ceil_div(p->M, 8), nf);
-  dft_forward_kernel<<<grid, dim3(32, 8), 0, st>>>(nodal, F, p->M, p->I, p->J,
-                                                    p->d_fbasis, wq);
-  return check_launch("dft_forward");
+  return launch_pdl("dft_forward", dft_forward_kernel, grid, dim3(32, 8), 0, st, nodal, F, p->M,
+                    p->I, p->J, p->d_fbasis, wq);
 }
 
 // ---------------------------------------------------------------------------

@@ -66,6 +66,8 @@ struct SwePrepArgs {
 // (spherical_harmonic.py:1164-1178) and clip_wavenumbers of vorticity and
 // potential before their inverse transforms (shallow_water.py:60-62).
 __global__ void swe_prep_kernel(SwePrepArgs a) {
+  pdl_trigger();
+  pdl_wait();
   const size_t ML = (size_t)a.M * a.L;
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= ML) return;
@@ -102,6 +104,8 @@ struct SweNodalArgs {
 // shallow_water.py:170-177: b = u (zeta + f) sec^2, g = u phi sec^2,
 // e = |u|^2 sec^2 / 2 on the nodal grid.
 __global__ void swe_nodal_kernel(SweNodalArgs a) {
+  pdl_trigger();
+  pdl_wait();
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= a.IJ) return;
   const size_t plane = blockIdx.y;
@@ -164,6 +168,8 @@ __device__ __forceinline__ void swe_tendency(const SwePostArgs& a, int mb, int k
 }
 
 __global__ void swe_post_kernel(SwePostArgs a) {
+  pdl_trigger();
+  pdl_wait();
   const size_t ML = (size_t)a.M * a.L;
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= ML) return;
@@ -196,6 +202,8 @@ struct SweStageArgs {
 
 template <int kStage>
 __global__ void swe_stage_kernel(SwePostArgs a, SweStageArgs s) {
+  pdl_trigger();
+  pdl_wait();
   const size_t ML = (size_t)a.M * a.L;
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= ML) return;
@@ -254,6 +262,8 @@ struct SweImplicitArgs {
 
 // shallow_water.py:207-230, elementwise per (layer, m, l).
 __global__ void swe_implicit_kernel(SweImplicitArgs a) {
+  pdl_trigger();
+  pdl_wait();
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= a.ML) return;
   const int l = idx % a.L;
@@ -347,16 +357,14 @@ int swe_products(dino_swe* s, const float* state, cudaStream_t st) {
     SwePrepArgs a{state, s->d_aux, K, mem, s->M, s->L, p->lw, p->d_deriv, p->d_invlap,
                   (float)(1.0 / p->radius)};
     dim3 grid(ceil_div((int)s->ML, 256), K, mem);
-    swe_prep_kernel<<<grid, 256, 0, st>>>(a);
-    DINO_TRY(check_launch("swe_prep"));
+    DINO_TRY(launch_pdl("swe_prep", swe_prep_kernel, grid, 256, 0, st, a));
   }
   DINO_TRY(sht_inverse_segs(p, one_seg(s->d_aux, 4 * mK), s->d_nodal, 4 * mK, s->d_work,
                             s->work_fields, st));
   {
     SweNodalArgs a{s->d_nodal, s->d_fwd_in, s->J, s->IJ, (size_t)mK, s->d_lat};
     dim3 grid(ceil_div((int)s->IJ, 256), mK);
-    swe_nodal_kernel<<<grid, 256, 0, st>>>(a);
-    DINO_TRY(check_launch("swe_nodal"));
+    DINO_TRY(launch_pdl("swe_nodal", swe_nodal_kernel, grid, 256, 0, st, a));
   }
   return sht_forward_to(p, s->d_fwd_in, s->d_fwd_out, 5 * mK, s->d_work, s->work_fields, st);
 }
@@ -369,8 +377,7 @@ SwePostArgs post_args(dino_swe* s, const float* state, float* tend) {
 int swe_explicit_impl(dino_swe* s, const float* state, float* tend, cudaStream_t st) {
   DINO_TRY(swe_products(s, state, st));
   dim3 grid(ceil_div((int)s->ML, 256), s->K, s->mem);
-  swe_post_kernel<<<grid, 256, 0, st>>>(post_args(s, state, tend));
-  return check_launch("swe_post");
+  return launch_pdl("swe_post", swe_post_kernel, grid, 256, 0, st, post_args(s, state, tend));
 }
 
 // One filtered SIL3 step of s->d_y in place.
@@ -385,15 +392,15 @@ int swe_step_once(dino_swe* s, double dt, const float* filter, cudaStream_t st) 
   a.out = s->d_Y[0];
   a.cf = (float)(dt / 3);
   a.cg = a.eta = (float)(dt / 6);
-  swe_stage_kernel<1><<<grid, 256, 0, st>>>(post_args(s, s->d_y, s->d_f[0]), a);
-  DINO_TRY(check_launch("swe_stage"));
+  DINO_TRY(launch_pdl("swe_stage", swe_stage_kernel<1>, grid, 256, 0, st,
+                      post_args(s, s->d_y, s->d_f[0]), a));
   DINO_TRY(swe_products(s, s->d_Y[0], st));
   a.out = s->d_Y[1];
   a.c0 = (float)(dt / 6);
   a.cf = (float)(dt / 2);
   a.cg = a.eta = (float)(dt / 3);
-  swe_stage_kernel<2><<<grid, 256, 0, st>>>(post_args(s, s->d_Y[0], s->d_f[1]), a);
-  DINO_TRY(check_launch("swe_stage"));
+  DINO_TRY(launch_pdl("swe_stage", swe_stage_kernel<2>, grid, 256, 0, st,
+                      post_args(s, s->d_Y[0], s->d_f[1]), a));
   DINO_TRY(swe_products(s, s->d_Y[1], st));
   a.out = s->d_y;
   a.filter = filter;
@@ -402,8 +409,8 @@ int swe_step_once(dino_swe* s, double dt, const float* filter, cudaStream_t st) 
   a.cf = (float)dt;
   a.cg = (float)(3 * dt / 8);
   a.eta = (float)(dt / 4);
-  swe_stage_kernel<3><<<grid, 256, 0, st>>>(post_args(s, s->d_Y[1], nullptr), a);
-  return check_launch("swe_stage");
+  return launch_pdl("swe_stage", swe_stage_kernel<3>, grid, 256, 0, st,
+                    post_args(s, s->d_Y[1], nullptr), a);
 }
 
 int swe_step_impl(dino_swe* s, float* state, double dt, const double* host_filter, int n_steps,
@@ -465,8 +472,7 @@ int swe_implicit_impl(dino_swe* s, const float* in, float* out, int mode, double
   SweImplicitArgs a{in, out, s->d_phiref, s->plan->d_lap, (float)eta, mode, s->K, s->mem,
                     s->L, s->ML};
   dim3 grid(ceil_div((int)s->ML, 256), s->K, s->mem);
-  swe_implicit_kernel<<<grid, 256, 0, st>>>(a);
-  return check_launch("swe_implicit");
+  return launch_pdl("swe_implicit", swe_implicit_kernel, grid, 256, 0, st, a);
 }
 
 }  // namespace

@@ -1,0 +1,95 @@
+"""Dependent launches that overlap: back-to-back calls give the bits of calls
+that are waited for.
+
+Kernels of large grids start while their predecessor is finishing, so a missing
+wait would let one read or overwrite what the other still uses.  Transforms,
+operators and steps run in a row on alternating inputs, without any
+synchronisation, on grids with one and with several chunks per transform and
+grids below and above the size from which launches overlap; every result must
+equal, bit for bit, the one of a call that was waited for.
+"""
+
+import functools
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from dinosaur_b200 import coordinate_systems  # noqa: E402
+from dinosaur_b200 import primitive_equations as pe  # noqa: E402
+from dinosaur_b200 import sigma_coordinates  # noqa: E402
+from dinosaur_b200 import spherical_harmonic as sh  # noqa: E402
+from dinosaur_b200 import time_integration as ti  # noqa: E402
+from dinosaur_b200 import units  # noqa: E402
+
+
+def grid_of(name, precision):
+  impl = functools.partial(sh.CudaSphericalHarmonics, precision=precision)
+  return getattr(sh.Grid, name)(spherical_harmonics_impl=impl)
+
+
+def field(grid, lead, power, seed):
+  rng = np.random.default_rng(seed)
+  _, l = np.meshgrid(*grid.modal_axes, indexing='ij')
+  x = rng.standard_normal(lead + l.shape) * grid.mask / (l + 1.0) ** power
+  return torch.as_tensor(x, device='cuda', dtype=torch.float32)
+
+
+@pytest.mark.parametrize('name,fields,precision', [
+    ('T21', 3, 'fp32'), ('TL95', 70, 'fp32'), ('T85', 150, 'bf16x3'),
+    ('TL255', 130, 'bf16x3'), ('TL127', 40, 'tf32x3')])
+def test_transforms_in_a_row(name, fields, precision):
+  g = grid_of(name, precision)
+  xs = [field(g, (fields,), 1.5, s) for s in (0, 1)]
+  def chain(x):
+    n = g.to_nodal(x)
+    m = g.to_modal(n)
+    return n, m, g.laplacian(m), g.to_nodal(g.d_dlon(m))
+  want = []
+  for x in xs:
+    out = chain(x)
+    torch.cuda.synchronize()
+    want.append([t.clone() for t in out])
+  torch.cuda.synchronize()
+  got = [chain(xs[i % 2]) for i in range(8)]
+  torch.cuda.synchronize()
+  for i, out in enumerate(got):
+    for a, b in zip(out, want[i % 2]):
+      assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize('name,layers,members', [('T21', 5, 1), ('T42', 12, 6), ('TL127', 6, 1)])
+def test_steps_and_gradients_in_a_row(name, layers, members):
+  g = grid_of(name, 'fp32')
+  coords = coordinate_systems.CoordinateSystem(
+      g, sigma_coordinates.SigmaCoordinates.equidistant(layers))
+  eq = pe.PrimitiveEquationsSigma(np.linspace(220.0, 290.0, layers),
+                                  field(g, (), 2.0, 9).cpu().numpy() * 1e-4, coords,
+                                  units.SimUnits())
+  lead = (members,) if members > 1 else ()
+  def state(s):
+    lnps = 0.02 * field(g, lead + (1,), 2.0, s + 3)
+    lnps[..., 0, 0] += 2 * np.sqrt(np.pi) * 45.0
+    return pe.State(0.05 * field(g, lead + (layers,), 1.0, s),
+                    0.005 * field(g, lead + (layers,), 1.0, s + 1),
+                    5.0 * field(g, lead + (layers,), 1.5, s + 2), lnps)
+  step = ti.repeated(ti.imex_rk_sil3(eq, 0.05), 2)
+  leaves = lambda s: [s.vorticity, s.divergence, s.temperature_variation,
+                      s.log_surface_pressure]
+  def run(s):
+    xs = [x.detach().clone().requires_grad_(True) for x in leaves(s)]
+    out = leaves(step(pe.State(*xs)))
+    sum(o.square().sum() for o in out).backward()
+    return leaves(step(s)) + [o.detach() for o in out] + [x.grad for x in xs]
+  states = [state(10), state(20)]
+  want = []
+  for s in states:
+    want.append([t.clone() for t in run(s)])
+    torch.cuda.synchronize()
+  got = [run(states[i % 2]) for i in range(4)]
+  torch.cuda.synchronize()
+  for i, out in enumerate(got):
+    for a, b in zip(out, want[i % 2]):
+      assert torch.equal(a, b)
