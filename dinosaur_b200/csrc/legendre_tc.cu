@@ -542,13 +542,12 @@ __device__ __forceinline__ void tc_seq(int i, int kb1, int& k, int& p) {
 // B = Op::kKB (K entries per block) and C = Op::kChunk (per 16-byte chunk):
 //   inverse: A_p[r][kk] = x[b][row][m + 2 (B k + kk) + p]  (0 past l = L - 1)
 //   forward: A_p[r][jj] = G[j] + (-1)^p G[J - 1 - j], j = B k + jj  (0 past Jh)
-// A task is one (row, 16-byte chunk); each thread loads Op::kUnroll tasks
-// before converting any, so that enough bytes are in flight to cover the
-// latency.
+// A task is one (row, 16-byte chunk); each thread holds Op::kUnroll tasks, a
+// whole K block's share (512 / 192 -> 3, 1024 / 192 -> 6), so a K block costs
+// one round trip to memory, and its loads are issued before the producers wait
+// for free stages.
 template <class Op>
 constexpr int kTcTasks = 128 * (Op::kRowBytes / 16);
-// Tasks per producer thread in flight in the inverse: all of a split-BF16 K
-// block's (512 / 192 -> 3), so each K block costs one round trip to memory.
 template <class Op>
 constexpr int kInvUnroll = Op::kUnroll;
 
@@ -556,15 +555,15 @@ constexpr int kInvUnroll = Op::kUnroll;
 // (both parities).  S = m mod 4 places them at entries S .. S + 2C - 1 of a
 // window of W = 2C + 4 floats that starts 16-byte aligned (W / 4 float4).
 template <class Op, int S>
-__device__ __forceinline__ void tc_produce_inverse(const TcArgs& a, int m, int tile, int rows,
-                                                   int k, uint8_t* t0, uint8_t* t1, int pt) {
-  constexpr uint32_t kTile = 128u * Op::kRowBytes;
-  constexpr int C = Op::kChunk, W = 2 * C + 4, U = kInvUnroll<Op>;
-  for (int q0 = pt; q0 < kTcTasks<Op>; q0 += U * kTcProducers) {
-    float w[U][W];
+struct TcInverse {
+  static constexpr int C = Op::kChunk, W = 2 * C + 4, U = kInvUnroll<Op>;
+  float w[U][W];
+
+  __device__ __forceinline__ void load(const TcArgs& a, int m, int tile, int rows, int k,
+                                       int pt) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int q = q0 + u * kTcProducers;
+      const int q = pt + u * kTcProducers;
 #pragma unroll
       for (int e = 0; e < W; ++e) w[u][e] = 0.f;
       if (q >= kTcTasks<Op>) continue;
@@ -577,7 +576,7 @@ __device__ __forceinline__ void tc_produce_inverse(const TcArgs& a, int m, int t
       const int l0 = 2 * Op::kKB * k + 2 * C * c;  // relative to l = m
       const int lim = (a.L - m) - l0;             // valid entries from l0
       const float* src = seg_field(a.in, b, (size_t)a.M * a.L) + (size_t)row * a.L + m + l0;
-      if (a.vec && lim >= W) {
+      if (lim >= W) {
         const float4* w4 = reinterpret_cast<const float4*>(src - S);
 #pragma unroll
         for (int i = 0; i < W / 4; ++i) {
@@ -592,9 +591,12 @@ __device__ __forceinline__ void tc_produce_inverse(const TcArgs& a, int m, int t
         for (int e = 0; e < 2 * C; ++e) w[u][e + S] = (e < lim) ? __ldg(src + e) : 0.f;
       }
     }
+  }
+  __device__ __forceinline__ void store(uint8_t* t0, uint8_t* t1, int pt) {
+    constexpr uint32_t kTile = 128u * Op::kRowBytes;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int q = q0 + u * kTcProducers;
+      const int q = pt + u * kTcProducers;
       if (q >= kTcTasks<Op>) continue;
       const uint32_t off = sw_off<Op>(q / (Op::kRowBytes / 16), q % (Op::kRowBytes / 16));
       // Entries S .. S+2C-1: even l - m are parity 0, odd ones parity 1.
@@ -602,7 +604,7 @@ __device__ __forceinline__ void tc_produce_inverse(const TcArgs& a, int m, int t
       if (t1) put_split<Op>(w[u], S + 1, 2, t1, t1 + kTile, off);
     }
   }
-}
+};
 
 // Inverse, rows at any alignment (L not a multiple of 4, or a segment that
 // starts off a 16-byte boundary): the same tasks, each read as W / 4 float4 of
@@ -613,17 +615,16 @@ __device__ __forceinline__ void tc_produce_inverse(const TcArgs& a, int m, int t
 // 16-byte boundary at or before the task's first entry: inside the caller's
 // allocation, which starts on a 256-byte boundary (device allocations do).
 template <class Op>
-__device__ __forceinline__ void tc_produce_inverse_any(const TcArgs& a, int m, int tile,
-                                                       int rows, int k, uint8_t* t0,
-                                                       uint8_t* t1, int pt) {
-  constexpr uint32_t kTile = 128u * Op::kRowBytes;
-  constexpr int C = Op::kChunk, W = 2 * C + 4, U = kInvUnroll<Op>;
-  for (int q0 = pt; q0 < kTcTasks<Op>; q0 += U * kTcProducers) {
-    float w[U][W];
-    int sh[U];
+struct TcInverseAny {
+  static constexpr int C = Op::kChunk, W = 2 * C + 4, U = kInvUnroll<Op>;
+  float w[U][W];
+  int sh[U];
+
+  __device__ __forceinline__ void load(const TcArgs& a, int m, int tile, int rows, int k,
+                                       int pt) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int q = q0 + u * kTcProducers;
+      const int q = pt + u * kTcProducers;
 #pragma unroll
       for (int e = 0; e < W; ++e) w[u][e] = 0.f;
       sh[u] = 0;
@@ -654,9 +655,12 @@ __device__ __forceinline__ void tc_produce_inverse_any(const TcArgs& a, int m, i
         for (int e = 0; e < 2 * C; ++e) w[u][e] = (e < lim) ? __ldg(src + e) : 0.f;
       }
     }
+  }
+  __device__ __forceinline__ void store(uint8_t* t0, uint8_t* t1, int pt) {
+    constexpr uint32_t kTile = 128u * Op::kRowBytes;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int q = q0 + u * kTcProducers;
+      const int q = pt + u * kTcProducers;
       if (q >= kTcTasks<Op>) continue;
       // o[e] = w[sh + e]: shift by 1, then by 2.
       float y[2 * C + 2], o[2 * C];
@@ -669,20 +673,20 @@ __device__ __forceinline__ void tc_produce_inverse_any(const TcArgs& a, int m, i
       if (t1) put_split<Op>(o, 1, 2, t1, t1 + kTile, off);
     }
   }
-}
+};
 
 // Forward: a task covers the C latitudes j0 .. j0 + C - 1 and their mirrors.
 template <class Op>
-__device__ __forceinline__ void tc_produce_forward(const TcArgs& a, int m, int tile, int rows,
-                                                   int k, uint8_t* t0, uint8_t* t1, int pt) {
-  constexpr uint32_t kTile = 128u * Op::kRowBytes;
-  constexpr int C = Op::kChunk, U = Op::kUnroll;
-  const bool vec = (a.J & 3) == 0;
-  for (int q0 = pt; q0 < kTcTasks<Op>; q0 += U * kTcProducers) {
-    float d[U][C], e[U][C];  // G[j0 + t], G[J - 1 - j0 - t]
+struct TcForward {
+  static constexpr int C = Op::kChunk, U = Op::kUnroll;
+  float d[U][C], e[U][C];  // G[j0 + t], G[J - 1 - j0 - t]
+
+  __device__ __forceinline__ void load(const TcArgs& a, int m, int tile, int rows, int k,
+                                       int pt) {
+    const bool vec = (a.J & 3) == 0;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int q = q0 + u * kTcProducers;
+      const int q = pt + u * kTcProducers;
 #pragma unroll
       for (int t = 0; t < C; ++t) d[u][t] = e[u][t] = 0.f;
       if (q >= kTcTasks<Op>) continue;
@@ -716,9 +720,12 @@ __device__ __forceinline__ void tc_produce_forward(const TcArgs& a, int m, int t
         }
       }
     }
+  }
+  __device__ __forceinline__ void store(uint8_t* t0, uint8_t* t1, int pt) {
+    constexpr uint32_t kTile = 128u * Op::kRowBytes;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int q = q0 + u * kTcProducers;
+      const int q = pt + u * kTcProducers;
       if (q >= kTcTasks<Op>) continue;
       const uint32_t off = sw_off<Op>(q / (Op::kRowBytes / 16), q % (Op::kRowBytes / 16));
       float sv[C], dv[C];
@@ -731,7 +738,7 @@ __device__ __forceinline__ void tc_produce_forward(const TcArgs& a, int m, int t
       if (t1) put_split<Op>(dv, 0, 1, t1, t1 + kTile, off);
     }
   }
-}
+};
 
 // L2 prefetches of the rows of K block k: block 0's before the CTA's set-up
 // barrier (barrier init, TMEM allocation), so that the set-up overlaps their
@@ -768,20 +775,37 @@ __device__ __forceinline__ void tc_prefetch_block(const TcArgs& a, int m, int ti
   }
 }
 
-template <bool kForward, class Op>
-__device__ __forceinline__ void tc_produce(const TcArgs& a, int m, int tile, int rows, int k,
-                                           uint8_t* t0, uint8_t* t1, int pt) {
-  if (kForward) {
-    tc_produce_forward<Op>(a, m, tile, rows, k, t0, t1, pt);
-  } else if (!a.vec) {
-    tc_produce_inverse_any<Op>(a, m, tile, rows, k, t0, t1, pt);
-  } else {
-    switch (m & 3) {
-      case 0: tc_produce_inverse<Op, 0>(a, m, tile, rows, k, t0, t1, pt); break;
-      case 1: tc_produce_inverse<Op, 1>(a, m, tile, rows, k, t0, t1, pt); break;
-      case 2: tc_produce_inverse<Op, 2>(a, m, tile, rows, k, t0, t1, pt); break;
-      default: tc_produce_inverse<Op, 3>(a, m, tile, rows, k, t0, t1, pt); break;
-    }
+// The producer loop: block k's parities go to consecutive stages, and block
+// k + 1's rows are prefetched into L2 meanwhile.  kEarly: the loads of block
+// k + 1 are issued as soon as block k has left the registers, so that they
+// overlap the wait for its stages to be free (split-BF16 TL255, 64 fields:
+// forward 23.4 -> 19.0 us, inverse 23.2 -> 22.1; split-TF32 T170 forward 22.7 ->
+// 21.1).  The split-TF32 inverse, whose six tasks a thread fill the registers,
+// loads after the wait (17.7 us; early 19.9).
+template <bool kForward, class Op, class Tasks>
+__device__ __forceinline__ void tc_produce(const TcArgs& a, int m, int tile, int rows, int pt,
+                                           int kblk0, int kblk1, uint8_t* base,
+                                           uint32_t stage_bytes, uint64_t* full_bar,
+                                           uint64_t* empty_bar) {
+  static_assert(Tasks::U * kTcProducers >= kTcTasks<Op>, "a K block in one round");
+  constexpr bool kEarly = kForward || Op::kFmt == OpBf16::kFmt;
+  Tasks t;
+  if (kEarly) t.load(a, m, tile, rows, 0, pt);
+  for (int k = 0; k < kblk0; ++k) {
+    const bool two = k < kblk1;
+    const int i0 = two ? 2 * k : k + kblk1;
+    const int s0 = i0 % a.stages, u0 = i0 / a.stages;
+    const int s1 = (i0 + 1) % a.stages, u1 = (i0 + 1) / a.stages;
+    if (k + 1 < kblk0) tc_prefetch_block<kForward, Op>(a, m, tile, rows, k + 1, pt);
+    if (u0 > 0 && !mbar_wait(&empty_bar[s0], (u0 - 1) & 1, a.err, 4)) break;
+    if (two && u1 > 0 && !mbar_wait(&empty_bar[s1], (u1 - 1) & 1, a.err, 4)) break;
+    if (!kEarly) t.load(a, m, tile, rows, k, pt);
+    t.store(base + (size_t)s0 * stage_bytes, two ? base + (size_t)s1 * stage_bytes : nullptr, pt);
+    // Make the generic-proxy stores visible to the tensor cores.
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    mbar_arrive(&full_bar[s0]);
+    if (two) mbar_arrive(&full_bar[s1]);
+    if (kEarly && k + 1 < kblk0) t.load(a, m, tile, rows, k + 1, pt);
   }
 }
 
@@ -929,23 +953,24 @@ legendre_tc_kernel(const __grid_constant__ CUtensorMap tBh,
     // Arrives once every MMA issued above has completed.
     umma_commit(&done_bar);
   } else if (warp >= 2) {
-    // A producers: block k's parities go to consecutive stages.
+    // A producers.
     const int pt = threadIdx.x - 64;
-    for (int k = 0; k < kblk[0]; ++k) {
-      const bool two = k < kblk[1];
-      const int i0 = two ? 2 * k : k + kblk[1];
-      const int s0 = i0 % a.stages, u0 = i0 / a.stages;
-      const int s1 = (i0 + 1) % a.stages, u1 = (i0 + 1) / a.stages;
-      if (u0 > 0 && !mbar_wait(&empty_bar[s0], (u0 - 1) & 1, a.err, 4)) break;
-      if (two && u1 > 0 && !mbar_wait(&empty_bar[s1], (u1 - 1) & 1, a.err, 4)) break;
-      uint8_t* t0 = base + (size_t)s0 * stage_bytes;
-      uint8_t* t1 = two ? base + (size_t)s1 * stage_bytes : nullptr;
-      if (k + 1 < kblk[0]) tc_prefetch_block<kForward, Op>(a, m, tile, rows, k + 1, pt);
-      tc_produce<kForward, Op>(a, m, tile, rows, k, t0, t1, pt);
-      // Make the generic-proxy stores visible to the tensor cores.
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      mbar_arrive(&full_bar[s0]);
-      if (two) mbar_arrive(&full_bar[s1]);
+    auto produce = [&](auto tasks) {
+      using Tasks = decltype(tasks);
+      tc_produce<kForward, Op, Tasks>(a, m, tile, rows, pt, kblk[0], kblk[1], base, stage_bytes,
+                                      full_bar, empty_bar);
+    };
+    if constexpr (kForward) {
+      produce(TcForward<Op>{});
+    } else if (!a.vec) {
+      produce(TcInverseAny<Op>{});
+    } else {
+      switch (m & 3) {
+        case 0: produce(TcInverse<Op, 0>{}); break;
+        case 1: produce(TcInverse<Op, 1>{}); break;
+        case 2: produce(TcInverse<Op, 2>{}); break;
+        default: produce(TcInverse<Op, 3>{}); break;
+      }
     }
     if (kForward) {
       // The structural zeros l < m of this tile's rows, while the MMAs of
