@@ -25,10 +25,9 @@ namespace dino {
 // Legendre contraction, FP32 SIMT
 // ---------------------------------------------------------------------------
 
-constexpr int kLegTB = 128;  // (field, cos/sin) rows per CTA
-constexpr int kLegTN = 32;   // latitudes (inverse) or l values (forward) per CTA
+constexpr int kLegTN = 32;   // latitudes (inverse) per CTA
 constexpr int kLegKC = 16;   // contraction chunk
-constexpr int kLegThreads = 128;
+// (field, cos/sin) rows, and threads, per CTA: 128, or 64 for short batches.
 
 // Row r of the m-slice: m == 0 has one row per field (cos), m > 0 has two.
 __device__ __forceinline__ void row_map(int m, int r, int& b, int& row) {
@@ -41,13 +40,19 @@ __device__ __forceinline__ void row_map(int m, int r, int& b, int& row) {
   }
 }
 
-// Each thread stages 4 rows x 4 contraction indices of a 128 x 16 operand
-// chunk: rows (tid / 4) + 32 i, indices 4 (tid % 4) .. + 3.  Row pointers are
+// Each thread stages 4 rows x 4 contraction indices of a TB x 16 operand
+// chunk: rows (tid / 4) + TB / 4 i, indices 4 (tid % 4) .. + 3.  Row pointers are
 // resolved once per CTA; the next chunk is prefetched into registers while
 // the current one is consumed from shared memory.
 
-// out_fourier[b][row][j] for all j from modal rows (inverse contraction).
-__global__ void __launch_bounds__(kLegThreads)
+// out_fourier[b][row][j] for all j from modal rows (inverse contraction).  Two
+// rows share an f32x2 FMA: the loop was bound by its issue slots and its
+// shared-memory reads together, and a value's place in two registers is free.
+// The bound of three CTAs of 128 an SM keeps the accumulators out of memory
+// (four spill: TL255, 64 fields 56 us).  TL159, 75 fields 26.0 -> 24.4 us, TL255,
+// 64 fields 42.4 -> 40.1, T42, 900 fields 11.6 -> 10.5.
+template <int TB>
+__global__ void __launch_bounds__(TB, 3 * 128 / TB)
 legendre_inverse_simt(Segs in, float* __restrict__ out, int B, int M, int L,
                       int J, int Jh, const float* __restrict__ ptab,
                       const int64_t* __restrict__ ptab_off) {
@@ -55,13 +60,13 @@ legendre_inverse_simt(Segs in, float* __restrict__ out, int B, int M, int L,
   pdl_wait();
   const int m = blockIdx.z;
   const int rows = (m == 0) ? B : 2 * B;
-  const int r0 = blockIdx.y * kLegTB;
+  const int r0 = blockIdx.y * TB;
   if (r0 >= rows) return;
   const int j0 = blockIdx.x * kLegTN;
   const int Lm = L - m;
   const float* P = ptab + ptab_off[m];
 
-  __shared__ __align__(16) float Xs[kLegKC][kLegTB + 4];
+  __shared__ __align__(16) float Xs[kLegKC][TB + 4];
   __shared__ __align__(16) float Ps[kLegKC][kLegTN];
 
   const int tid = threadIdx.x;
@@ -71,7 +76,7 @@ legendre_inverse_simt(Segs in, float* __restrict__ out, int B, int M, int L,
   const float* xrow[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int r = r0 + (tid >> 2) + 32 * i;
+    const int r = r0 + (tid >> 2) + TB / 4 * i;
     xrow[i] = nullptr;
     if (r < rows) {
       int b, row;
@@ -79,9 +84,10 @@ legendre_inverse_simt(Segs in, float* __restrict__ out, int B, int M, int L,
       xrow[i] = seg_field(in, b, (size_t)M * L) + (size_t)row * L + m;
     }
   }
-  const int pk = tid >> 3, pj = (tid & 7) * 4;  // P chunk: 16 x 32 as float4
+  constexpr int kPv = 128 / TB;  // float4 of the 16 x 32 table chunk per thread
+  const int pk = tid >> 3, pj = (tid & 7) * 4;
   float xv[4][4];
-  float4 pv;
+  float4 pv[kPv];
   auto fetch = [&](int kc) {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -90,26 +96,29 @@ legendre_inverse_simt(Segs in, float* __restrict__ out, int B, int M, int L,
         const int k = kc + lq * 4 + e;
         xv[i][e] = (xrow[i] && k < Lm) ? xrow[i][k] : 0.f;
       }
-    const int k = kc + pk;
-    const int j = j0 + pj;
-    // Vector load only when the row start is 16-byte aligned (Jh % 4 == 0;
-    // the per-m table offsets are multiples of Jh).
-    if ((Jh & 3) == 0 && k < Lm && j + 3 < Jh) {
-      pv = *reinterpret_cast<const float4*>(P + (size_t)k * Jh + j);
-    } else {
-      float t[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        t[e] = (k < Lm && j + e < Jh) ? P[(size_t)k * Jh + j + e] : 0.f;
-      pv = make_float4(t[0], t[1], t[2], t[3]);
+    for (int i = 0; i < kPv; ++i) {
+      const int k = kc + pk + TB / 8 * i;
+      const int j = j0 + pj;
+      // Vector load only when the row start is 16-byte aligned (Jh % 4 == 0;
+      // the per-m table offsets are multiples of Jh).
+      if ((Jh & 3) == 0 && k < Lm && j + 3 < Jh) {
+        pv[i] = *reinterpret_cast<const float4*>(P + (size_t)k * Jh + j);
+      } else {
+        float t[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          t[e] = (k < Lm && j + e < Jh) ? P[(size_t)k * Jh + j + e] : 0.f;
+        pv[i] = make_float4(t[0], t[1], t[2], t[3]);
+      }
     }
   };
 
-  float accE[8][4], accO[8][4];
+  float2 aE[4][4], aO[4][4];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int t = 0; t < 4; ++t) accE[i][t] = accO[i][t] = 0.f;
+    for (int t = 0; t < 4; ++t) aE[i][t] = aO[i][t] = make_float2(0.f, 0.f);
 
   fetch(0);
   for (int kc = 0; kc < Lm; kc += kLegKC) {
@@ -117,32 +126,41 @@ legendre_inverse_simt(Segs in, float* __restrict__ out, int B, int M, int L,
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) Xs[lq * 4 + e][(tid >> 2) + 32 * i] = xv[i][e];
-    *reinterpret_cast<float4*>(&Ps[pk][pj]) = pv;
+      for (int e = 0; e < 4; ++e) Xs[lq * 4 + e][(tid >> 2) + TB / 4 * i] = xv[i][e];
+#pragma unroll
+    for (int i = 0; i < kPv; ++i)
+      *reinterpret_cast<float4*>(&Ps[pk + TB / 8 * i][pj]) = pv[i];
     __syncthreads();
     if (kc + kLegKC < Lm) fetch(kc + kLegKC);
 #pragma unroll
     for (int kk = 0; kk < kLegKC; kk += 2) {
-      float4 xa = *reinterpret_cast<const float4*>(&Xs[kk][ty * 8]);
-      float4 xb = *reinterpret_cast<const float4*>(&Xs[kk][ty * 8 + 4]);
-      float4 pp = *reinterpret_cast<const float4*>(&Ps[kk][tx * 4]);
-      float xe[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
-      float pe[4] = {pp.x, pp.y, pp.z, pp.w};
+      auto step = [&](int k, float2 (&acc)[4][4]) {
+        const float4 xa = *reinterpret_cast<const float4*>(&Xs[k][ty * 8]);
+        const float4 xb = *reinterpret_cast<const float4*>(&Xs[k][ty * 8 + 4]);
+        const float4 pp = *reinterpret_cast<const float4*>(&Ps[k][tx * 4]);
+        const float2 x[4] = {make_float2(xa.x, xa.y), make_float2(xa.z, xa.w),
+                             make_float2(xb.x, xb.y), make_float2(xb.z, xb.w)};
+        const float p[4] = {pp.x, pp.y, pp.z, pp.w};
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+        for (int t = 0; t < 4; ++t)
 #pragma unroll
-        for (int t = 0; t < 4; ++t) accE[i][t] = fmaf(xe[i], pe[t], accE[i][t]);
-      xa = *reinterpret_cast<const float4*>(&Xs[kk + 1][ty * 8]);
-      xb = *reinterpret_cast<const float4*>(&Xs[kk + 1][ty * 8 + 4]);
-      pp = *reinterpret_cast<const float4*>(&Ps[kk + 1][tx * 4]);
-      float xo[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
-      float po[4] = {pp.x, pp.y, pp.z, pp.w};
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int t = 0; t < 4; ++t) accO[i][t] = fmaf(xo[i], po[t], accO[i][t]);
+          for (int i = 0; i < 4; ++i)
+            acc[i][t] = __ffma2_rn(x[i], make_float2(p[t], p[t]), acc[i][t]);
+      };
+      step(kk, aE);
+      step(kk + 1, aO);
     }
   }
+  float accE[8][4], accO[8][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      accE[2 * i][t] = aE[i][t].x;
+      accE[2 * i + 1][t] = aE[i][t].y;
+      accO[2 * i][t] = aO[i][t].x;
+      accO[2 * i + 1][t] = aO[i][t].y;
+    }
 
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
@@ -174,14 +192,18 @@ legendre_inverse_simt(Segs in, float* __restrict__ out, int B, int M, int L,
 }
 
 // out_modal[b][row][l] = sum_j p[m,j,l] G[b][row][j] (forward contraction);
-// writes zeros for l < m.  A CTA covers 128 rows and TN values of l (64 for
+// writes zeros for l < m.  A CTA covers TB rows and TN values of l (64 for
 // long l ranges, 32 for short ones, which keeps more CTAs per SM): thread
 // (tx, ty) accumulates rows 8 ty .. 8 ty + 7 at l - m = k0 + tx + 8 t,
 // t < TN / 8, all of one parity, so it reads only the symmetric (even) or
 // antisymmetric (odd) latitude fold.  Folds and table chunks are fetched with
 // float4 loads where the rows allow.
-template <int TN>
-__global__ void __launch_bounds__(kLegThreads)
+// Two rows share an f32x2 FMA, and the two folds lie half a bank line apart,
+// because the lanes of a read take both: TL159, 75 fields 44.4 -> 36.7 us, T42,
+// 900 fields 17.9 -> 15.3, TL255, 64 fields 74.3 -> 68.3, TL95, 600 fields 51.0 ->
+// 47.6.
+template <int TN, int TB>
+__global__ void __launch_bounds__(TB)
 legendre_forward_simt(const float* __restrict__ G, float* __restrict__ out,
                       int B, int M, int L, int J, int Jh,
                       const float* __restrict__ ptab,
@@ -190,11 +212,11 @@ legendre_forward_simt(const float* __restrict__ G, float* __restrict__ out,
   pdl_wait();
   const int m = blockIdx.z;
   const int rows = (m == 0) ? B : 2 * B;
-  const int r0 = blockIdx.y * kLegTB;
+  const int r0 = blockIdx.y * TB;
   if (r0 >= rows) return;
   const int Lm = L - m;
   constexpr int TT = TN / 8;           // l values per thread
-  constexpr int PV = TN / 8;           // table values fetched per thread and chunk
+  constexpr int PV = TN * kLegKC / TB; // table values fetched per thread and chunk
   constexpr int PT = kLegKC / PV;      // threads per table row
   const int k0 = blockIdx.x * TN;  // l - m offset of this tile
   const int tid = threadIdx.x;
@@ -203,7 +225,7 @@ legendre_forward_simt(const float* __restrict__ G, float* __restrict__ out,
 
   if (blockIdx.x == 0 && m > 0) {
     // Structural zeros l < m of the rows handled by this CTA.
-    for (int idx = tid; idx < kLegTB * m; idx += kLegThreads) {
+    for (int idx = tid; idx < TB * m; idx += TB) {
       int rl = idx / m, l = idx % m;
       int r = r0 + rl;
       if (r < rows) {
@@ -216,15 +238,19 @@ legendre_forward_simt(const float* __restrict__ G, float* __restrict__ out,
   if (k0 >= Lm) return;
   const float* P = ptab + ptab_off[m];
 
-  __shared__ __align__(16) float Ss[kLegKC][kLegTB + 4];
-  __shared__ __align__(16) float Ds[kLegKC][kLegTB + 4];
+  // The antisymmetric fold lies half a bank line (16 floats) off the symmetric
+  // one's banks: the lanes of a read take both.
+  constexpr int kFoldStride = TB + 4, kDs = kLegKC * kFoldStride + 16;
+  __shared__ __align__(16) float folds[kDs + kLegKC * kFoldStride];
+  float(*Ss)[kFoldStride] = reinterpret_cast<float(*)[kFoldStride]>(folds);
+  float(*Ds)[kFoldStride] = reinterpret_cast<float(*)[kFoldStride]>(folds + kDs);
   __shared__ float Ps[kLegKC][TN + 1];
 
   const int lq = tid & 3;
   const float* grow[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int r = r0 + (tid >> 2) + 32 * i;
+    const int r = r0 + (tid >> 2) + TB / 4 * i;
     grow[i] = nullptr;
     if (r < rows) {
       int b, row;
@@ -286,11 +312,11 @@ legendre_forward_simt(const float* __restrict__ G, float* __restrict__ out,
     }
   };
 
-  float acc[8][TT];
+  float2 acc[4][TT];  // row pairs
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int t = 0; t < TT; ++t) acc[i][t] = 0.f;
+    for (int t = 0; t < TT; ++t) acc[i][t] = make_float2(0.f, 0.f);
 
   fetch(0);
   for (int jc = 0; jc < Jh; jc += kLegKC) {
@@ -299,8 +325,8 @@ legendre_forward_simt(const float* __restrict__ G, float* __restrict__ out,
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        Ss[lq * 4 + e][(tid >> 2) + 32 * i] = sv[i][e];
-        Ds[lq * 4 + e][(tid >> 2) + 32 * i] = dv[i][e];
+        Ss[lq * 4 + e][(tid >> 2) + TB / 4 * i] = sv[i][e];
+        Ds[lq * 4 + e][(tid >> 2) + TB / 4 * i] = dv[i][e];
       }
 #pragma unroll
     for (int e = 0; e < PV; ++e) Ps[pjq + e][pl_] = pvr[e];
@@ -309,16 +335,17 @@ legendre_forward_simt(const float* __restrict__ G, float* __restrict__ out,
     const float* fold = (tx & 1) ? &Ds[0][0] : &Ss[0][0];
 #pragma unroll
     for (int jj = 0; jj < kLegKC; ++jj) {
-      float4 fa = *reinterpret_cast<const float4*>(fold + jj * (kLegTB + 4) + ty * 8);
-      float4 fb = *reinterpret_cast<const float4*>(fold + jj * (kLegTB + 4) + ty * 8 + 4);
-      float f8[8] = {fa.x, fa.y, fa.z, fa.w, fb.x, fb.y, fb.z, fb.w};
-      float pw[TT];
+      float4 fa = *reinterpret_cast<const float4*>(fold + jj * (TB + 4) + ty * 8);
+      float4 fb = *reinterpret_cast<const float4*>(fold + jj * (TB + 4) + ty * 8 + 4);
+      const float2 f4[4] = {make_float2(fa.x, fa.y), make_float2(fa.z, fa.w),
+                            make_float2(fb.x, fb.y), make_float2(fb.z, fb.w)};
 #pragma unroll
-      for (int t = 0; t < TT; ++t) pw[t] = Ps[jj][tx + 8 * t];
+      for (int t = 0; t < TT; ++t) {
+        const float pw = Ps[jj][tx + 8 * t];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int t = 0; t < TT; ++t) acc[i][t] = fmaf(f8[i], pw[t], acc[i][t]);
+        for (int i = 0; i < 4; ++i)
+          acc[i][t] = __ffma2_rn(f4[i], make_float2(pw, pw), acc[i][t]);
+      }
     }
   }
 
@@ -332,28 +359,42 @@ legendre_forward_simt(const float* __restrict__ G, float* __restrict__ out,
 #pragma unroll
     for (int t = 0; t < TT; ++t) {
       int k = k0 + tx + 8 * t;
-      if (k < Lm) o[k] = acc[i][t];
+      if (k < Lm) o[k] = (i & 1) ? acc[i >> 1][t].y : acc[i >> 1][t].x;
     }
   }
+}
+
+// Rows per CTA: 64 where that saves half a row tile of one or two (rows of one
+// or three 64-row tiles), or where 128 leave fewer than `few` CTAs; else 128,
+// which reads the table half as often.  Forward / inverse us with 128 and 64
+// rows: T213, 20 fields (40 rows) 55.9 -> 42.1 / 30.2 -> 24.2; T85, 15 fields 16.6
+// -> 14.6; TL159, 75 fields (150 rows) 36.9, 37.0 / 24.8 -> 21.8; T42, 121 fields
+// (172 CTAs forward) 9.6 -> 8.1; TL127, 33 fields inverse 12.7 -> 14.2; TL255, 64
+// fields 68 -> 74.
+static int leg_rows(const dino_plan* p, int nf, int tiles, int few) {
+  const int half = ceil_div(2 * nf, 64);
+  const bool short_grid = (int64_t)ceil_div(2 * nf, 128) * tiles * p->lw < few;
+  return (half == 1 || half == 3 || short_grid) ? 64 : 128;
 }
 
 // The FP32 SIMT inverse contraction regardless of the plan's precision.
 int legendre_inverse_fp32(dino_plan* p, const Segs& in, float* out, int nf,
                           cudaStream_t st) {
   NvtxRange range("inv_legendre");
-  dim3 grid(ceil_div(p->Jh, kLegTN), ceil_div(2 * nf, kLegTB), p->lw);
-  return launch_pdl("legendre_inverse_simt", legendre_inverse_simt, grid, kLegThreads, 0, st, in,
-                    out, nf, p->M, p->L, p->J, p->Jh, p->d_ptab, p->d_ptab_off);
+  const int tiles = ceil_div(p->Jh, kLegTN), tb = leg_rows(p, nf, tiles, 0);
+  return launch_pdl("legendre_inverse_simt",
+                    tb == 64 ? legendre_inverse_simt<64> : legendre_inverse_simt<128>,
+                    dim3(tiles, ceil_div(2 * nf, tb), p->lw), tb, 0, st, in, out, nf, p->M, p->L,
+                    p->J, p->Jh, p->d_ptab, p->d_ptab_off);
 }
 
 int legendre_inverse(dino_plan* p, const Segs& in, float* out, int nf,
                      cudaStream_t st) {
-  NvtxRange range("inv_legendre");
-  if (p->precision != DINO_PREC_FP32 && !tc_use_simt(p, false))
+  if (p->precision != DINO_PREC_FP32 && !tc_use_simt(p, false)) {
+    NvtxRange range("inv_legendre");
     return tc_legendre_inverse(p, in, out, nf, st);
-  dim3 grid(ceil_div(p->Jh, kLegTN), ceil_div(2 * nf, kLegTB), p->lw);
-  return launch_pdl("legendre_inverse_simt", legendre_inverse_simt, grid, kLegThreads, 0, st, in,
-                    out, nf, p->M, p->L, p->J, p->Jh, p->d_ptab, p->d_ptab_off);
+  }
+  return legendre_inverse_fp32(p, in, out, nf, st);
 }
 
 int legendre_forward(dino_plan* p, const float* G, float* out, int nf,
@@ -367,15 +408,13 @@ int legendre_forward(dino_plan* p, const float* G, float* out, int nf,
 // The FP32 SIMT forward contraction regardless of the plan's precision.
 int legendre_forward_fp32(dino_plan* p, const float* G, float* out, int nf,
                           cudaStream_t st) {
-  if (p->L > 64) {
-    dim3 grid(ceil_div(p->L, 64), ceil_div(2 * nf, kLegTB), p->lw);
-    return launch_pdl("legendre_forward_simt", legendre_forward_simt<64>, grid, kLegThreads, 0,
-                      st, G, out, nf, p->M, p->L, p->J, p->Jh, p->d_ptab, p->d_ptab_off);
-  } else {
-    dim3 grid(ceil_div(p->L, 32), ceil_div(2 * nf, kLegTB), p->lw);
-    return launch_pdl("legendre_forward_simt", legendre_forward_simt<32>, grid, kLegThreads, 0,
-                      st, G, out, nf, p->M, p->L, p->J, p->Jh, p->d_ptab, p->d_ptab_off);
-  }
+  const int tn = p->L > 64 ? 64 : 32, tiles = ceil_div(p->L, tn);
+  const int tb = leg_rows(p, nf, tiles, 2 * 148);
+  auto* kernel = tn == 64
+                     ? (tb == 64 ? legendre_forward_simt<64, 64> : legendre_forward_simt<64, 128>)
+                     : (tb == 64 ? legendre_forward_simt<32, 64> : legendre_forward_simt<32, 128>);
+  return launch_pdl("legendre_forward_simt", kernel, dim3(tiles, ceil_div(2 * nf, tb), p->lw), tb,
+                    0, st, G, out, nf, p->M, p->L, p->J, p->Jh, p->d_ptab, p->d_ptab_off);
 }
 
 // ---------------------------------------------------------------------------

@@ -166,3 +166,18 @@ def test_shape_and_argument_errors():
   with pytest.raises(ValueError):
     sh.Grid(longitude_wavenumbers=10, total_wavenumbers=5, longitude_nodes=64,
             latitude_nodes=32).plan
+
+
+@pytest.mark.parametrize('fields', [1, 31, 33, 65, 97, 130])
+@pytest.mark.parametrize('wavenumbers', [7, 33, 66])
+def test_row_tiles_of_the_fp32_contractions(wavenumbers, fields):
+  # 64- and 128-row CTAs around their edges (one, three and more 64-row tiles,
+  # one row past a tile), short and long l ranges (32- and 64-wide tiles), odd
+  # latitude counts; bound as above.
+  g = sh.Grid.with_wavenumbers(wavenumbers)
+  o = osht.Grid.with_wavenumbers(wavenumbers)
+  x = ostates.sht_modal_input(o, fields, seed=fields)
+  ref = o.to_nodal(x.astype(np.float64))
+  assert rel_err(g.to_nodal(x), ref) < 2e-6
+  z = ref.astype(np.float32)
+  assert rel_err(g.to_modal(z), o.to_modal(z.astype(np.float64))) < 2e-6
