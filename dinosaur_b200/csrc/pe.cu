@@ -348,8 +348,8 @@ __device__ __forceinline__ void st_vec(float* p, const float (&x)[V]) {
 // latitude count J is a multiple of V, so they lie on one meridian).
 // kTracers = false compiles out the tracer windows (dry states).
 // Every field of the next level is loaded while a level is computed (moist
-// TL255 / 32 x 4: 570 -> 541 us a launch; T21 / 12: 10.0 -> 9.3 us).
-constexpr int kNodalCols = 32, kNodalMaxChunks = 2;
+// TL255 / 32 x 4: 570 -> 541 us a launch).
+constexpr int kNodalCols = 32, kNodalMaxChunks = 4;
 
 template <bool kTracers, int V>
 __global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
@@ -2400,13 +2400,15 @@ static int pe_nodal_inputs(dino_pe* pe, const float* state, cudaStream_t st) {
   return DINO_OK;
 }
 
-// Level chunks per column for pe_nodal_kernel: two from eight levels on.  The
+// Level chunks per column for pe_nodal_kernel: four from eight levels on.  The
 // count depends on the levels alone, so that a state's sums are formed in the
 // same order, and its tendencies have the same bits, in any batch.  Measured
-// with one, two and four chunks (us a launch): T21 / 12 14.0, 9.3, 7.9; T42 / 24
-// x 16 37.2, 37.7, 43.4; TL255 / 32 45.0, 45.2, 48.5; TL95 / 19 moist x 3 38.7,
-// 40.9, 39.6; TL255 / 32 moist x 4 547, 541, 561.
-static int nodal_chunks(const dino_pe* pe) { return pe->K >= 8 ? kNodalMaxChunks : 1; }
+// with two and four chunks (us a launch): T21 / 12 9.8, 7.4; T42 / 20 13.9, 8.9;
+// T42 / 24 x 16 37.5, 41.3; TL255 / 32 46.2, 45.3; TL95 / 19 moist x 3 38.8, 38.8;
+// TL255 / 32 moist x 4 541, 558.
+static int nodal_chunks(const dino_pe* pe) {
+  return pe->K >= 8 ? kNodalMaxChunks : pe->K >= 4 ? 2 : 1;
+}
 
 // Adjacent columns per thread for pe_nodal_kernel: two for dry states where
 // the latitude count is even (122 registers; four need 188 and run slower),

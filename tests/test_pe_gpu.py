@@ -223,9 +223,10 @@ def test_level_chunks_agree_across_batch_sizes():
     assert err < 1e-6, (k, err)
 
 
-@pytest.mark.parametrize('layers,moist', [(2, False), (9, False), (19, True), (24, False)])
+@pytest.mark.parametrize('layers,moist', [(2, False), (5, False), (9, False), (19, True),
+                                          (24, False)])
 def test_level_chunks_give_the_same_bits(layers, moist):
-  # The chunk count (one below eight levels, else two) does not depend on the
+  # The chunk count (one, two or four by the levels) does not depend on the
   # batch, so every member's tendencies have the bits of the state alone.
   kw = dict(tracers=_tracers, humidity='specific_humidity') if moist else {}
   og, oeq, st, g, eq = make('T42', layers=layers, **kw)
