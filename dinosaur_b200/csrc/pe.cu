@@ -166,15 +166,16 @@ struct PrepArgs {
 constexpr int kModalTX = 32, kModalTY = 8;
 
 // The forward passes (pe_prep_kernel, pe_post_kernel): a CTA of 32 x 8 threads
-// covers a tile of 32 rows x 32 l, four rows a thread, and walks `ppt` planes.
+// covers a tile of 32 rows x 32 l, four rows a thread, and walks the planes
+// blockIdx.z, blockIdx.z + gridDim.z, ...
 constexpr int kTile = 32;
 constexpr int kTileRows = kTile / kModalTY;  // rows per thread
 
-// Planes per CTA of a modal pass with `tiles` (row, l) tiles: a CTA loads its
-// operator coefficients once for all of them, but small grids need the planes
-// spread to fill the chip (T21 / 12 levels, 2 tiles: eight planes a CTA left 4
-// CTAs and 19.6 us for the post-pass).  Eight where that still gives eight
-// CTAs per SM.
+// Planes per thread of an adjoint pass with `tiles` (row, l) tiles: a thread
+// loads its operator coefficients once for all of them, but small grids need
+// the planes spread to fill the chip (T21 / 12 levels, 2 tiles: eight planes a
+// CTA left 4 CTAs and 19.6 us for the post-pass).  Eight where that still
+// gives eight CTAs per SM.
 static int planes_per_cta(int tiles, int planes, int sms) {
   int ppt = 8;
   while (ppt > 1 && (int64_t)tiles * ceil_div(planes, ppt) < 8LL * sms) ppt /= 2;
@@ -221,7 +222,7 @@ struct ModalPoint {
 // (and humidity): reads the state planes once, writes the aux planes once.
 // Every load of a plane's four rows is issued before its first store (24 in
 // flight a thread), because a store that might alias stops the loads behind it.
-__global__ void __launch_bounds__(kModalTX * kModalTY, 3) pe_prep_kernel(PrepArgs a, int ppt) {
+__global__ void __launch_bounds__(kModalTX * kModalTY, 3) pe_prep_kernel(PrepArgs a) {
   pdl_trigger();
   pdl_wait();
   const int l0 = blockIdx.x * kTile, row0 = blockIdx.y * kTile;
@@ -240,9 +241,7 @@ __global__ void __launch_bounds__(kModalTX * kModalTY, 3) pe_prep_kernel(PrepArg
       {min(row0 + (int)threadIdx.y + 2 * kModalTY, a.M - 1), l, a.L, a.lw, a.deriv, 0},
       {min(row0 + (int)threadIdx.y + 3 * kModalTY, a.M - 1), l, a.L, a.lw, a.deriv, 0}};
   // Rows past the last are clamped to it and write its value again.
-  const int q0 = blockIdx.z * ppt;
-  const int q1 = min(q0 + ppt, a.K * a.mem);
-  for (int q = q0; q < q1; ++q) {
+  for (int q = blockIdx.z; q < a.K * a.mem; q += gridDim.z) {
     const int mb = q / a.K, k = q - mb * a.K;
     const float* vort = a.state + pl(a.p_vort, mb, a.K, k) * ML;
     const float* div = a.state + pl(a.p_div, mb, a.K, k) * ML;
@@ -1060,16 +1059,22 @@ struct StageArgs {
 // that neither Y* nor the g_j pass through the row-major layout.  A tile below
 // the triangle has f = 0 but for the orography term of div, so its forward
 // outputs and f_j are not read (nearly half of the tiles).  All loads of two
-// rows (and the plane's g) are issued before the stores that follow them.
-// kNf: -1 for the plain post-pass, else the number of earlier f_j.
-template <int kNf>
-__global__ void __launch_bounds__(kModalTX * kModalTY, 3)
-    pe_post_kernel(PostArgs a, StageArgs s, int ppt) {
+// rows (one with tracers) and the plane's g are issued before the stores that
+// follow them.
+// kNf: -1 for the plain post-pass, else the number of earlier f_j.  kTracers =
+// false compiles the tracers and humidity out.  One plane a CTA: eight hold
+// their coefficients but leave too few loads in flight (three stages of TL255 /
+// 32: 331 us with eight planes, 240 with two, 236 with one; moist x 4: 2415,
+// 2193, 2181).  Registers against warps: dry, two rows at three CTAs an SM 236 us,
+// one row at four 239; moist x 4, 2181 and 1977.
+template <int kNf, bool kTracers>
+__global__ void __launch_bounds__(kModalTX * kModalTY, kTracers ? 4 : 3)
+    pe_post_kernel(PostArgs a, StageArgs s) {
   pdl_trigger();
   pdl_wait();
   constexpr bool kStage = kNf >= 0;
   constexpr int kF = kNf > 0 ? kNf : 1;  // array sizes
-  constexpr int kPair = 2;               // rows whose loads are in flight together
+  constexpr int kPair = kTracers ? 1 : 2;  // rows whose loads are in flight together
   __shared__ float tile[kStage ? 2 : 1][kStage ? 3 : 1][kTile][kTile + 1];
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int l0 = blockIdx.x * kTile, row0 = blockIdx.y * kTile;
@@ -1082,11 +1087,10 @@ __global__ void __launch_bounds__(kModalTX * kModalTY, 3)
   const float filt = (kStage && s.filter) ? s.filter[lc] : 1.f;
   const float ir = a.inv_radius;
   const int n = 2 * K + 1;
-  const int q0 = blockIdx.z * ppt;
-  const int q1 = min(q0 + ppt, K * a.mem);
-  for (int q = q0; q < q1; ++q) {
+  int buf = 0;
+  for (int q = blockIdx.z; q < K * a.mem; q += gridDim.z, buf ^= 1) {
     const int mb = q / K, k = q - mb * K;
-    float(*tl)[kTile][kTile + 1] = tile[kStage ? (q & 1) : 0];
+    float(*tl)[kTile][kTile + 1] = tile[kStage ? buf : 0];
     // Entry of y0 + sum_j fc_j f_j + fself f; f_j = f below the triangle.
     struct Old {
       float y, f[kF];
@@ -1149,7 +1153,7 @@ __global__ void __launch_bounds__(kModalTX * kModalTY, 3)
           vT[i].dn = FM(a.o_vT)[p.id];
           KE[i] = FM(a.o_KE)[p.idx];
           Tn[i] = FM(a.o_Tn)[p.idx];
-          if (a.hum >= 0) {
+          if (kTracers && a.hum >= 0) {
             vh[i] = FM(a.o_vh)[p.idx];
             gh[i] = FM(a.o_gh)[p.idx];
             dh[i] = FM(a.o_dh)[p.idx];
@@ -1186,7 +1190,7 @@ __global__ void __launch_bounds__(kModalTX * kModalTY, 3)
         }
       }
     }
-    for (int t = 0; t < a.nT; ++t) {
+    for (int t = 0; kTracers && t < a.nT; ++t) {
       const int ob = a.o_tr + 3 * t * a.mem * K;
       const size_t pq = pl(a.p_tr + t * a.mem * K, mb, K, k) * ML;
       float fq[kTileRows];
@@ -2318,12 +2322,11 @@ static int get_filter(dino_pe* pe, const double* host, float** out) {
   return DINO_OK;
 }
 
-// Launch shapes of the modal passes and their planes per CTA (thread).
-static dim3 tile_grid(const dino_pe* pe, int* ppt) {
-  const int tl = ceil_div(pe->L, kTile), tr = ceil_div(pe->M, kTile);
-  const int planes = pe->K * pe->mem;
-  *ppt = planes_per_cta(tl * tr, planes, pe->sms);
-  return dim3(tl, tr, ceil_div(planes, *ppt));
+// Launch shapes of the forward modal passes (`planes` planes a CTA, more only
+// past the grid's limit) and of the adjoint ones (planes per thread in *ppt).
+static dim3 tile_grid(const dino_pe* pe, int planes) {
+  const int n = ceil_div(pe->K * pe->mem, planes);
+  return dim3(ceil_div(pe->L, kTile), ceil_div(pe->M, kTile), n < 32768 ? n : 32768);
 }
 static dim3 modal_grid(const dino_pe* pe, int* ppt) {
   const int tl = ceil_div(pe->L, kModalTX), tr = ceil_div(pe->M, kModalTY);
@@ -2373,9 +2376,11 @@ static int pe_nodal_inputs(dino_pe* pe, const float* state, cudaStream_t st) {
     a.lap = p->d_lap;
     a.invlap = p->d_invlap;
     a.inv_radius = (float)(1.0 / p->radius);
-    int ppt = 0;
-    const dim3 grid = tile_grid(pe, &ppt);
-    DINO_TRY(launch_pdl("pe_prep", pe_prep_kernel, grid, dim3(kModalTX, kModalTY), 0, st, a, ppt));
+    // Two planes a CTA where many CTAs remain (TL255 / 32: 19.6 us, one 21.3).
+    const dim3 one = tile_grid(pe, 1);
+    const bool many = (int64_t)one.x * one.y * one.z >= 16LL * pe->sms;
+    DINO_TRY(launch_pdl("pe_prep", pe_prep_kernel, many ? tile_grid(pe, 2) : one,
+                        dim3(kModalTX, kModalTY), 0, st, a));
   }
   // 2. inverse SHT of [state kinds][aux][ln ps (Held-Suarez)]
   {
@@ -2604,10 +2609,9 @@ static PostArgs make_post_args(dino_pe* pe, float* tend) {
 
 static int pe_explicit_impl(dino_pe* pe, const float* state, float* tend, cudaStream_t st) {
   DINO_TRY(pe_explicit_products(pe, state, st));
-  int ppt = 0;
-  const dim3 grid = tile_grid(pe, &ppt);
-  return launch_pdl("pe_post", pe_post_kernel<-1>, grid, dim3(kModalTX, kModalTY), 0, st,
-                    make_post_args(pe, tend), StageArgs{}, ppt);
+  auto* kernel = pe->nT > 0 ? pe_post_kernel<-1, true> : pe_post_kernel<-1, false>;
+  return launch_pdl("pe_post", kernel, tile_grid(pe, 1), dim3(kModalTX, kModalTY), 0, st,
+                    make_post_args(pe, tend), StageArgs{});
 }
 
 struct Term {
@@ -2643,13 +2647,15 @@ static int launch_stage(dino_pe* pe, const float* y0, std::initializer_list<Term
   s.out = out;
   s.lm = pe->d_lm_in;
   s.Cp = pe->Cp;
-  int ppt = 0;
-  const dim3 grid = tile_grid(pe, &ppt);
-  const PostArgs a = make_post_args(pe, keep_f);
-  const dim3 block(kModalTX, kModalTY);
   // The stage with two earlier f_j is also the one with two g_j.
-  auto* kernel = s.nf == 0 ? pe_post_kernel<0> : s.nf == 1 ? pe_post_kernel<1> : pe_post_kernel<2>;
-  return launch_pdl("pe_stage", kernel, grid, block, 0, st, a, s, ppt);
+  auto pick = [&](auto tracers) {
+    constexpr bool T = decltype(tracers)::value;
+    return s.nf == 0 ? pe_post_kernel<0, T> : s.nf == 1 ? pe_post_kernel<1, T>
+                                                        : pe_post_kernel<2, T>;
+  };
+  auto* kernel = pe->nT > 0 ? pick(std::true_type{}) : pick(std::false_type{});
+  return launch_pdl("pe_stage", kernel, tile_grid(pe, 1), dim3(kModalTX, kModalTY), 0, st,
+                    make_post_args(pe, keep_f), s);
 }
 
 // One filtered imex_rk_sil3 step in place (time_integration.py:329-405 with
