@@ -53,7 +53,7 @@ class _ModalOp(torch.autograd.Function):
 
 
 def _needs_grad(x):
-  return torch.is_grad_enabled() and x.requires_grad
+  return x.requires_grad and torch.is_grad_enabled()
 
 
 def sht_inverse(plan, x):

@@ -36,6 +36,9 @@ def tree_map(f, x, *rest):
 
 
 def map_over_nonscalars(f, x):
+  if isinstance(x, torch.Tensor):  # the common single leaf
+    return f(x) if x.ndim > 0 else x
+
   def g(leaf):
     if _is_array(leaf) and leaf.ndim > 0:
       return f(leaf)

@@ -23,6 +23,7 @@ import numpy as np
 import torch
 
 from dinosaur_b200 import _lib
+from dinosaur_b200 import autograd
 from dinosaur_b200 import pytree
 
 Array = Any
@@ -133,13 +134,13 @@ class _SphericalHarmonicBasis:
 
 def as_device_tensor(x, dtype=torch.float32) -> torch.Tensor:
   """Contiguous CUDA float32 tensor view/copy of x (NumPy or torch)."""
-  if not torch.cuda.is_available():
+  if isinstance(x, torch.Tensor) and x.is_cuda:
+    t = x
+  elif not torch.cuda.is_available():
     raise RuntimeError('dinosaur_b200 needs a CUDA device; none is available '
                        '(there is no CPU fallback)')
-  if isinstance(x, torch.Tensor):
-    t = x
-    if not t.is_cuda:
-      t = t.cuda()
+  elif isinstance(x, torch.Tensor):
+    t = x.cuda()
   else:
     t = torch.as_tensor(np.asarray(x), device='cuda')
   if t.dtype != dtype:
@@ -166,6 +167,7 @@ class Plan:
   def __init__(self, lw, tw, nodes_lon, nodes_lat, spacing, radius=1.0,
                precision='fp32', max_fields=None, host_nodes=None):
     self.lw, self.L, self.I, self.J = lw, tw, nodes_lon, nodes_lat
+    self._fns = {}
     self.M = 2 * lw - 1
     if max_fields is None:
       per_field = self.M * self.J * 4
@@ -207,6 +209,11 @@ class Plan:
 
   # -- raw calls on flat batches -------------------------------------------
   def _check(self, x: torch.Tensor, trailing: tuple[int, int], what: str):
+    # What every valid input passes, in one expression; the reasons follow.
+    if (isinstance(x, torch.Tensor) and x.is_cuda and x.dtype is torch.float32
+        and x.is_contiguous() and x.ndim >= 2 and x.shape[-2] == trailing[0]
+        and x.shape[-1] == trailing[1] and x.get_device() == self.device):
+      return
     if not isinstance(x, torch.Tensor) or not x.is_cuda:
       raise ValueError(f'{what}: expected a CUDA tensor')
     if x.dtype != torch.float32 or not x.is_contiguous():
@@ -218,36 +225,32 @@ class Plan:
       raise ValueError(f'{what}: tensor on cuda:{x.device.index}, plan on '
                        f'cuda:{self.device}')
 
-  def _call(self, name, x: torch.Tensor, out_shape, nfields):
-    out = torch.empty(out_shape, device=x.device, dtype=torch.float32)
-    fn = getattr(_lib.lib(), name)
-    _lib.check(fn(self.handle, ptr(x), ptr(out), nfields, stream_handle()),
-               name)
+  def _transform(self, name, x: torch.Tensor, rows_in, rows_out, what):
+    """One batched call: fields of shape rows_in to fields of shape rows_out."""
+    self._check(x, rows_in, what)
+    out = x.new_empty(x.shape[:-2] + rows_out)
+    fn = self._fns.get(name)
+    if fn is None:
+      fn = self._fns[name] = getattr(_lib.lib(), name)
+    _lib.check(fn(self.handle, x.data_ptr(), out.data_ptr(),
+                  x.numel() // (rows_in[0] * rows_in[1]), stream_handle()), name)
     return out
 
   def inverse(self, x: torch.Tensor) -> torch.Tensor:
-    self._check(x, (self.M, self.L), 'inverse')
-    lead = x.shape[:-2]
-    n = int(np.prod(lead)) if lead else 1
-    return self._call('dino_sht_inverse', x, lead + (self.I, self.J), n)
+    return self._transform('dino_sht_inverse', x, (self.M, self.L), (self.I, self.J),
+                           'inverse')
 
   def forward(self, z: torch.Tensor) -> torch.Tensor:
-    self._check(z, (self.I, self.J), 'forward')
-    lead = z.shape[:-2]
-    n = int(np.prod(lead)) if lead else 1
-    return self._call('dino_sht_forward', z, lead + (self.M, self.L), n)
+    return self._transform('dino_sht_forward', z, (self.I, self.J), (self.M, self.L),
+                           'forward')
 
   def inverse_adjoint(self, g: torch.Tensor) -> torch.Tensor:
-    self._check(g, (self.I, self.J), 'inverse_adjoint')
-    lead = g.shape[:-2]
-    n = int(np.prod(lead)) if lead else 1
-    return self._call('dino_sht_inverse_adjoint', g, lead + (self.M, self.L), n)
+    return self._transform('dino_sht_inverse_adjoint', g, (self.I, self.J),
+                           (self.M, self.L), 'inverse_adjoint')
 
   def forward_adjoint(self, g: torch.Tensor) -> torch.Tensor:
-    self._check(g, (self.M, self.L), 'forward_adjoint')
-    lead = g.shape[:-2]
-    n = int(np.prod(lead)) if lead else 1
-    return self._call('dino_sht_forward_adjoint', g, lead + (self.I, self.J), n)
+    return self._transform('dino_sht_forward_adjoint', g, (self.M, self.L),
+                           (self.I, self.J), 'forward_adjoint')
 
   def describe(self) -> str:
     """Shapes, Legendre form and (split-BF16) the autotuned launch shapes."""
@@ -406,15 +409,12 @@ class CudaSphericalHarmonics(SphericalHarmonics):
     return _SphericalHarmonicBasis(f=f, p=p, w=w)
 
   def inverse_transform(self, x):
-    from dinosaur_b200 import autograd  # pylint: disable=g-import-not-at-top
     return autograd.sht_inverse(self.plan, as_device_tensor(x))
 
   def transform(self, x):
-    from dinosaur_b200 import autograd  # pylint: disable=g-import-not-at-top
     return autograd.sht_forward(self.plan, as_device_tensor(x))
 
   def longitudinal_derivative(self, x):
-    from dinosaur_b200 import autograd  # pylint: disable=g-import-not-at-top
     return autograd.modal_op(self.plan, 'd_dlon', as_device_tensor(x))
 
 
@@ -726,7 +726,6 @@ class Grid:
 
   # -- operators -------------------------------------------------------------
   def _op(self, name, x, arg=0):
-    from dinosaur_b200 import autograd  # pylint: disable=g-import-not-at-top
     out = autograd.modal_op(self.plan, name, to_real_layout(self, x), arg,
                             radius=1.0)
     return from_real_layout(self, out)
