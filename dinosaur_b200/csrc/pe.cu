@@ -9,9 +9,10 @@
 // described in include/dino_b200.h; one explicit evaluation is
 //   modal pre-pass -> inverse SHT -> fused nodal column kernel ->
 //   forward SHT -> modal post-pass,
-// and each RK stage is an elementwise combine over all planes plus one
-// per-(m, l) kernel for the implicit solve, the implicit terms of the
-// solution, the final combination and the filter.
+// and in a step the post-pass also forms the RK stage: its implicit planes go
+// in an l-major layout to one per-l operator product (the implicit solve, the
+// implicit terms of the solution, or the final combination and the filter),
+// whose result is scattered back into the state.
 
 #include <cmath>
 #include <cstring>

@@ -25,9 +25,10 @@ namespace dino {
 // Legendre contraction, FP32 SIMT
 // ---------------------------------------------------------------------------
 
+// A CTA has TB (field, cos/sin) rows and as many threads: 128, or 64 for short
+// batches (leg_rows).
 constexpr int kLegTN = 32;   // latitudes (inverse) per CTA
 constexpr int kLegKC = 16;   // contraction chunk
-// (field, cos/sin) rows, and threads, per CTA: 128, or 64 for short batches.
 
 // Row r of the m-slice: m == 0 has one row per field (cos), m > 0 has two.
 __device__ __forceinline__ void row_map(int m, int r, int& b, int& row) {
