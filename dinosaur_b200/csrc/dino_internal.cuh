@@ -60,7 +60,10 @@ int check_launch(const char* what);
 // plain launch would wait out.  Every kernel launched so calls pdl_wait() on
 // every path before it touches memory that an earlier kernel writes or reads,
 // so each still sees the whole of its predecessor (and, by the predecessor's
-// own wait, of everything before it).  Grids below kPdlMinCtas launch plainly:
+// own wait, of everything before it).  A kernel that takes something exclusive
+// on its SM before pdl_wait() (TMEM) calls pdl_trigger() only once it holds it:
+// no dependent CTA may exist while a predecessor's CTA still has to get its
+// share.  Grids below kPdlMinCtas launch plainly:
 // in a captured graph a programmatic edge between two short kernels costs more
 // than the tail it hides (T21 / 12 steps 517 us plainly, 551 with every launch
 // overlapped and 498 from 250 CTAs on; T85 shallow water 496, 620 and 497; T42 /

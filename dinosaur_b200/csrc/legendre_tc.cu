@@ -828,8 +828,8 @@ legendre_tc_kernel(const __grid_constant__ CUtensorMap tBh,
   const int m = a.m0 + blockIdx.y;
   const int tile = blockIdx.x;
   const int rows = (m == 0) ? a.nf : 2 * a.nf;
-  pdl_trigger();
   if (tile * 128 >= rows) {  // uniform for the CTA
+    pdl_trigger();
     pdl_wait();
     return;
   }
@@ -855,6 +855,7 @@ legendre_tc_kernel(const __grid_constant__ CUtensorMap tBh,
   }
   // Uniform early exits: no output column in this range.
   if ((kForward && cnt[0] == 0) || (!kForward && lo >= a.Jh)) {
+    pdl_trigger();
     pdl_wait();
     return;
   }
@@ -903,6 +904,10 @@ legendre_tc_kernel(const __grid_constant__ CUtensorMap tBh,
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
+  // Not before: a dependent contraction's CTA allocates TMEM ahead of its own
+  // pdl_wait, and could take the columns that this CTA still had to allocate,
+  // each then waiting for the other for good.
+  pdl_trigger();
   // Parity p accumulates at column p * Nsub (its corrections, when separate,
   // at (2 + p) * Nsub).
   const int acc_cols = a.Nsub;

@@ -1,0 +1,91 @@
+"""Rules of the kernels that may start while their predecessor finishes.
+
+``launch_pdl`` lets a grid come up during the last wave of the one before it,
+and a broken rule shows on the GPU only as a hang or a wrong value that depends
+on timing.  So the rules are read from the sources: these tests need no GPU.
+"""
+
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                    'dinosaur_b200', 'csrc')
+
+
+def source(path):
+  with open(path) as f:
+    text = f.read()
+  text = re.sub(r'/\*.*?\*/', ' ', text, flags=re.S)
+  return re.sub(r'//[^\n]*', ' ', text)
+
+
+SOURCES = {os.path.basename(p): source(p)
+           for p in sorted(glob.glob(os.path.join(CSRC, '*.cu*')))}
+
+
+def closing(text, start, pair):
+  """Index just past the bracket that closes text[start]."""
+  depth = 0
+  for i in range(start, len(text)):
+    depth += {pair[0]: 1, pair[1]: -1}.get(text[i], 0)
+    if depth == 0:
+      return i + 1
+  raise ValueError('unbalanced')
+
+
+def kernels():
+  """{name: (parameter list, body)} of every __global__ function."""
+  out = {}
+  for text in SOURCES.values():
+    for match in re.finditer(r'__global__\s+void\s+(?:__launch_bounds__\s*\()?', text):
+      i = match.end()
+      if match.group().rstrip().endswith('('):
+        i = closing(text, i - 1, '()')
+      name = re.compile(r'\s*(\w+)\s*\(').match(text, i)
+      end = closing(text, name.end() - 1, '()')
+      brace = text.index('{', end)
+      out[name.group(1)] = (text[name.end():end - 1], text[brace:closing(text, brace, '{}')])
+  return out
+
+
+KERNELS = kernels()
+DEPENDENT = sorted(k for k, (_, body) in KERNELS.items() if 'pdl_' in body)
+
+
+def test_the_kernels_are_found():
+  assert {'legendre_tc_kernel', 'legendre_forward_simt', 'rfft_inverse_kernel',
+          'pe_nodal_hybrid_kernel', 'swe_stage_kernel'} <= set(DEPENDENT)
+
+
+TENSOR_MEMORY = sorted(k for k, (_, body) in KERNELS.items() if 'tcgen05.alloc' in body)
+
+
+@pytest.mark.parametrize('name', TENSOR_MEMORY)
+def test_dependents_start_only_after_tensor_memory_is_held(name):
+  # A dependent CTA allocates tensor memory before it waits for its predecessor.
+  # If a CTA of the predecessor could still have to allocate then, the dependent
+  # could take the columns it needs and each would wait for the other for good.
+  _, body = KERNELS[name]
+  # Paths that return early hold no tensor memory.
+  body = re.sub(r'\{[^{}]*\breturn\s*;[^{}]*\}', ' ', body)
+  assert body.count('pdl_trigger()') == 1
+  before = body[:body.index('pdl_trigger()')]
+  # One thread's trigger counts for its CTA: the CTA's barrier lies between.
+  assert 'tcgen05.alloc' in before
+  assert '__syncthreads()' in before[before.index('tcgen05.alloc'):]
+
+
+@pytest.mark.parametrize('name', DEPENDENT)
+def test_every_dependent_kernel_waits(name):
+  # On every path: once at least, and before each early return.
+  _, body = KERNELS[name]
+  assert 'pdl_wait()' in body
+  first = body.index('pdl_wait()')
+  for match in re.finditer(r'\breturn\s*;', body):
+    assert match.start() > first, name
+  for match in re.finditer(r'\{([^{}]*)\breturn\s*;[^{}]*\}', body):
+    if match.start() < body.rindex('pdl_wait()'):
+      assert 'pdl_wait()' in match.group(1), name

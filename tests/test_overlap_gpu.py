@@ -17,6 +17,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
+from dinosaur_b200 import _lib  # noqa: E402
 from dinosaur_b200 import coordinate_systems  # noqa: E402
 from dinosaur_b200 import primitive_equations as pe  # noqa: E402
 from dinosaur_b200 import sigma_coordinates  # noqa: E402
@@ -41,7 +42,30 @@ def field(grid, lead, power, seed):
     ('T21', 3, 'fp32'), ('TL95', 70, 'fp32'), ('T85', 150, 'bf16x3'),
     ('TL255', 130, 'bf16x3'), ('TL127', 40, 'tf32x3')])
 def test_transforms_in_a_row(name, fields, precision):
+  check_transforms_in_a_row(grid_of(name, precision), fields)
+
+
+@pytest.mark.parametrize('name,fields,precision,inverse,forward', [
+    ('T213', 70, 'bf16x3', '160x2', '112x2'), ('TL255', 130, 'bf16x3', '128x2', '144x2'),
+    ('T106', 70, 'tf32x3', '80x2', '64x2'), ('TL127', 70, 'tf32x3', '64x2', '80x2')])
+def test_contractions_that_fill_tensor_memory_in_a_row(name, fields, precision, inverse,
+                                                       forward, monkeypatch):
+  # Launch shapes of which one CTA takes all 512 columns of tensor memory (the
+  # inverse at T213 and T106, the forward at TL255 and TL127) while the shared
+  # memory holds two: the CTAs of a launch and of its dependent queue for them,
+  # between a forward and the next inverse transform and in the timed launches
+  # of the plan's own set-up.
+  monkeypatch.setenv('DINO_B200_TC_SHAPE', f'inv:{inverse},fwd:{forward}')
   g = grid_of(name, precision)
+  described = g.plan.describe()
+  for shape in (inverse, forward):
+    rows, stages = shape.split('x')
+    assert f'ranges of {rows} rows, {stages} stages' in described, described
+  check_transforms_in_a_row(g, fields)
+  _lib.check(_lib.lib().dino_plan_status(g.plan.handle))
+
+
+def check_transforms_in_a_row(g, fields):
   xs = [field(g, (fields,), 1.5, s) for s in (0, 1)]
   def chain(x):
     n = g.to_nodal(x)
