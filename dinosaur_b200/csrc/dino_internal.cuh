@@ -63,7 +63,10 @@ int check_launch(const char* what);
 // own wait, of everything before it).  A kernel that takes something exclusive
 // on its SM before pdl_wait() (TMEM) calls pdl_trigger() only once it holds it:
 // no dependent CTA may exist while a predecessor's CTA still has to get its
-// share.  Grids below kPdlMinCtas launch plainly:
+// share.  Nor does such a kernel read a predecessor's results with __ldg or
+// through const __restrict__, which promise data that stays as it is for the
+// whole of the kernel and so may be read ahead of the wait; only a plan's
+// tables are read so.  Grids below kPdlMinCtas launch plainly:
 // in a captured graph a programmatic edge between two short kernels costs more
 // than the tail it hides (T21 / 12 steps 517 us plainly, 551 with every launch
 // overlapped and 498 from 250 CTAs on; T85 shallow water 496, 620 and 497; T42 /

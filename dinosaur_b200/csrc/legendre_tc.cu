@@ -580,7 +580,7 @@ struct TcInverse {
         const float4* w4 = reinterpret_cast<const float4*>(src - S);
 #pragma unroll
         for (int i = 0; i < W / 4; ++i) {
-          const float4 t = __ldg(w4 + i);
+          const float4 t = w4[i];
           w[u][4 * i] = t.x;
           w[u][4 * i + 1] = t.y;
           w[u][4 * i + 2] = t.z;
@@ -588,7 +588,7 @@ struct TcInverse {
         }
       } else {
 #pragma unroll
-        for (int e = 0; e < 2 * C; ++e) w[u][e + S] = (e < lim) ? __ldg(src + e) : 0.f;
+        for (int e = 0; e < 2 * C; ++e) w[u][e + S] = (e < lim) ? src[e] : 0.f;
       }
     }
   }
@@ -643,7 +643,7 @@ struct TcInverseAny {
         const float4* w4 = reinterpret_cast<const float4*>(src - R);
 #pragma unroll
         for (int i = 0; i < W / 4; ++i) {
-          const float4 t = __ldg(w4 + i);
+          const float4 t = w4[i];
           w[u][4 * i] = t.x;
           w[u][4 * i + 1] = t.y;
           w[u][4 * i + 2] = t.z;
@@ -652,7 +652,7 @@ struct TcInverseAny {
         sh[u] = R;
       } else {
 #pragma unroll
-        for (int e = 0; e < 2 * C; ++e) w[u][e] = (e < lim) ? __ldg(src + e) : 0.f;
+        for (int e = 0; e < 2 * C; ++e) w[u][e] = (e < lim) ? src[e] : 0.f;
       }
     }
   }
@@ -703,8 +703,8 @@ struct TcForward {
         // float4 (J and j0 are multiples of 4).
 #pragma unroll
         for (int i = 0; i < C / 4; ++i) {
-          const float4 f = __ldg(reinterpret_cast<const float4*>(gr + j0 + 4 * i));
-          const float4 g = __ldg(reinterpret_cast<const float4*>(gr + a.J - 4 * (i + 1) - j0));
+          const float4 f = *reinterpret_cast<const float4*>(gr + j0 + 4 * i);
+          const float4 g = *reinterpret_cast<const float4*>(gr + a.J - 4 * (i + 1) - j0);
           d[u][4 * i] = f.x; d[u][4 * i + 1] = f.y; d[u][4 * i + 2] = f.z; d[u][4 * i + 3] = f.w;
           e[u][4 * i] = g.w; e[u][4 * i + 1] = g.z; e[u][4 * i + 2] = g.y; e[u][4 * i + 3] = g.x;
         }
@@ -714,8 +714,8 @@ struct TcForward {
           const int j = j0 + t;
           if (j < a.Jh) {
             const int jm = a.J - 1 - j;
-            d[u][t] = __ldg(gr + j);
-            e[u][t] = (jm != j) ? __ldg(gr + jm) : 0.f;
+            d[u][t] = gr[j];
+            e[u][t] = (jm != j) ? gr[jm] : 0.f;
           }
         }
       }

@@ -790,10 +790,8 @@ __global__ void __launch_bounds__(kHybThreads) pe_nodal_hybrid_kernel(HybridArgs
   const int j = (int)(col % (unsigned)a.J);
   const float sec2 = a.lat[j];
   const float fcor = a.lat[a.J + j];
-  // The inputs are read-only for the kernel's duration: read-only loads may
-  // run ahead of the output stores.
   auto ld = [&](int base, int k) -> float {
-    return __ldg(a.nod + ((size_t)base + (size_t)mb * K + k) * IJ + col);
+    return a.nod[((size_t)base + (size_t)mb * K + k) * IJ + col];
   };
   auto st = [&](int base, int k, float v) {
     a.fwd[((size_t)base + (size_t)mb * K + k) * IJ + col] = v;
@@ -804,13 +802,13 @@ __global__ void __launch_bounds__(kHybThreads) pe_nodal_hybrid_kernel(HybridArgs
   auto pr_if = [&](int i) -> float { return i < K ? lev(i, 8) : s_hyb[K * kHybPack + 2]; };
   auto ipr_if = [&](int i) -> float { return i < K ? lev(i, 12) : s_hyb[K * kHybPack + 3]; };
   auto bpr_if = [&](int i) -> float { return i < K ? lev(i, 13) : s_hyb[K * kHybPack + 4]; };
-  const float gx = __ldg(a.nod + ((size_t)a.p_gx + mb) * IJ + col);
-  const float gy = __ldg(a.nod + ((size_t)a.p_gy + mb) * IJ + col);
+  const float gx = a.nod[((size_t)a.p_gx + mb) * IJ + col];
+  const float gy = a.nod[((size_t)a.p_gy + mb) * IJ + col];
   const float psr = a.ps_ref;
   // The uniform part c_00 / (2 sqrt(pi)) - ln p_s_ref in FP64: both terms
   // are ~45 and their FP32 roundings would be ~5e-6 of a difference ~1e-2.
   const float rel = (float)((double)a.lnps_modal[(size_t)mb * a.ML] * a.inv_y00 - a.ln_ps_ref) +
-                    __ldg(a.nod + ((size_t)a.p_lnps + mb) * IJ + col);
+                    a.nod[((size_t)a.p_lnps + mb) * IJ + col];
   const float ps = psr * expf(rel);
   const float dps = psr * expm1f(rel);  // p_s - p_s_ref
   const float floor_s = 1e-6f * ps, floor_r = 1e-6f * psr;

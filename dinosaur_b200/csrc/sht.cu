@@ -205,7 +205,7 @@ legendre_inverse_simt(Segs in, float* __restrict__ out, int B, int M, int L,
 // 47.6.
 template <int TN, int TB>
 __global__ void __launch_bounds__(TB)
-legendre_forward_simt(const float* __restrict__ G, float* __restrict__ out,
+legendre_forward_simt(const float* G, float* __restrict__ out,
                       int B, int M, int L, int J, int Jh,
                       const float* __restrict__ ptab,
                       const int64_t* __restrict__ ptab_off) {
@@ -764,7 +764,7 @@ __device__ __forceinline__ void fft_passes(float4* S, const float4* tw, First fi
 // The two columns of a row for one thread: one 8-byte access when kVec (even
 // J and 8-byte aligned bases, so `cols` is 0 or 2), else scalar ones.
 template <bool kVec>
-__device__ __forceinline__ float2 ld_cols(const float* __restrict__ g, int cols) {
+__device__ __forceinline__ float2 ld_cols(const float* g, int cols) {
   if (kVec)
     return cols ? *reinterpret_cast<const float2*>(g) : make_float2(0.f, 0.f);
   return make_float2(cols > 0 ? g[0] : 0.f, cols > 1 ? g[1] : 0.f);
@@ -789,7 +789,7 @@ __device__ __forceinline__ void st_cols(float* g, float2 v, int cols) {
 // in place in shared memory and the last writes the nodal rows.
 template <int N, bool kVec>
 __global__ void __launch_bounds__(FftCfg<N>::threads, FftCfg<N>::ctas)
-rfft_inverse_kernel(const float* __restrict__ F, float* __restrict__ out,
+rfft_inverse_kernel(const float* F, float* __restrict__ out,
                     int M, int lw, int J, const float2* __restrict__ tw_n,
                     const float2* __restrict__ tw_i,
                     const float* __restrict__ wq) {
@@ -875,7 +875,7 @@ rfft_inverse_kernel(const float* __restrict__ F, float* __restrict__ out,
 // U = -i conj(w_I^k) d, X[k] = s + U and X[N-k] = conj(s - U).
 template <int N, bool kVec>
 __global__ void __launch_bounds__(FftCfg<N>::threads, FftCfg<N>::ctas)
-rfft_forward_kernel(const float* __restrict__ x, float* __restrict__ F, int M,
+rfft_forward_kernel(const float* x, float* __restrict__ F, int M,
                     int lw, int J, const float2* __restrict__ tw_n,
                     const float2* __restrict__ tw_i,
                     const float* __restrict__ wq) {
@@ -943,7 +943,7 @@ rfft_forward_kernel(const float* __restrict__ x, float* __restrict__ F, int M,
 
 // Generic longitude transforms by direct summation with the FP32 real basis
 // f[i][row] (any I, any lw <= I).
-__global__ void dft_inverse_kernel(const float* __restrict__ F,
+__global__ void dft_inverse_kernel(const float* F,
                                    float* __restrict__ out, int M, int I, int J,
                                    const float* __restrict__ f,
                                    const float* __restrict__ wq) {
@@ -961,7 +961,7 @@ __global__ void dft_inverse_kernel(const float* __restrict__ F,
   out[((size_t)b * I + i) * J + j] = acc;
 }
 
-__global__ void dft_forward_kernel(const float* __restrict__ x,
+__global__ void dft_forward_kernel(const float* x,
                                    float* __restrict__ F, int M, int I, int J,
                                    const float* __restrict__ f,
                                    const float* __restrict__ wq) {

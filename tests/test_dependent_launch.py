@@ -89,3 +89,25 @@ def test_every_dependent_kernel_waits(name):
   for match in re.finditer(r'\{([^{}]*)\breturn\s*;[^{}]*\}', body):
     if match.start() < body.rindex('pdl_wait()'):
       assert 'pdl_wait()' in match.group(1), name
+
+
+# Plan tables: written once when the plan is made, before any launch of these kernels.
+TABLES = {'ptab', 'ptab_off', 'tw_n', 'tw_i', 'wq', 'f'}
+
+
+@pytest.mark.parametrize('name', DEPENDENT)
+def test_earlier_results_are_not_declared_read_only(name):
+  # A const __restrict__ pointer says that nothing writes what it points to while
+  # the kernel runs, and lets its loads move over the wait; the predecessor may
+  # still be writing then.
+  parameters, _ = KERNELS[name]
+  read_only = re.findall(r'const\s+\w+\s*\*\s*__restrict__\s+(\w+)', parameters)
+  assert set(read_only) <= TABLES, name
+
+
+def test_no_read_only_loads():
+  # __ldg and ld.global.nc make the same promise wherever they are called.
+  for name, text in SOURCES.items():
+    assert '__ldg' not in text and 'ld.global.nc' not in text, name
+    for match in re.finditer(r'__device__[^;{]*?\(([^)]*)\)\s*\{', text):
+      assert not re.search(r'const[^,]*\*\s*__restrict__', match.group(1)), name

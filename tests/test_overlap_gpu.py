@@ -2,11 +2,12 @@
 that are waited for.
 
 Kernels of large grids start while their predecessor is finishing, so a missing
-wait would let one read or overwrite what the other still uses.  Transforms,
-operators and steps run in a row on alternating inputs, without any
-synchronisation, on grids with one and with several chunks per transform and
-grids below and above the size from which launches overlap; every result must
-equal, bit for bit, the one of a call that was waited for.
+wait would let one read or overwrite what the other still uses.  Transforms
+(with the real FFT and with direct sums, at all precisions), operators, and
+steps and gradients of every form of the equations run in a row on alternating
+inputs, without any synchronisation, on grids with one and with several chunks
+per transform and grids below and above the size from which launches overlap;
+every result must equal, bit for bit, the one of a call that was waited for.
 """
 
 import functools
@@ -19,7 +20,11 @@ pytestmark = pytest.mark.gpu
 
 from dinosaur_b200 import _lib  # noqa: E402
 from dinosaur_b200 import coordinate_systems  # noqa: E402
+from dinosaur_b200 import held_suarez  # noqa: E402
+from dinosaur_b200 import hybrid_coordinates  # noqa: E402
+from dinosaur_b200 import layer_coordinates  # noqa: E402
 from dinosaur_b200 import primitive_equations as pe  # noqa: E402
+from dinosaur_b200 import shallow_water  # noqa: E402
 from dinosaur_b200 import sigma_coordinates  # noqa: E402
 from dinosaur_b200 import spherical_harmonic as sh  # noqa: E402
 from dinosaur_b200 import time_integration as ti  # noqa: E402
@@ -84,30 +89,19 @@ def check_transforms_in_a_row(g, fields):
       assert torch.equal(a, b)
 
 
-@pytest.mark.parametrize('name,layers,members', [('T21', 5, 1), ('T42', 12, 6), ('TL127', 6, 1)])
-def test_steps_and_gradients_in_a_row(name, layers, members):
-  g = grid_of(name, 'fp32')
-  coords = coordinate_systems.CoordinateSystem(
-      g, sigma_coordinates.SigmaCoordinates.equidistant(layers))
-  eq = pe.PrimitiveEquationsSigma(np.linspace(220.0, 290.0, layers),
-                                  field(g, (), 2.0, 9).cpu().numpy() * 1e-4, coords,
-                                  units.SimUnits())
-  lead = (members,) if members > 1 else ()
-  def state(s):
-    lnps = 0.02 * field(g, lead + (1,), 2.0, s + 3)
-    lnps[..., 0, 0] += 2 * np.sqrt(np.pi) * 45.0
-    return pe.State(0.05 * field(g, lead + (layers,), 1.0, s),
-                    0.005 * field(g, lead + (layers,), 1.0, s + 1),
-                    5.0 * field(g, lead + (layers,), 1.5, s + 2), lnps)
-  step = ti.repeated(ti.imex_rk_sil3(eq, 0.05), 2)
-  leaves = lambda s: [s.vorticity, s.divergence, s.temperature_variation,
-                      s.log_surface_pressure]
-  def run(s):
-    xs = [x.detach().clone().requires_grad_(True) for x in leaves(s)]
-    out = leaves(step(pe.State(*xs)))
-    sum(o.square().sum() for o in out).backward()
-    return leaves(step(s)) + [o.detach() for o in out] + [x.grad for x in xs]
-  states = [state(10), state(20)]
+@pytest.mark.parametrize('wavenumbers,fields', [(7, 5), (70, 30)])
+def test_direct_longitude_sums_in_a_row(wavenumbers, fields):
+  # 3 N + 1 longitudes: no real FFT; few and many CTAs.
+  check_transforms_in_a_row(sh.Grid.with_wavenumbers(wavenumbers), fields)
+
+
+def leaves(s):
+  return [s.vorticity, s.divergence, s.temperature_variation, s.log_surface_pressure,
+          *s.tracers.values()]
+
+
+def check_in_a_row(run, states):
+  """run(state) -> list of tensors: unsynchronised calls on alternating states."""
   want = []
   for s in states:
     want.append([t.clone() for t in run(s)])
@@ -116,4 +110,61 @@ def test_steps_and_gradients_in_a_row(name, layers, members):
   torch.cuda.synchronize()
   for i, out in enumerate(got):
     for a, b in zip(out, want[i % 2]):
+      assert torch.isfinite(a).all()
       assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize('form,name,layers,members,precision', [
+    ('dry', 'T21', 5, 1, 'fp32'), ('dry', 'T42', 12, 6, 'fp32'), ('dry', 'TL127', 6, 1, 'fp32'),
+    ('moist', 'T21', 5, 1, 'fp32'), ('moist', 'T42', 9, 6, 'fp32'),
+    ('held_suarez', 'T42', 9, 6, 'fp32'), ('hybrid', 'TL127', 6, 2, 'fp32'),
+    ('hybrid', 'TL127', 6, 2, 'tf32x3'), ('moist', 'TL127', 6, 2, 'bf16x3')])
+def test_steps_and_gradients_in_a_row(form, name, layers, members, precision):
+  g = grid_of(name, precision)
+  if form == 'hybrid':
+    vertical = hybrid_coordinates.HybridCoordinates.analytic_ecmwf_like(layers)
+  else:
+    vertical = sigma_coordinates.SigmaCoordinates.equidistant(layers)
+  coords = coordinate_systems.CoordinateSystem(g, vertical)
+  tref = np.linspace(220.0, 290.0, layers)
+  kw = dict(humidity_key='specific_humidity') if form == 'moist' else {}
+  cls = pe.PrimitiveEquationsHybrid if form == 'hybrid' else pe.PrimitiveEquationsSigma
+  specs = units.SimUnits()
+  eq = cls(tref, field(g, (), 2.0, 9).cpu().numpy() * 1e-4, coords, specs, **kw)
+  if form == 'held_suarez':
+    eq = ti.compose_equations([eq, held_suarez.HeldSuarezForcingSigma(coords, specs, tref)])
+  lead = (members,) if members > 1 else ()
+  def state(s):
+    lnps = 0.02 * field(g, lead + (1,), 2.0, s + 3)
+    lnps[..., 0, 0] += 2 * np.sqrt(np.pi) * 45.0
+    tracers = {}
+    if form == 'moist':
+      tracers['specific_humidity'] = 1e-3 * field(g, lead + (layers,), 1.5, s + 4)
+    return pe.State(0.05 * field(g, lead + (layers,), 1.0, s),
+                    0.005 * field(g, lead + (layers,), 1.0, s + 1),
+                    5.0 * field(g, lead + (layers,), 1.5, s + 2), lnps, tracers=tracers)
+  step = ti.repeated(ti.imex_rk_sil3(eq, 0.05), 2)
+  def run(s):
+    if form == 'hybrid':  # no step VJP
+      return leaves(step(s)) + leaves(eq.explicit_terms(s))
+    xs = [x.detach().clone().requires_grad_(True) for x in leaves(s)]
+    out = leaves(step(pe.State(*xs[:4], tracers=dict(zip(s.tracers, xs[4:])))))
+    sum(o.square().sum() for o in out).backward()
+    return leaves(step(s)) + [o.detach() for o in out] + [x.grad for x in xs]
+  check_in_a_row(run, [state(10), state(20)])
+
+
+@pytest.mark.parametrize('name,layers,members', [('T21', 2, 1), ('TL127', 3, 4)])
+def test_shallow_water_steps_in_a_row(name, layers, members):
+  g = grid_of(name, 'fp32')
+  coords = coordinate_systems.CoordinateSystem(g, layer_coordinates.LayerCoordinates(layers))
+  eq = shallow_water.ShallowWaterEquations(
+      coords, units.SimUnits(), field(g, (), 2.0, 9).cpu().numpy() * 1e-3,
+      np.linspace(0.04, 0.06, layers), densities=np.linspace(1.0, 1.5, layers))
+  lead = (members, layers) if members > 1 else (layers,)
+  state = lambda s: shallow_water.State(0.05 * field(g, lead, 1.0, s),
+                                        0.005 * field(g, lead, 1.0, s + 1),
+                                        0.005 * field(g, lead, 1.0, s + 2))
+  step = ti.repeated(ti.imex_rk_sil3(eq, 0.05), 2)
+  check_in_a_row(lambda s: [*vars(step(s)).values(), *vars(eq.explicit_terms(s)).values()],
+                 [state(10), state(20)])
