@@ -466,7 +466,8 @@ template <int kSign>
 __device__ __forceinline__ cpair csub_i(cpair a, cpair b) {
   return cadd_i<-kSign>(a, b);
 }
-// a (wr + i wi), the same factor for both columns; nwi = -wi.
+// a (wr + i wi), the same factor for both columns; nwi = -wi.  One product of
+// each part is rounded, the other is inside the FMA.
 __device__ __forceinline__ cpair cmul_w(cpair a, float2 wr, float2 wi, float2 nwi) {
   return {pfma(a.re, wr, pmul(a.im, nwi)), pfma(a.re, wi, pmul(a.im, wr))};
 }
@@ -724,8 +725,7 @@ __device__ __forceinline__ void stockham_pass(const float4* tw, Load load, Store
         for (int r = 1; r < R; ++r) {
           const float4 w = tw[r * k * stride];
           const float2 wr = make_float2(w.x, w.y), wi = make_float2(w.z, w.w);
-          const cpair a = v[it][r];
-          v[it][r] = {psub(pmul(a.re, wr), pmul(a.im, wi)), pfma(a.re, wi, pmul(a.im, wr))};
+          v[it][r] = cmul_w(v[it][r], wr, wi, pmul(wi, dup(-1.f)));
         }
       }
       dft_reg<R, kSign>(v[it]);
@@ -852,7 +852,7 @@ rfft_inverse_kernel(const float* F, float* __restrict__ out,
       const float2 w = tw_i[k];
       const float2 wr = dup(w.x), wi = dup(w.y);
       const float2 tr = pfma(br, wr, pmul(q, wi));
-      const float2 ti = psub(pmul(br, wi), pmul(q, wr));
+      const float2 ti = pfma(br, wi, pmul(q, dup(-w.x)));
       st_cpair(S + k * P + p, {psub(ar, ti), padd(ai, tr)});
       st_cpair(S + (N - k) * P + p, {padd(ar, ti), psub(tr, ai)});
     }
@@ -928,7 +928,7 @@ rfft_forward_kernel(const float* x, float* __restrict__ F, int M,
     const float2 wr = dup(w.x), wi = dup(w.y);
     const float2 sr = padd(zk.re, zn.re), si = psub(zk.im, zn.im);  // 2 s
     const float2 dr = psub(zk.re, zn.re), di = padd(zk.im, zn.im);  // 2 d
-    const float2 ur = psub(pmul(wr, di), pmul(wi, dr));
+    const float2 ur = pfma(wr, di, pmul(dup(-w.y), dr));
     const float2 v = pfma(wi, di, pmul(wr, dr));  // -Im 2U
     if (k < lw) {
       st_cols<kVec>(fk, pmul(padd(sr, ur), ah), cols);
