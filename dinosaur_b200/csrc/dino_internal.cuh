@@ -110,6 +110,18 @@ __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// A new device array with the values of src.  A copy from pageable memory may
+// return before its last part has arrived, and a caller's non-blocking stream
+// does not wait for the default one, so the copy is waited for.
+template <typename T>
+int upload(T** dst, const std::vector<T>& src) {
+  DINO_CHECK_CUDA(cudaMalloc((void**)dst, sizeof(T) * (src.empty() ? 1 : src.size())));
+  if (src.empty()) return DINO_OK;
+  DINO_CHECK_CUDA(cudaMemcpy(*dst, src.data(), sizeof(T) * src.size(), cudaMemcpyHostToDevice));
+  DINO_CHECK_CUDA(cudaStreamSynchronize(0));
+  return DINO_OK;
+}
+
 // An NVTX range over the enclosing scope, so that profilers group the
 // kernels a phase launches under the reference's names for its phases
 // (inv_legendre, inv_fourier, fwd_fourier, fwd_legendre: the named calls of

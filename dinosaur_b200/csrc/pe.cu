@@ -2259,9 +2259,7 @@ static int get_matrix(dino_pe* pe, int kind, double eta, const double* host_filt
   if (host_filter) consts.insert(consts.end(), host_filter, host_filter + L);
   double* dc = nullptr;
   auto build = [&]() -> int {
-    DINO_CHECK_CUDA(cudaMalloc(&dc, sizeof(double) * consts.size()));
-    DINO_CHECK_CUDA(cudaMemcpy(dc, consts.data(), sizeof(double) * consts.size(),
-                               cudaMemcpyHostToDevice));
+    DINO_TRY(upload(&dc, consts));
     DINO_CHECK_CUDA(cudaMalloc(&m.d, sizeof(float) * (size_t)L * m.nin * m.RP));
     DINO_CHECK_CUDA(cudaMemset(pe->d_flag, 0, sizeof(int)));
     MatBuildArgs b{};
@@ -2313,9 +2311,12 @@ static int get_filter(dino_pe* pe, const double* host, float** out) {
   }
   std::vector<float> f(pe->L);
   for (int l = 0; l < pe->L; ++l) f[l] = (float)host[l];
-  float* d;
-  DINO_CHECK_CUDA(cudaMalloc(&d, sizeof(float) * pe->L));
-  DINO_CHECK_CUDA(cudaMemcpy(d, f.data(), sizeof(float) * pe->L, cudaMemcpyHostToDevice));
+  float* d = nullptr;
+  const int rc = upload(&d, f);
+  if (rc != DINO_OK) {
+    cudaFree(d);
+    return rc;
+  }
   pe->filter_cache.push_back({std::vector<double>(host, host + pe->L), d});
   *out = d;
   return DINO_OK;
@@ -2916,14 +2917,6 @@ static int pe_step_vjp_impl(dino_pe* pe, const float* y, const float* out_ct,
   return DINO_OK;
 }
 
-template <typename T>
-static int upload_vec(T** dst, const std::vector<T>& v) {
-  DINO_CHECK_CUDA(cudaMalloc((void**)dst, sizeof(T) * (v.empty() ? 1 : v.size())));
-  if (!v.empty())
-    DINO_CHECK_CUDA(cudaMemcpy(*dst, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice));
-  return DINO_OK;
-}
-
 static void pe_free(dino_pe* pe) {
   if (!pe) return;
   if (pe->graph.exec) cudaGraphExecDestroy(pe->graph.exec);
@@ -3016,7 +3009,7 @@ static int pe_build(dino_pe* pe, const dino_pe_desc* d) {
     hp[(size_t)K * kHybPack + 2] = (float)pK;
     hp[(size_t)K * kHybPack + 3] = (float)(1.0 / std::max(pK, 1e-6 * psr));
     hp[(size_t)K * kHybPack + 4] = (float)(B[K] / std::max(pK, 1e-6 * psr));
-    DINO_TRY(upload_vec(&pe->d_hyb, hp));
+    DINO_TRY(upload(&pe->d_hyb, hp));
   }
 
   // Level constants.
@@ -3060,7 +3053,7 @@ static int pe_build(dino_pe* pe, const dino_pe_desc* d) {
     q[12] = lev[lo.trefdiff + k];
     q[13] = k > 0 ? lev[lo.trefdiff + k - 1] : 0.f;
   }
-  DINO_TRY(upload_vec(&pe->d_levpack, pack));
+  DINO_TRY(upload(&pe->d_levpack, pack));
   DINO_TRY(nodal_prepare(K));
   {
     int dev = 0;
@@ -3077,11 +3070,11 @@ static int pe_build(dino_pe* pe, const dino_pe_desc* d) {
     lat[2 * J + j] = (float)(std::sin(latr) * std::sin(latr));
     lat[3 * J + j] = (float)(std::cos(latr) * std::cos(latr));
   }
-  DINO_TRY(upload_vec(&pe->d_lat, lat));
+  DINO_TRY(upload(&pe->d_lat, lat));
   {
     std::vector<float> orog(pe->ML, 0.f);
     if (d->orography_modal) std::memcpy(orog.data(), d->orography_modal, sizeof(float) * pe->ML);
-    DINO_TRY(upload_vec(&pe->d_orog, orog));
+    DINO_TRY(upload(&pe->d_orog, orog));
   }
 
   // Field bookkeeping.

@@ -135,15 +135,6 @@ __global__ void legendre_table_kernel(int lw, int L, int Jh,
   }
 }
 
-template <typename T>
-static int upload(T** dst, const std::vector<T>& src) {
-  DINO_CHECK_CUDA(cudaMalloc((void**)dst, sizeof(T) * (src.empty() ? 1 : src.size())));
-  if (!src.empty())
-    DINO_CHECK_CUDA(cudaMemcpy(*dst, src.data(), sizeof(T) * src.size(),
-                               cudaMemcpyHostToDevice));
-  return DINO_OK;
-}
-
 static void plan_free(dino_plan* p) {
   if (!p) return;
   if (p->side) {
@@ -173,19 +164,17 @@ static int plan_build(dino_plan* p, const dino_grid_desc* d) {
   DINO_CHECK_CUDA(cudaGetDevice(&p->device));
 
   // Nodes and weights (FP64).
-  DINO_CHECK_CUDA(cudaMalloc(&p->d_x64, sizeof(double) * J));
-  DINO_CHECK_CUDA(cudaMalloc(&p->d_w64, sizeof(double) * J));
   if (p->spacing == DINO_SPACING_GAUSS) {
+    DINO_CHECK_CUDA(cudaMalloc(&p->d_x64, sizeof(double) * J));
+    DINO_CHECK_CUDA(cudaMalloc(&p->d_w64, sizeof(double) * J));
     int half = (J + 1) / 2;
     gauss_nodes_kernel<<<ceil_div(half, 128), 128>>>(J, p->d_x64, p->d_w64);
     DINO_TRY(check_launch("gauss_nodes"));
   } else {
     DINO_REQUIRE(d->host_nodes && d->host_weights, DINO_ERR_ARG,
                  "non-Gauss latitude spacing needs host_nodes/host_weights");
-    DINO_CHECK_CUDA(cudaMemcpy(p->d_x64, d->host_nodes, sizeof(double) * J,
-                               cudaMemcpyHostToDevice));
-    DINO_CHECK_CUDA(cudaMemcpy(p->d_w64, d->host_weights, sizeof(double) * J,
-                               cudaMemcpyHostToDevice));
+    DINO_TRY(upload(&p->d_x64, std::vector<double>(d->host_nodes, d->host_nodes + J)));
+    DINO_TRY(upload(&p->d_w64, std::vector<double>(d->host_weights, d->host_weights + J)));
   }
   p->h_x64.resize(J);
   p->h_w64.resize(J);

@@ -286,13 +286,6 @@ __global__ void swe_implicit_kernel(SweImplicitArgs a) {
   }
 }
 
-template <typename T>
-int upload(T** dst, const std::vector<T>& v) {
-  DINO_CHECK_CUDA(cudaMalloc(dst, sizeof(T) * v.size()));
-  DINO_CHECK_CUDA(cudaMemcpy(*dst, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice));
-  return DINO_OK;
-}
-
 void swe_free(dino_swe* s) {
   if (!s) return;
   cudaFree(s->d_dens);

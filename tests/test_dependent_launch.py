@@ -1,8 +1,9 @@
-"""Rules of the kernels that may start while their predecessor finishes.
+"""Rules of order between kernels and copies, read from the sources.
 
 ``launch_pdl`` lets a grid come up during the last wave of the one before it,
-and a broken rule shows on the GPU only as a hang or a wrong value that depends
-on timing.  So the rules are read from the sources: these tests need no GPU.
+and callers' streams are not ordered with the default one.  A broken rule shows
+on the GPU only as a hang or a wrong value that depends on timing, so the rules
+are read from the sources: these tests need no GPU.
 """
 
 import glob
@@ -111,3 +112,15 @@ def test_no_read_only_loads():
     assert '__ldg' not in text and 'ld.global.nc' not in text, name
     for match in re.finditer(r'__device__[^;{]*?\(([^)]*)\)\s*\{', text):
       assert not re.search(r'const[^,]*\*\s*__restrict__', match.group(1)), name
+
+
+def test_uploads_are_finished_before_they_return():
+  # A copy from pageable host memory may return while its last part is still on
+  # its way, and kernels on a caller's non-blocking stream do not wait for the
+  # default stream.  So every upload goes through upload(), which waits.
+  copies = {name: text.count('cudaMemcpyHostToDevice') for name, text in SOURCES.items()}
+  assert {k: v for k, v in copies.items() if v} == {'dino_internal.cuh': 1}
+  text = SOURCES['dino_internal.cuh']
+  start = text.index('{', text.index('int upload('))
+  body = text[start:closing(text, start, '{}')]
+  assert body.index('cudaMemcpyHostToDevice') < body.index('cudaStreamSynchronize')
