@@ -14,8 +14,11 @@
 // generic tableau loop over tensors, which the host could not issue as fast as
 // the GPU ran them.
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <exception>
+#include <mutex>
 #include <vector>
 
 #include "dino_internal.cuh"
@@ -35,19 +38,25 @@ struct dino_swe {
   float* d_work = nullptr;
   int work_fields = 0;
   // SIL3 step (allocated by the first one): the state it advances, the two
-  // stage states, f0 and f1, the uploaded filters and the captured step.
+  // stage states, f0 and f1, and the captured steps.
   float* d_y = nullptr;
   float* d_Y[2] = {nullptr, nullptr};
   float* d_f[2] = {nullptr, nullptr};
-  struct Filter {
-    std::vector<double> host;
-    float* dev;
+  // The captured step of one time step and filter (empty: none), with the
+  // filter on the device.  Calls take turns between a few of them (a forward and
+  // a backward sweep, a halved time step); the least recently used goes.
+  struct Step {
+    double dt = 0;
+    std::vector<double> host_filter;
+    float* d_filter = nullptr;
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    uint64_t used = 0;
   };
-  std::vector<Filter> filters;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  double graph_dt = 0;
-  const float* graph_filter = nullptr;
+  static constexpr size_t kMaxSteps = 8;
+  std::vector<Step> steps;
+  uint64_t calls = 0;
+  std::mutex mu;  // held while a step is found and queued
 };
 
 namespace dino {
@@ -286,6 +295,12 @@ __global__ void swe_implicit_kernel(SweImplicitArgs a) {
   }
 }
 
+void step_free(dino_swe::Step* g) {
+  if (g->exec) cudaGraphExecDestroy(g->exec);
+  if (g->graph) cudaGraphDestroy(g->graph);
+  cudaFree(g->d_filter);
+}
+
 void swe_free(dino_swe* s) {
   if (!s) return;
   cudaFree(s->d_dens);
@@ -297,12 +312,10 @@ void swe_free(dino_swe* s) {
   cudaFree(s->d_fwd_in);
   cudaFree(s->d_fwd_out);
   cudaFree(s->d_work);
-  if (s->exec) cudaGraphExecDestroy(s->exec);
-  if (s->graph) cudaGraphDestroy(s->graph);
+  for (auto& g : s->steps) step_free(&g);
   cudaFree(s->d_y);
   for (float* b : s->d_Y) cudaFree(b);
   for (float* b : s->d_f) cudaFree(b);
-  for (auto& f : s->filters) cudaFree(f.dev);
   delete s;
 }
 
@@ -406,56 +419,77 @@ int swe_step_once(dino_swe* s, double dt, const float* filter, cudaStream_t st) 
                     post_args(s, s->d_Y[1], nullptr), a);
 }
 
+// Uploads the filter and captures the step of g.
+int swe_capture(dino_swe* s, dino_swe::Step* g) {
+  if (!g->host_filter.empty())
+    DINO_TRY(upload(&g->d_filter,
+                    std::vector<float>(g->host_filter.begin(), g->host_filter.end())));
+  DINO_TRY(sht_prepare(s->plan));
+  // Captured on a private stream, so that the caller's stream (possibly the
+  // legacy default one) never enters capture mode.
+  cudaStream_t cap;
+  DINO_CHECK_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
+  cudaError_t ce = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
+  int rc = DINO_OK;
+  if (ce == cudaSuccess) {
+    rc = swe_step_once(s, g->dt, g->d_filter, cap);
+    ce = cudaStreamEndCapture(cap, &g->graph);
+  }
+  cudaStreamDestroy(cap);
+  if (rc != DINO_OK) return rc;
+  DINO_CHECK_CUDA(ce);
+  ce = cudaGraphInstantiate(&g->exec, g->graph, 0);
+  if (ce != cudaSuccess) g->exec = nullptr;
+  DINO_CHECK_CUDA(ce);
+  return DINO_OK;
+}
+
+// The captured step of (dt, filter), captured now if it is not among the last.
+int swe_find_step(dino_swe* s, double dt, const double* host_filter, cudaGraphExec_t* exec) {
+  const size_t n = host_filter ? (size_t)s->L : 0;
+  for (auto& g : s->steps)
+    if (g.dt == dt && g.host_filter.size() == n &&
+        (n == 0 || std::memcmp(g.host_filter.data(), host_filter, sizeof(double) * n) == 0)) {
+      g.used = ++s->calls;
+      *exec = g.exec;
+      return DINO_OK;
+    }
+  dino_swe::Step g;
+  g.dt = dt;
+  if (n) g.host_filter.assign(host_filter, host_filter + n);
+  s->steps.reserve(dino_swe::kMaxSteps);
+  const int rc = swe_capture(s, &g);
+  if (rc != DINO_OK) {
+    step_free(&g);
+    return rc;
+  }
+  g.used = ++s->calls;
+  *exec = g.exec;
+  if (s->steps.size() < dino_swe::kMaxSteps) {
+    s->steps.push_back(std::move(g));
+    return DINO_OK;
+  }
+  auto old = std::min_element(s->steps.begin(), s->steps.end(),
+                              [](const auto& a, const auto& b) { return a.used < b.used; });
+  // Its last launch may still be queued and read its filter.
+  DINO_CHECK_CUDA(cudaDeviceSynchronize());
+  step_free(&*old);
+  *old = std::move(g);
+  return DINO_OK;
+}
+
 int swe_step_impl(dino_swe* s, float* state, double dt, const double* host_filter, int n_steps,
                   cudaStream_t st) {
+  std::lock_guard<std::mutex> lock(s->mu);
   const size_t bytes = sizeof(float) * 3 * (size_t)s->mem * s->K * s->ML;
   for (float** b : {&s->d_y, &s->d_Y[0], &s->d_Y[1], &s->d_f[0], &s->d_f[1]})
     if (!*b) DINO_CHECK_CUDA(cudaMalloc(b, bytes));
-  const float* filter = nullptr;
-  if (host_filter) {
-    for (auto& f : s->filters)
-      if (std::memcmp(f.host.data(), host_filter, sizeof(double) * s->L) == 0) filter = f.dev;
-    if (!filter) {
-      std::vector<float> w(s->L);
-      for (int l = 0; l < s->L; ++l) w[l] = (float)host_filter[l];
-      float* dev = nullptr;
-      DINO_TRY(upload(&dev, w));
-      s->filters.push_back({std::vector<double>(host_filter, host_filter + s->L), dev});
-      filter = dev;
-    }
-  }
-  if (!(s->exec && s->graph_dt == dt && s->graph_filter == filter)) {
-    if (s->exec) cudaGraphExecDestroy(s->exec);
-    if (s->graph) cudaGraphDestroy(s->graph);
-    s->exec = nullptr;
-    s->graph = nullptr;
-    DINO_TRY(sht_prepare(s->plan));
-    // Captured on a private stream, so that the caller's stream (possibly the
-    // legacy default one) never enters capture mode.
-    cudaStream_t cap;
-    DINO_CHECK_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-    cudaError_t ce = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
-    int rc = DINO_OK;
-    cudaGraph_t graph = nullptr;
-    if (ce == cudaSuccess) {
-      rc = swe_step_once(s, dt, filter, cap);
-      ce = cudaStreamEndCapture(cap, &graph);
-    }
-    cudaStreamDestroy(cap);
-    if (rc != DINO_OK || ce != cudaSuccess) {
-      if (graph) cudaGraphDestroy(graph);
-      if (rc != DINO_OK) return rc;
-      DINO_CHECK_CUDA(ce);
-    }
-    s->graph = graph;
-    DINO_CHECK_CUDA(cudaGraphInstantiate(&s->exec, graph, 0));
-    s->graph_dt = dt;
-    s->graph_filter = filter;
-  }
+  cudaGraphExec_t exec = nullptr;
+  DINO_TRY(swe_find_step(s, dt, host_filter, &exec));
   // The captured step works on the object's own buffer, so one capture serves
   // every caller's state; two copies a call.
   DINO_CHECK_CUDA(cudaMemcpyAsync(s->d_y, state, bytes, cudaMemcpyDeviceToDevice, st));
-  for (int i = 0; i < n_steps; ++i) DINO_CHECK_CUDA(cudaGraphLaunch(s->exec, st));
+  for (int i = 0; i < n_steps; ++i) DINO_CHECK_CUDA(cudaGraphLaunch(exec, st));
   DINO_CHECK_CUDA(cudaMemcpyAsync(state, s->d_y, bytes, cudaMemcpyDeviceToDevice, st));
   return DINO_OK;
 }
@@ -536,7 +570,12 @@ int dino_swe_step(dino_swe* s, float* state, double dt, const double* host_filte
   DINO_REQUIRE(s && state, DINO_ERR_ARG, "dino_swe_step: null argument");
   DINO_REQUIRE(n_steps >= 0, DINO_ERR_ARG, "n_steps must be >= 0");
   if (n_steps == 0) return DINO_OK;
-  return swe_step_impl(s, state, dt, host_filter, n_steps, (cudaStream_t)stream);
+  try {
+    return swe_step_impl(s, state, dt, host_filter, n_steps, (cudaStream_t)stream);
+  } catch (const std::exception& e) {
+    set_error(std::string("dino_swe_step: ") + e.what());
+    return DINO_ERR_CUDA;
+  }
 }
 
 }  // extern "C"

@@ -313,8 +313,9 @@ DINO_API int dino_swe_implicit_inverse(dino_swe* swe, const float* d_state,
 /* Advances d_state in place by n_steps of imex_rk_sil3 with time step dt
  * (time_integration.py:375-405), each followed by multiplication with the
  * per-l filter scaling (host array of length L; NULL = none), from one
- * captured CUDA graph per (dt, filter).  The first call allocates the step's
- * work buffers; calls on one object must not overlap in time. */
+ * captured CUDA graph per (dt, filter), of which the eight used last are kept.
+ * The first call allocates the step's work buffers; calls on one object must
+ * not overlap in time. */
 DINO_API int dino_swe_step(dino_swe* swe, float* d_state, double dt,
                            const double* host_filter, int32_t n_steps,
                            void* stream);
