@@ -570,6 +570,7 @@ int dino_swe_step(dino_swe* s, float* state, double dt, const double* host_filte
   DINO_REQUIRE(s && state, DINO_ERR_ARG, "dino_swe_step: null argument");
   DINO_REQUIRE(n_steps >= 0, DINO_ERR_ARG, "n_steps must be >= 0");
   if (n_steps == 0) return DINO_OK;
+  DINO_REQUIRE(std::isfinite(dt), DINO_ERR_ARG, "step_size must be finite");
   try {
     return swe_step_impl(s, state, dt, host_filter, n_steps, (cudaStream_t)stream);
   } catch (const std::exception& e) {

@@ -246,3 +246,15 @@ def test_steppers_in_turn_cost_what_one_costs():
   per_call(3)
   one, three = per_call(1), per_call(3)
   assert three < 1.5 * one, (one, three)
+
+
+def generic_stepper(eq, dt):
+  return ti.imex_runge_kutta(ti.SIL3_TABLEAU, eq, dt)
+
+
+@pytest.mark.parametrize('dt', [np.nan, np.inf])
+def test_steppers_refuse_a_time_step_that_is_not_finite(dt):
+  _, eq, state = small_case()
+  for step in (generic_stepper(eq, dt), ti.imex_rk_sil3(eq, dt)):
+    with pytest.raises(ValueError, match='finite'):
+      step(state)
