@@ -16,6 +16,7 @@ which follows the reference step for step.
 from __future__ import annotations
 
 import dataclasses
+import numbers
 from typing import Any, Callable, Sequence
 
 import numpy as np
@@ -336,8 +337,11 @@ def repeated(fn, steps: int, scan_fn=None):
   del scan_fn
   if steps == 1:
     return fn
-  if isinstance(fn, (FusedSIL3Step, FusedShallowWaterStep)):
+  if isinstance(fn, FusedSIL3Step):
     return dataclasses.replace(fn, n_steps=fn.n_steps * steps)
+  if (isinstance(fn, FusedShallowWaterStep) and isinstance(steps, numbers.Integral)
+      and steps > 0):  # the loop below returns the state itself, or refuses
+    return dataclasses.replace(fn, n_steps=fn.n_steps * int(steps))
 
   def f_repeated(x):
     for _ in range(steps):

@@ -258,3 +258,14 @@ def test_steppers_refuse_a_time_step_that_is_not_finite(dt):
   for step in (generic_stepper(eq, dt), ti.imex_rk_sil3(eq, dt)):
     with pytest.raises(ValueError, match='finite'):
       step(state)
+
+
+def test_repeated_takes_the_counts_that_a_loop_takes():
+  _, eq, state = small_case()
+  for step in (generic_stepper(eq, 0.05), ti.imex_rk_sil3(eq, 0.05)):
+    assert ti.repeated(step, 0)(state) is state
+    assert ti.repeated(step, -2)(state) is state
+    with pytest.raises(TypeError):
+      ti.repeated(step, 2.0)(state)
+  two = ti.repeated(ti.imex_rk_sil3(eq, 0.05), np.int64(2))
+  assert isinstance(two, ti.FusedShallowWaterStep) and two.n_steps == 2
