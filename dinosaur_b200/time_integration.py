@@ -318,8 +318,9 @@ def step_with_filters(step_fn, filters: Sequence[Callable]):
       s = np.asarray(f.scaling, np.float64)
       scaling = s if scaling is None else scaling * s
     return dataclasses.replace(step_fn, filter_scaling=scaling)
+  # Exactly this filter: a subclass may do something else.
   if (isinstance(step_fn, FusedShallowWaterStep) and step_fn.n_steps == 1 and all(
-      isinstance(f, SpectralStepFilter) and np.shape(f.scaling) ==
+      type(f) is SpectralStepFilter and np.shape(f.scaling) ==  # pylint: disable=unidiomatic-typecheck
       (step_fn.equation.coords.horizontal.total_wavenumbers,) for f in filters)):
     return dataclasses.replace(step_fn, filters=step_fn.filters + tuple(filters))
 

@@ -269,3 +269,16 @@ def test_repeated_takes_the_counts_that_a_loop_takes():
       ti.repeated(step, 2.0)(state)
   two = ti.repeated(ti.imex_rk_sil3(eq, 0.05), np.int64(2))
   assert isinstance(two, ti.FusedShallowWaterStep) and two.n_steps == 2
+
+
+def test_a_subclass_of_the_spectral_filter_is_called():
+  grid, eq, state = small_case()
+
+  class Halving(ti.SpectralStepFilter):
+
+    def __call__(self, u, u_next):
+      return sw.State(*[0.5 * x for x in vars(u_next).values()])
+
+  step = ti.imex_rk_sil3(eq, 0.05)
+  halved = ti.step_with_filters(step, [Halving(np.ones(grid.total_wavenumbers))])(state)
+  assert torch.equal(halved.potential, 0.5 * step(state).potential)
