@@ -57,16 +57,17 @@ int check_launch(const char* what);
 // Launches a kernel that may start while the one before it on the stream is
 // finishing (programmatic dependent launch): its CTAs are brought up, and do
 // what needs no earlier result, during the predecessor's last wave, which a
-// plain launch would wait out.  Every kernel launched so calls pdl_wait() on
-// every path before it touches memory that an earlier kernel writes or reads,
-// so each still sees the whole of its predecessor (and, by the predecessor's
-// own wait, of everything before it).  A kernel that takes something exclusive
-// on its SM before pdl_wait() (TMEM) calls pdl_trigger() only once it holds it:
-// no dependent CTA may exist while a predecessor's CTA still has to get its
-// share.  Nor does such a kernel read a predecessor's results with __ldg or
-// through const __restrict__, which promise data that stays as it is for the
-// whole of the kernel and so may be read ahead of the wait; only a plan's
-// tables are read so.  Grids below kPdlMinCtas launch plainly:
+// plain launch would wait out.  Three rules hold for every kernel launched so:
+//  - It calls pdl_wait() on every path before it touches memory that an earlier
+//    kernel writes or reads, so it still sees the whole of its predecessor (and,
+//    by the predecessor's own wait, of everything before it).
+//  - If it takes something exclusive on its SM before pdl_wait() (TMEM), it calls
+//    pdl_trigger() only once it holds it: no dependent CTA may exist while a
+//    predecessor's CTA still has to get its share.
+//  - It does not read a predecessor's results with __ldg or through const
+//    __restrict__, which promise data that stays as it is for the whole of the
+//    kernel and so may be read ahead of the wait; only a plan's tables are read so.
+// Grids below kPdlMinCtas (less than two CTAs an SM of this chip) launch plainly:
 // in a captured graph a programmatic edge between two short kernels costs more
 // than the tail it hides (T21 / 12 steps 517 us plainly, 551 with every launch
 // overlapped and 498 from 250 CTAs on; T85 shallow water 496, 620 and 497; T42 /
@@ -200,6 +201,7 @@ struct dino_plan {
   // Shapes.
   int lw = 0, L = 0, I = 0, J = 0, M = 0, Jh = 0, N = 0;
   int spacing = 0, precision = 0, max_fields = 0, device = 0;
+  int sms = 0;  // multiprocessors of the device
   double radius = 1.0;
   bool fft = false;  // I / 2 has a real FFT (else longitude sums are direct)
   // FP64 nodes and weights (device and host copies).

@@ -75,7 +75,6 @@ struct dino_pe {
   float* d_hyb = nullptr;  // per-level constants of pe_nodal_hybrid_kernel
   // Device constants.
   float* d_levpack = nullptr;  // per-level constants, packed per level (kLevPack)
-  int sms = 148;               // multiprocessors of the device
   float* d_lat = nullptr;   // per-latitude constants: sec2, f, sin2, cos2
   float* d_orog = nullptr;  // modal orography [M][L]
   // Field bookkeeping (planes).
@@ -2331,7 +2330,7 @@ static dim3 tile_grid(const dino_pe* pe, int planes) {
 static dim3 modal_grid(const dino_pe* pe, int* ppt) {
   const int tl = ceil_div(pe->L, kModalTX), tr = ceil_div(pe->M, kModalTY);
   const int planes = pe->K * pe->mem;
-  *ppt = planes_per_cta(tl * tr, planes, pe->sms);
+  *ppt = planes_per_cta(tl * tr, planes, pe->plan->sms);
   return dim3(tl, tr, ceil_div(planes, *ppt));
 }
 
@@ -2378,7 +2377,7 @@ static int pe_nodal_inputs(dino_pe* pe, const float* state, cudaStream_t st) {
     a.inv_radius = (float)(1.0 / p->radius);
     // Two planes a CTA where many CTAs remain (TL255 / 32: 19.6 us, one 21.3).
     const dim3 one = tile_grid(pe, 1);
-    const bool many = (int64_t)one.x * one.y * one.z >= 16LL * pe->sms;
+    const bool many = (int64_t)one.x * one.y * one.z >= 16LL * pe->plan->sms;
     DINO_TRY(launch_pdl("pe_prep", pe_prep_kernel, many ? tile_grid(pe, 2) : one,
                         dim3(kModalTX, kModalTY), 0, st, a));
   }
@@ -3055,11 +3054,6 @@ static int pe_build(dino_pe* pe, const dino_pe_desc* d) {
   }
   DINO_TRY(upload(&pe->d_levpack, pack));
   DINO_TRY(nodal_prepare(K));
-  {
-    int dev = 0;
-    DINO_CHECK_CUDA(cudaGetDevice(&dev));
-    DINO_CHECK_CUDA(cudaDeviceGetAttribute(&pe->sms, cudaDevAttrMultiProcessorCount, dev));
-  }
   // Latitude constants: sec^2, Coriolis 2 Omega sin, sin^2, cos^2.
   std::vector<float> lat(4 * J);
   for (int j = 0; j < J; ++j) {

@@ -162,6 +162,7 @@ static void plan_free(dino_plan* p) {
 static int plan_build(dino_plan* p, const dino_grid_desc* d) {
   const int lw = p->lw, L = p->L, I = p->I, J = p->J, M = p->M, Jh = p->Jh;
   DINO_CHECK_CUDA(cudaGetDevice(&p->device));
+  DINO_CHECK_CUDA(cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device));
 
   // Nodes and weights (FP64).
   if (p->spacing == DINO_SPACING_GAUSS) {

@@ -410,7 +410,7 @@ int legendre_forward(dino_plan* p, const float* G, float* out, int nf,
 int legendre_forward_fp32(dino_plan* p, const float* G, float* out, int nf,
                           cudaStream_t st) {
   const int tn = p->L > 64 ? 64 : 32, tiles = ceil_div(p->L, tn);
-  const int tb = leg_rows(p, nf, tiles, 2 * 148);
+  const int tb = leg_rows(p, nf, tiles, 2 * p->sms);
   auto* kernel = tn == 64
                      ? (tb == 64 ? legendre_forward_simt<64, 64> : legendre_forward_simt<64, 128>)
                      : (tb == 64 ? legendre_forward_simt<32, 64> : legendre_forward_simt<32, 128>);

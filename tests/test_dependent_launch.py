@@ -124,3 +124,8 @@ def test_uploads_are_finished_before_they_return():
   start = text.index('{', text.index('int upload('))
   body = text[start:closing(text, start, '{}')]
   assert body.index('cudaMemcpyHostToDevice') < body.index('cudaStreamSynchronize')
+
+
+def test_launch_rules_ask_the_device_for_its_multiprocessors():
+  for name, text in SOURCES.items():
+    assert not re.search(r'\b148\b', text), name
