@@ -1073,7 +1073,7 @@ __global__ void __launch_bounds__(kModalTX * kModalTY, kTracers ? 4 : 3)
   constexpr bool kStage = kNf >= 0;
   constexpr int kF = kNf > 0 ? kNf : 1;  // array sizes
   constexpr int kPair = kTracers ? 1 : 2;  // rows whose loads are in flight together
-  __shared__ float tile[kStage ? 2 : 1][kStage ? 3 : 1][kTile][kTile + 1];
+  __shared__ float tl[kStage ? 3 : 1][kTile][kTile + 1];
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int l0 = blockIdx.x * kTile, row0 = blockIdx.y * kTile;
   const int l = l0 + tx, lc = min(l, a.L - 1);
@@ -1085,10 +1085,8 @@ __global__ void __launch_bounds__(kModalTX * kModalTY, kTracers ? 4 : 3)
   const float filt = (kStage && s.filter) ? s.filter[lc] : 1.f;
   const float ir = a.inv_radius;
   const int n = 2 * K + 1;
-  int buf = 0;
-  for (int q = blockIdx.z; q < K * a.mem; q += gridDim.z, buf ^= 1) {
+  for (int q = blockIdx.z; q < K * a.mem; q += gridDim.z) {
     const int mb = q / K, k = q - mb * K;
-    float(*tl)[kTile][kTile + 1] = tile[kStage ? buf : 0];
     // Entry of y0 + sum_j fc_j f_j + fself f; f_j = f below the triangle.
     struct Old {
       float y, f[kF];
@@ -1228,8 +1226,6 @@ __global__ void __launch_bounds__(kModalTX * kModalTY, kTracers ? 4 : 3)
     }
 #undef FM
     if (!kStage) continue;
-    // One barrier a plane: the next plane uses the other tile buffer, which
-    // everyone has finished reading before passing this plane's barrier.
     __syncthreads();
     if (trow < a.M) {
 #pragma unroll
@@ -1255,6 +1251,8 @@ __global__ void __launch_bounds__(kModalTX * kModalTY, kTracers ? 4 : 3)
         }
       }
     }
+    // Another plane (past the grid's limit only) writes the tile again.
+    if (q + (int)gridDim.z < K * a.mem) __syncthreads();
   }
 }
 

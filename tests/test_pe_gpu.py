@@ -431,3 +431,28 @@ def test_fused_step_matches_tableau_loop(wavenumbers, layers, members, moist, be
   for a, b in zip(leaves(got), leaves(want)):
     a, b = a.double(), b.double()
     assert float((a - b).abs().max() / b.abs().max()) < 5e-6
+
+
+def test_more_planes_than_the_grid_holds():
+  # 33000 (member, level) planes: some CTAs of the pre-pass and of the stage take
+  # two.  Every member's sums are formed in the order of the state alone.
+  layers, members = 2, 16500
+  rng = np.random.default_rng(3)
+  g = sh.Grid.with_wavenumbers(9)
+  coords = coordinate_systems.CoordinateSystem(
+      g, sigma_coordinates.SigmaCoordinates.equidistant(layers))
+  _, l = np.meshgrid(*g.modal_axes, indexing='ij')
+  def field(amplitude, k, mean=0.0):
+    x = amplitude * rng.standard_normal((members, k) + l.shape) * g.mask / (l + 1.0) ** 1.5
+    x[..., 0, 0] += 2 * np.sqrt(np.pi) * mean
+    return torch.as_tensor(x, device='cuda', dtype=torch.float32)
+  state = pe.State(field(0.05, layers), field(0.005, layers), field(5.0, layers),
+                   field(0.01, 1, 45.0))
+  eq = pe.PrimitiveEquationsSigma(np.linspace(220.0, 290.0, layers),
+                                  np.zeros(l.shape, np.float32), coords, units.SimUnits())
+  step = ti.imex_rk_sil3(eq, 0.05)
+  got = step(state)
+  for i in (0, 1, 116, 16383, 16384, members - 1):
+    want = step(pe.State(*[getattr(state, k)[i] for k in KEYS]))
+    for k in KEYS:
+      assert torch.equal(getattr(got, k)[i], getattr(want, k)), (i, k)
