@@ -337,30 +337,36 @@ __device__ __forceinline__ void st_vec(float* p, const float (&x)[V]) {
   }
 }
 
-// One thread per (V adjacent columns, chunk of levels): blockDim =
-// (kNodalCols, C), chunk c holding levels [c K / C, (c + 1) K / C).  The
-// column totals and the prefix sums that sigma-dot needs come from per-chunk
-// partial sums exchanged through shared memory, so a thread walks K / C
-// levels.  A chunk's running sums are its partial sum formed in the same
-// order, so the sigma-dot of a half level shared by two chunks is the same in
-// both.  V columns share each address computation and level coefficient (the
-// latitude count J is a multiple of V, so they lie on one meridian).
-// kTracers = false compiles out the tracer windows (dry states).
+// Parts of a column for pe_nodal_kernel.  The count depends on the levels alone,
+// so that a state's sums are formed in the same order, and its tendencies have
+// the same bits, in any batch and with any number of threads.
+constexpr int kNodalCols = 32, kNodalMaxParts = 4;
+__host__ __device__ inline int nodal_parts(int K) {
+  return K >= 8 ? kNodalMaxParts : K >= 4 ? 2 : 1;
+}
+
+// C threads per V adjacent columns: blockDim = (kNodalCols, C).  The S parts of
+// a column hold the levels [s K / S, (s + 1) K / S) and thread c the parts
+// [c S / C, (c + 1) S / C), one part with tracers.  The column totals and the
+// prefix sums that sigma-dot needs come from the parts' sums exchanged through
+// shared memory, so a thread walks K / C levels.  A part starts from those sums
+// also where its thread held the part above, so it has the same bits whether
+// one thread holds the two or two.  V columns share each address computation
+// and level coefficient (the latitude count J is a multiple of V, so they lie on
+// one meridian).  kTracers = false compiles out the tracer windows (dry states).
 // Every field of the next level is loaded while a level is computed (moist
 // TL255 / 32 x 4: 570 -> 541 us a launch).
-constexpr int kNodalCols = 32, kNodalMaxChunks = 4;
-
 template <bool kTracers, int V>
-__global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
+__global__ void __launch_bounds__(kNodalCols * kNodalMaxParts)
     pe_nodal_kernel(NodalArgs a) {
   pdl_trigger();
   pdl_wait();
   extern __shared__ float4 s_lev[];  // [K][kLevPack / 4]
-  __shared__ float s_e[kNodalMaxChunks][kNodalCols * V];
-  __shared__ float s_f[kNodalMaxChunks][kNodalCols * V];
-  __shared__ float s_g[kTracers ? kNodalMaxChunks : 1][kNodalCols * V];
+  __shared__ float s_e[kNodalMaxParts][kNodalCols * V];
+  __shared__ float s_f[kNodalMaxParts][kNodalCols * V];
+  __shared__ float s_g[kTracers ? kNodalMaxParts : 1][kNodalCols * V];
   const int tx = threadIdx.x, c = threadIdx.y, C = blockDim.y;
-  const int K = a.K;
+  const int K = a.K, S = nodal_parts(K);
   for (int i = c * kNodalCols + tx; i < K * (kLevPack / 4); i += kNodalCols * C)
     s_lev[i] = reinterpret_cast<const float4*>(a.levpack)[i];
   __syncthreads();
@@ -370,7 +376,9 @@ __global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
   const unsigned col = (blockIdx.x * kNodalCols + tx) * V;
   const bool active = col < IJ;
   const int mb = blockIdx.y;
-  const int k0 = (c * K) / C, k1 = ((c + 1) * K) / C;
+  // This thread's parts.
+  const int s0 = kTracers ? c : c * S / C, s1 = kTracers ? c + 1 : (c + 1) * S / C;
+  const int k0 = (s0 * K) / S;
   const int nT = kTracers ? a.nT : 0;
   const int hum = kTracers ? a.hum : -1;
   const int j = active ? (int)(col % (unsigned)a.J) : 0;
@@ -392,17 +400,21 @@ __global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
   const float rv1 = a.Rv_over_R - 1.f;
   float gx[V], gy[V];
 
-  // Pass 1: this chunk's share of the column totals of u.grad(ln ps) and of
-  // (div + u.grad ln ps), both weighted by the layer thickness
-  // (cumulative_sigma_integral, last level), and (moist) of the geopotential
-  // suffix sum of the virtual-temperature difference.
-  float pe_[V], pf_[V], pg_[V];
-#pragma unroll
-  for (int i = 0; i < V; ++i) pe_[i] = pf_[i] = pg_[i] = 0.f;
   if (active) {
     ld_vec(gx, a.nod + ((size_t)a.p_gx + mb) * IJ + col);
     ld_vec(gy, a.nod + ((size_t)a.p_gy + mb) * IJ + col);
-    for (int k = k0; k < k1; ++k) {
+  }
+
+  // Pass 1: the parts' shares of the column totals of u.grad(ln ps) and of
+  // (div + u.grad ln ps), both weighted by the layer thickness
+  // (cumulative_sigma_integral, last level), and (moist) of the geopotential
+  // suffix sum of the virtual-temperature difference.
+  for (int s = s0; s < s1; ++s) {
+    const int ka = (s * K) / S, kb = active ? ((s + 1) * K) / S : 0;
+    float pe_[V], pf_[V], pg_[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) pe_[i] = pf_[i] = pg_[i] = 0.f;
+    for (int k = ka; k < kb; ++k) {
       const unsigned o = (unsigned)k * IJ;
       const float ds = s_lev[4 * k].x;
       float u[V], v[V], d[V];
@@ -417,7 +429,7 @@ __global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
       }
     }
     if (hum >= 0) {
-      for (int k = max(k0, 1); k < k1; ++k) {
+      for (int k = max(ka, 1); k < kb; ++k) {
         const unsigned o = (unsigned)k * IJ;
         const float4 c1 = s_lev[4 * k + 1];
         const float tr = s_lev[4 * k].w;
@@ -428,12 +440,12 @@ __global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
         for (int i = 0; i < V; ++i) pg_[i] += (c1.z + c1.w) * (h[i] * (T[i] + tr) * rv1);
       }
     }
-  }
 #pragma unroll
-  for (int i = 0; i < V; ++i) {
-    s_e[c][tx * V + i] = pe_[i];
-    s_f[c][tx * V + i] = pf_[i];
-    if (kTracers) s_g[c][tx * V + i] = pg_[i];
+    for (int i = 0; i < V; ++i) {
+      s_e[s][tx * V + i] = pe_[i];
+      s_f[s][tx * V + i] = pf_[i];
+      if (kTracers) s_g[s][tx * V + i] = pg_[i];
+    }
   }
   __syncthreads();
   if (!active) return;
@@ -441,13 +453,13 @@ __global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
 #pragma unroll
   for (int i = 0; i < V; ++i) {
     Fe[i] = Ff[i] = pre_e[i] = pre_f[i] = 0.f;
-    for (int cc = 0; cc < C; ++cc) {
-      if (cc == c) {
+    for (int s = 0; s < S; ++s) {
+      if (s == s0) {
         pre_e[i] = Fe[i];
         pre_f[i] = Ff[i];
       }
-      Fe[i] += s_e[cc][tx * V + i];
-      Ff[i] += s_f[cc][tx * V + i];
+      Fe[i] += s_e[s][tx * V + i];
+      Ff[i] += s_f[s][tx * V + i];
     }
   }
 
@@ -455,27 +467,29 @@ __global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
   // G[k][h] = R alpha_k (h = k), R (alpha_h + alpha_{h-1}) (h > k): a suffix
   // sum evaluated bottom-up (get_geopotential_weights_sigma, :306-338).
   if (hum >= 0) {
-    float suffix[V];
-#pragma unroll
-    for (int i = 0; i < V; ++i) {
-      suffix[i] = 0.f;
-      for (int cc = C - 1; cc > c; --cc) suffix[i] += s_g[cc][tx * V + i];
-    }
     float* Ogh = out(a.o_gh);
-    for (int k = k1 - 1; k >= k0; --k) {
-      const unsigned o = (unsigned)k * IJ;
-      const float4 c1 = s_lev[4 * k + 1];
-      const float tr = s_lev[4 * k].w;
-      float h[V], T[V], g[V];
-      ld_vec(h, Ph + o);
-      ld_vec(T, PT + o);
+    for (int s = s1 - 1; s >= s0; --s) {
+      float suffix[V];
 #pragma unroll
       for (int i = 0; i < V; ++i) {
-        const float td = h[i] * (T[i] + tr) * rv1;
-        g[i] = a.R * (c1.z * td + suffix[i]);
-        suffix[i] += (c1.z + c1.w) * td;
+        suffix[i] = 0.f;
+        for (int ss = S - 1; ss > s; --ss) suffix[i] += s_g[ss][tx * V + i];
       }
-      st_vec(Ogh + o, g);
+      for (int k = ((s + 1) * K) / S - 1; k >= (s * K) / S; --k) {
+        const unsigned o = (unsigned)k * IJ;
+        const float4 c1 = s_lev[4 * k + 1];
+        const float tr = s_lev[4 * k].w;
+        float h[V], T[V], g[V];
+        ld_vec(h, Ph + o);
+        ld_vec(T, PT + o);
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+          const float td = h[i] * (T[i] + tr) * rv1;
+          g[i] = a.R * (c1.z * td + suffix[i]);
+          suffix[i] += (c1.z + c1.w) * td;
+        }
+        st_vec(Ogh + o, g);
+      }
     }
   }
 
@@ -505,7 +519,7 @@ __global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
   float laplnps[V];
   if (hum >= 0) ld_vec(laplnps, a.nod + ((size_t)a.p_laplnps + mb) * IJ + col);
 
-  // Pass 2: everything else, streaming over the chunk's levels top-down with
+  // Pass 2: everything else, streaming over the thread's levels top-down with
   // a window of (k-1, k, k+1) for the vertically advected fields.  The level
   // coefficients hold zero for the half levels outside the column, and the
   // window reads level K-1 again in place of a level K, so the boundary terms
@@ -547,163 +561,180 @@ __global__ void __launch_bounds__(kNodalCols * kNodalMaxChunks)
   float zeta_n[V], div_n[V];
   ld_vec(zeta_n, Pz + o0);
   ld_vec(div_n, Pd + o0);
-  for (int k = k0; k < k1; ++k) {
-    const unsigned o = (unsigned)k * IJ;
-    const unsigned on = (k + 1 < K) ? o + IJ : o;
-    const float4 c0 = s_lev[4 * k], c1 = s_lev[4 * k + 1];
-    const float4 c2 = s_lev[4 * k + 2], c3 = s_lev[4 * k + 3];
-    const float ds = c0.x, inv_ds = c0.y, ss = c0.z, tr = c0.w;
-    const float ci_dn = c1.x, ci_up = c1.y, al = c1.z, al_up = c1.w;
-    float u_n[V], v_n[V], T_n[V], zeta[V], div[V];
-    ld_vec(u_n, Pu + on);
-    ld_vec(v_n, Pv + on);
-    ld_vec(T_n, PT + on);
+#pragma unroll 1
+  for (int s = s0, k = k0; s < s1; ++s) {
+    if (s > s0) {
+      // The next part starts from the same prefix sums as in a thread of its own.
+      const float ssu = s_lev[4 * (k - 1)].z;
 #pragma unroll
-    for (int i = 0; i < V; ++i) {
-      zeta[i] = zeta_n[i];
-      div[i] = div_n[i];
+      for (int i = 0; i < V; ++i) {
+        pre_e[i] += s_e[s - 1][tx * V + i];
+        pre_f[i] += s_f[s - 1][tx * V + i];
+        loc_e[i] = loc_f[i] = 0.f;
+        fe_prev[i] = pre_e[i];
+        ff_prev[i] = pre_f[i];
+        sd_up_f[i] = ssu * Ff[i] - pre_f[i];
+        sd_up_e[i] = ssu * Fe[i] - pre_e[i];
+      }
     }
-    ld_vec(zeta_n, Pz + on);
-    ld_vec(div_n, Pd + on);
-    float q_n[kTracers ? kMaxTracers : 1][V];
-    if (kTracers) {
+    for (const int k1 = ((s + 1) * K) / S; k < k1; ++k) {
+      const unsigned o = (unsigned)k * IJ;
+      const unsigned on = (k + 1 < K) ? o + IJ : o;
+      const float4 c0 = s_lev[4 * k], c1 = s_lev[4 * k + 1];
+      const float4 c2 = s_lev[4 * k + 2], c3 = s_lev[4 * k + 3];
+      const float ds = c0.x, inv_ds = c0.y, ss = c0.z, tr = c0.w;
+      const float ci_dn = c1.x, ci_up = c1.y, al = c1.z, al_up = c1.w;
+      float u_n[V], v_n[V], T_n[V], zeta[V], div[V];
+      ld_vec(u_n, Pu + on);
+      ld_vec(v_n, Pv + on);
+      ld_vec(T_n, PT + on);
 #pragma unroll
-      for (int t = 0; t < kMaxTracers; ++t)
-        if (t < nT) ld_vec(q_n[t], Pq + t * tstride + on);
-    }
-    float gqx[V], gqy[V];
-    if (hum >= 0) {
-      ld_vec(gqx, a.nod + pl(a.p_gqx, mb, K, 0) * IJ + col + o);
-      ld_vec(gqy, a.nod + pl(a.p_gqy, mb, K, 0) * IJ + col + o);
-    }
-    float rAu[V], rAv[V], rKE[V], ruT[V], rvT[V], rTn[V], rhs[V], rvh[V], rdh[V];
-    float sdn_f[V], sdn_e[V];
-#pragma unroll
-    for (int i = 0; i < V; ++i) {
-      const float ugl = (u_c[i] * gx[i] + v_c[i] * gy[i]) * sec2[i];
-      loc_e[i] += ugl * ds;
-      loc_f[i] += (div[i] + ugl) * ds;
-      const float fe = pre_e[i] + loc_e[i];
-      const float ff = pre_f[i] + loc_f[i];
-      const float sd_dn_f = ss * Ff[i] - ff;  // sigma-dot at k + 1/2
-      const float sd_dn_e = ss * Fe[i] - fe;
-      sdn_f[i] = sd_dn_f;
-      sdn_e[i] = sd_dn_e;
-      // centered_vertical_advection(w, x)[k] = -0.5 (w_{k+1/2} dx_{k+1/2} +
-      // w_{k-1/2} dx_{k-1/2}) (sigma_coordinates.py:344-405).
-      auto vadv = [&](float xp, float xc, float xn) {
-        return -0.5f * (sd_dn_f * ((xn - xc) * ci_dn) + sd_up_f[i] * ((xc - xp) * ci_up));
-      };
-      float q_h = 0.f;
-      if (kTracers && hum >= 0) {
+      for (int i = 0; i < V; ++i) {
+        zeta[i] = zeta_n[i];
+        div[i] = div_n[i];
+      }
+      ld_vec(zeta_n, Pz + on);
+      ld_vec(div_n, Pd + on);
+      float q_n[kTracers ? kMaxTracers : 1][V];
+      if (kTracers) {
 #pragma unroll
         for (int t = 0; t < kMaxTracers; ++t)
-          if (t == hum) q_h = q_c[t][i];
+          if (t < nT) ld_vec(q_n[t], Pq + t * tstride + on);
       }
-      // curl_and_div_tendencies (:1001-1059)
-      const float adj = (hum >= 0) ? 1.f + rv1 * q_h : 1.f;
-      const float rt = a.R * T_c[i] * adj;
-      float sdu = 0.f, sdv = 0.f;
-      if (a.vadv) {
-        sdu = -vadv(u_p[i], u_c[i], u_n[i]);
-        sdv = -vadv(v_p[i], v_c[i], v_n[i]);
-      }
-      const float tv = zeta[i] + fcor[i];
-      float Au = -v_c[i] * tv * sec2[i] + (sdu + rt * gx[i]) * sec2[i];
-      float Av = u_c[i] * tv * sec2[i] + (sdv + rt * gy[i]) * sec2[i];
-      if (a.hs) {
-        // Rayleigh drag folded in: curl/div of -(-kv u / cos^2).
-        Au += c2.x * u_c[i] * sec2[i];
-        Av += c2.x * v_c[i] * sec2[i];
-      }
-      rAu[i] = Au;
-      rAv[i] = Av;
-      rKE[i] = (u_c[i] * u_c[i] + v_c[i] * v_c[i]) * sec2[i] * 0.5f;
-      ruT[i] = u_c[i] * T_c[i] * sec2[i];
-      rvT[i] = v_c[i] * T_c[i] * sec2[i];
-      // Temperature: horizontal nodal term, vertical advection, adiabatic.
-      float Tn = T_c[i] * div[i];
-      if (a.vadv) Tn += vadv(T_p[i], T_c[i], T_n[i]);
-      if (a.tref_varies) Tn += -0.5f * (sd_dn_e * c3.x + sd_up_e[i] * c3.y);
-      const float ge = (al * fe + al_up * fe_prev[i]) * inv_ds;
-      const float gf = (al * ff + al_up * ff_prev[i]) * inv_ds;
-      const float mean_part = tr * (ugl - ge);
-      float var_part;
-      if (hum < 0) {
-        var_part = T_c[i] * (ugl - gf);
-      } else {
-        const float den = 1.f + (a.Cpv_over_Cp - 1.f) * q_h;
-        const float tv_var = T_c[i] * ((1.f + rv1 * q_h) / den);
-        const float tv_ref = tr * (((a.Rv_over_R - a.Cpv_over_Cp) * q_h) / den);
-        var_part = (tv_var + tv_ref) * (ugl - gf);
-      }
-      rTn[i] = Tn + a.kappa * (mean_part + var_part);
+      float gqx[V], gqy[V];
       if (hum >= 0) {
-        const float coef = tr * a.Rv_minus_R;
-        rvh[i] = coef * sec2[i] * (gx[i] * gqy[i] - gy[i] * gqx[i]);
-        rdh[i] = coef * sec2[i] * (gqx[i] * gx[i] + gqy[i] * gy[i]) +
-                 q_h * laplnps[i] * tr * a.Rv_minus_R;
+        ld_vec(gqx, a.nod + pl(a.p_gqx, mb, K, 0) * IJ + col + o);
+        ld_vec(gqy, a.nod + pl(a.p_gqy, mb, K, 0) * IJ + col + o);
       }
-      if (a.hs) {
-        // held_suarez.py:105-120, :138-151, with log(p / p0) = log(sigma / p0)
-        // + ln ps, so (p / p0)^kappa = (sigma / p0)^kappa ps^kappa.
-        const float kt = a.hs_ka + hs_dk[i] * c2.y;
-        float teq = c2.z * hs_e[i] * (hs_A0[i] - hs_B0[i] * c2.w);
-        teq = fmaxf(a.hs_minT, teq);
-        rhs[i] = -kt * (tr + T_c[i] - teq);
-      }
-      fe_prev[i] = fe;
-      ff_prev[i] = ff;
-    }
-    st_vec(OAu + o, rAu);
-    st_vec(OAv + o, rAv);
-    st_vec(OKE + o, rKE);
-    st_vec(OuT + o, ruT);
-    st_vec(OvT + o, rvT);
-    st_vec(OTn + o, rTn);
-    if (hum >= 0) {
-      st_vec(a.fwd + pl(a.o_vh, mb, K, 0) * IJ + col + o, rvh);
-      st_vec(a.fwd + pl(a.o_dh, mb, K, 0) * IJ + col + o, rdh);
-    }
-    if (a.hs) st_vec(a.fwd + pl(a.o_hsT, mb, K, 0) * IJ + col + o, rhs);
-    // Tracers: u q, v q (times sec^2) and q div + vertical advection.
-    if (kTracers) {
+      float rAu[V], rAv[V], rKE[V], ruT[V], rvT[V], rTn[V], rhs[V], rvh[V], rdh[V];
+      float sdn_f[V], sdn_e[V];
 #pragma unroll
-      for (int t = 0; t < kMaxTracers; ++t) {
-        if (t >= nT) break;
-        float* ob = Otr + 3 * t * tstride;
-        float fu[V], fv[V], fq[V];
+      for (int i = 0; i < V; ++i) {
+        const float ugl = (u_c[i] * gx[i] + v_c[i] * gy[i]) * sec2[i];
+        loc_e[i] += ugl * ds;
+        loc_f[i] += (div[i] + ugl) * ds;
+        const float fe = pre_e[i] + loc_e[i];
+        const float ff = pre_f[i] + loc_f[i];
+        const float sd_dn_f = ss * Ff[i] - ff;  // sigma-dot at k + 1/2
+        const float sd_dn_e = ss * Fe[i] - fe;
+        sdn_f[i] = sd_dn_f;
+        sdn_e[i] = sd_dn_e;
+        // centered_vertical_advection(w, x)[k] = -0.5 (w_{k+1/2} dx_{k+1/2} +
+        // w_{k-1/2} dx_{k-1/2}) (sigma_coordinates.py:344-405).
+        auto vadv = [&](float xp, float xc, float xn) {
+          return -0.5f * (sd_dn_f * ((xn - xc) * ci_dn) + sd_up_f[i] * ((xc - xp) * ci_up));
+        };
+        float q_h = 0.f;
+        if (kTracers && hum >= 0) {
 #pragma unroll
-        for (int i = 0; i < V; ++i) {
-          fu[i] = u_c[i] * q_c[t][i] * sec2[i];
-          fv[i] = v_c[i] * q_c[t][i] * sec2[i];
-          float qn = q_c[t][i] * div[i];
-          if (a.vadv)
-            qn += -0.5f * (sdn_f[i] * ((q_n[t][i] - q_c[t][i]) * ci_dn) +
-                           sd_up_f[i] * ((q_c[t][i] - q_p[t][i]) * ci_up));
-          fq[i] = qn;
+          for (int t = 0; t < kMaxTracers; ++t)
+            if (t == hum) q_h = q_c[t][i];
         }
-        st_vec(ob + o, fu);
-        st_vec(ob + tstride + o, fv);
-        st_vec(ob + 2 * tstride + o, fq);
-      }
-    }
-    // Advance the window.
-#pragma unroll
-    for (int i = 0; i < V; ++i) {
-      sd_up_f[i] = sdn_f[i];
-      sd_up_e[i] = sdn_e[i];
-      u_p[i] = u_c[i]; v_p[i] = v_c[i]; T_p[i] = T_c[i];
-      u_c[i] = u_n[i]; v_c[i] = v_n[i]; T_c[i] = T_n[i];
-    }
-    if (kTracers) {
-#pragma unroll
-      for (int t = 0; t < kMaxTracers; ++t)
-#pragma unroll
-        for (int i = 0; i < V; ++i) {
-          q_p[t][i] = q_c[t][i];
-          q_c[t][i] = q_n[t][i];
+        // curl_and_div_tendencies (:1001-1059)
+        const float adj = (hum >= 0) ? 1.f + rv1 * q_h : 1.f;
+        const float rt = a.R * T_c[i] * adj;
+        float sdu = 0.f, sdv = 0.f;
+        if (a.vadv) {
+          sdu = -vadv(u_p[i], u_c[i], u_n[i]);
+          sdv = -vadv(v_p[i], v_c[i], v_n[i]);
         }
+        const float tv = zeta[i] + fcor[i];
+        float Au = -v_c[i] * tv * sec2[i] + (sdu + rt * gx[i]) * sec2[i];
+        float Av = u_c[i] * tv * sec2[i] + (sdv + rt * gy[i]) * sec2[i];
+        if (a.hs) {
+          // Rayleigh drag folded in: curl/div of -(-kv u / cos^2).
+          Au += c2.x * u_c[i] * sec2[i];
+          Av += c2.x * v_c[i] * sec2[i];
+        }
+        rAu[i] = Au;
+        rAv[i] = Av;
+        rKE[i] = (u_c[i] * u_c[i] + v_c[i] * v_c[i]) * sec2[i] * 0.5f;
+        ruT[i] = u_c[i] * T_c[i] * sec2[i];
+        rvT[i] = v_c[i] * T_c[i] * sec2[i];
+        // Temperature: horizontal nodal term, vertical advection, adiabatic.
+        float Tn = T_c[i] * div[i];
+        if (a.vadv) Tn += vadv(T_p[i], T_c[i], T_n[i]);
+        if (a.tref_varies) Tn += -0.5f * (sd_dn_e * c3.x + sd_up_e[i] * c3.y);
+        const float ge = (al * fe + al_up * fe_prev[i]) * inv_ds;
+        const float gf = (al * ff + al_up * ff_prev[i]) * inv_ds;
+        const float mean_part = tr * (ugl - ge);
+        float var_part;
+        if (hum < 0) {
+          var_part = T_c[i] * (ugl - gf);
+        } else {
+          const float den = 1.f + (a.Cpv_over_Cp - 1.f) * q_h;
+          const float tv_var = T_c[i] * ((1.f + rv1 * q_h) / den);
+          const float tv_ref = tr * (((a.Rv_over_R - a.Cpv_over_Cp) * q_h) / den);
+          var_part = (tv_var + tv_ref) * (ugl - gf);
+        }
+        rTn[i] = Tn + a.kappa * (mean_part + var_part);
+        if (hum >= 0) {
+          const float coef = tr * a.Rv_minus_R;
+          rvh[i] = coef * sec2[i] * (gx[i] * gqy[i] - gy[i] * gqx[i]);
+          rdh[i] = coef * sec2[i] * (gqx[i] * gx[i] + gqy[i] * gy[i]) +
+                   q_h * laplnps[i] * tr * a.Rv_minus_R;
+        }
+        if (a.hs) {
+          // held_suarez.py:105-120, :138-151, with log(p / p0) = log(sigma / p0)
+          // + ln ps, so (p / p0)^kappa = (sigma / p0)^kappa ps^kappa.
+          const float kt = a.hs_ka + hs_dk[i] * c2.y;
+          float teq = c2.z * hs_e[i] * (hs_A0[i] - hs_B0[i] * c2.w);
+          teq = fmaxf(a.hs_minT, teq);
+          rhs[i] = -kt * (tr + T_c[i] - teq);
+        }
+        fe_prev[i] = fe;
+        ff_prev[i] = ff;
+      }
+      st_vec(OAu + o, rAu);
+      st_vec(OAv + o, rAv);
+      st_vec(OKE + o, rKE);
+      st_vec(OuT + o, ruT);
+      st_vec(OvT + o, rvT);
+      st_vec(OTn + o, rTn);
+      if (hum >= 0) {
+        st_vec(a.fwd + pl(a.o_vh, mb, K, 0) * IJ + col + o, rvh);
+        st_vec(a.fwd + pl(a.o_dh, mb, K, 0) * IJ + col + o, rdh);
+      }
+      if (a.hs) st_vec(a.fwd + pl(a.o_hsT, mb, K, 0) * IJ + col + o, rhs);
+      // Tracers: u q, v q (times sec^2) and q div + vertical advection.
+      if (kTracers) {
+#pragma unroll
+        for (int t = 0; t < kMaxTracers; ++t) {
+          if (t >= nT) break;
+          float* ob = Otr + 3 * t * tstride;
+          float fu[V], fv[V], fq[V];
+#pragma unroll
+          for (int i = 0; i < V; ++i) {
+            fu[i] = u_c[i] * q_c[t][i] * sec2[i];
+            fv[i] = v_c[i] * q_c[t][i] * sec2[i];
+            float qn = q_c[t][i] * div[i];
+            if (a.vadv)
+              qn += -0.5f * (sdn_f[i] * ((q_n[t][i] - q_c[t][i]) * ci_dn) +
+                             sd_up_f[i] * ((q_c[t][i] - q_p[t][i]) * ci_up));
+            fq[i] = qn;
+          }
+          st_vec(ob + o, fu);
+          st_vec(ob + tstride + o, fv);
+          st_vec(ob + 2 * tstride + o, fq);
+        }
+      }
+      // Advance the window.
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        sd_up_f[i] = sdn_f[i];
+        sd_up_e[i] = sdn_e[i];
+        u_p[i] = u_c[i]; v_p[i] = v_c[i]; T_p[i] = T_c[i];
+        u_c[i] = u_n[i]; v_c[i] = v_n[i]; T_c[i] = T_n[i];
+      }
+      if (kTracers) {
+#pragma unroll
+        for (int t = 0; t < kMaxTracers; ++t)
+#pragma unroll
+          for (int i = 0; i < V; ++i) {
+            q_p[t][i] = q_c[t][i];
+            q_c[t][i] = q_n[t][i];
+          }
+      }
     }
   }
   if (c == 0) {
@@ -2402,14 +2433,19 @@ static int pe_nodal_inputs(dino_pe* pe, const float* state, cudaStream_t st) {
   return DINO_OK;
 }
 
-// Level chunks per column for pe_nodal_kernel: four from eight levels on.  The
-// count depends on the levels alone, so that a state's sums are formed in the
-// same order, and its tendencies have the same bits, in any batch.  Measured
-// with two and four chunks (us a launch): T21 / 12 9.8, 7.4; T42 / 20 13.9, 8.9;
-// T42 / 24 x 16 37.5, 41.3; TL255 / 32 46.2, 45.3; TL95 / 19 moist x 3 38.8, 38.8;
-// TL255 / 32 moist x 4 541, 558.
-static int nodal_chunks(const dino_pe* pe) {
-  return pe->K >= 8 ? kNodalMaxChunks : pe->K >= 4 ? 2 : 1;
+// Threads per column (pair) of pe_nodal_kernel: one per part, which single
+// members of small grids need (T21 / 12 with two and four threads 9.8, 7.4 us a
+// launch; T42 / 20 13.9, 8.9).  A thread loads a window of three levels anew at
+// its first part, so dry states take two threads where those alone fill the
+// chip one and a half times (16 warps an SM at 125 registers): explicit terms of
+// T42 / 24 x 16 182.3 with four, 180.1 us with two, Held-Suarez steps 717, 709;
+// x 12 140.2, 144.2; TL255 / 32 the same; one thread is never better.
+// With tracers a second part's code costs registers (124 -> 166; held at 128,
+// TL95 / 19 moist x 3 steps 956 -> 967 us), so there each part has its thread.
+static int nodal_threads(const dino_pe* pe, int V) {
+  const int parts = nodal_parts(pe->K);
+  const int64_t warps = (int64_t)ceil_div((int)(pe->IJ / V), kNodalCols) * pe->mem;
+  return pe->nT == 0 && parts > 2 && 2 * warps >= 24LL * pe->plan->sms ? 2 : parts;
 }
 
 // Adjacent columns per thread for pe_nodal_kernel: two for dry states where
@@ -2491,7 +2527,7 @@ static int launch_nodal(dino_pe* pe, const float* state, cudaStream_t st) {
   const NodalArgs a = make_nodal_args(pe);
   const int V = nodal_vec(pe);
   const dim3 grid(ceil_div((int)(pe->IJ / V), kNodalCols), pe->mem);
-  const dim3 block(kNodalCols, nodal_chunks(pe));
+  const dim3 block(kNodalCols, nodal_threads(pe, V));
   const size_t smem = nodal_smem(pe->K);
   auto* kernel = pe->nT > 0 ? pe_nodal_kernel<true, 1>
                             : V == 2 ? pe_nodal_kernel<false, 2> : pe_nodal_kernel<false, 1>;

@@ -223,19 +223,39 @@ def test_level_chunks_agree_across_batch_sizes():
     assert err < 1e-6, (k, err)
 
 
-@pytest.mark.parametrize('layers,moist', [(2, False), (5, False), (9, False), (19, True),
-                                          (24, False)])
-def test_level_chunks_give_the_same_bits(layers, moist):
-  # The chunk count (one, two or four by the levels) does not depend on the
-  # batch, so every member's tendencies have the bits of the state alone.
-  kw = dict(tracers=_tracers, humidity='specific_humidity') if moist else {}
-  og, oeq, st, g, eq = make('T42', layers=layers, **kw)
-  s1 = to_state(st)
-  batch = pe.State(*[torch.stack([getattr(s1, k)] * 16) for k in KEYS],
-                   tracers={k: torch.stack([v] * 16) for k, v in s1.tracers.items()})
-  ob, o1 = eq.explicit_terms(batch), eq.explicit_terms(s1)
-  for k in KEYS:
-    assert torch.equal(getattr(ob, k)[11], getattr(o1, k)), k
+@pytest.mark.parametrize('grid_name,layers,members,moist', [
+    ('T42', 2, 16, False), ('T42', 5, 16, False), ('T42', 9, 16, False), ('T42', 19, 16, True),
+    ('T42', 24, 16, False), ('odd', 9, 24, False), ('odd', 8, 24, True)])
+def test_members_have_the_bits_of_the_state_alone(grid_name, layers, members, moist):
+  # The column sums are formed over parts whose count follows from the levels
+  # (one, two or four), whether a thread holds one part (single states, tracers)
+  # or two (large dry batches); one or two columns a thread (odd latitudes).
+  g = sh.Grid.T42() if grid_name == 'T42' else sh.Grid.with_wavenumbers(24)
+  assert g.nodal_shape[1] % 2 == (grid_name == 'odd')
+  rng = np.random.default_rng(layers)
+  coords = coordinate_systems.CoordinateSystem(
+      g, sigma_coordinates.SigmaCoordinates.equidistant(layers))
+  _, l = np.meshgrid(*g.modal_axes, indexing='ij')
+  def field(amplitude, k, mean=0.0):
+    x = amplitude * rng.standard_normal((members, k) + l.shape) * g.mask / (l + 1.0) ** 1.5
+    x[..., 0, 0] += 2 * np.sqrt(np.pi) * mean
+    return torch.as_tensor(x, device='cuda', dtype=torch.float32)
+  tracers = {}
+  if moist:
+    tracers = {'specific_humidity': field(1e-3, layers, 5e-3), 'tracer': field(0.3, layers, 1.0)}
+  batch = pe.State(field(0.05, layers), field(0.005, layers), field(5.0, layers),
+                   field(0.01, 1, 45.0), tracers=tracers)
+  eq = pe.PrimitiveEquationsSigma(
+      np.linspace(220.0, 290.0, layers), np.zeros(l.shape, np.float32), coords,
+      units.SimUnits(), humidity_key='specific_humidity' if moist else None)
+  got = eq.explicit_terms(batch)
+  for i in (0, 1, members // 2, members - 1):
+    want = eq.explicit_terms(pe.State(*[getattr(batch, k)[i] for k in KEYS],
+                                      tracers={k: v[i] for k, v in tracers.items()}))
+    for k in KEYS:
+      assert torch.equal(getattr(got, k)[i], getattr(want, k)), (i, k)
+    for k in tracers:
+      assert torch.equal(got.tracers[k][i], want.tracers[k]), (i, k)
 
 
 def test_dry_tracer_advection_matches_oracle():
