@@ -2,10 +2,14 @@
 
 Every supported half length N = I / 2 (each radix schedule), with latitude
 counts that fill no 16-column tile, leave an even remainder or are odd (the
-scalar row path), at quadratic, linear (lw = N) and short truncations, and
-odd field counts, against the FP64 oracle.  Bound: relative L2 2e-6, as the
-other FP32 transform tests (FP32 Legendre sums 3e-7, FFT rounding below
-log2(2560) * 6e-8 = 7e-7).
+scalar row path), and odd field counts.  The longitude phase alone runs at the
+widest truncation (lw = N) on random rows of the full spectrum, against NumPy's
+FFT in 64 bits: no wavenumber is left out.  Bound: sqrt(log2(2 N)) * 6e-8 (one
+rounding a level of the transform, adding up at random), 1.2e-7 to 2.0e-7.  Whole
+transforms run against the FP64 oracle at up to 40 zonal wavenumbers (its cost
+limits them) and at linear truncation for three lengths.  Bound: relative L2
+2e-6, as the other FP32 transform tests (FP32 Legendre sums 3e-7, FFT rounding
+below log2(2560) * 6e-8 = 7e-7).
 """
 
 import numpy as np
@@ -31,7 +35,8 @@ def l2(a, b):
 @pytest.mark.parametrize('lat', [18, 33, 48])
 @pytest.mark.parametrize('n', LENGTHS)
 def test_lengths(n, lat):
-  # Longitude wavenumbers: up to the FFT's own limit lw = N on short rows.
+  # Longitude wavenumbers: up to the FFT's own limit lw = N on short rows, at
+  # most 40 (test_full_spectrum takes the rest).
   lw = min({18: n, 33: (2 * n) // 3, 48: max(2, n // 5)}[lat], 40)
   kw = dict(longitude_wavenumbers=lw, total_wavenumbers=lw + 1,
             longitude_nodes=2 * n, latitude_nodes=lat)
@@ -48,6 +53,19 @@ def test_linear_truncation(n):
   kw = dict(longitude_wavenumbers=n, total_wavenumbers=n + 1,
             longitude_nodes=2 * n, latitude_nodes=n)
   og, g = osht.Grid(**kw), sh.Grid(**kw)
+  x = ost.sht_modal_input(og, 2).astype(np.float64)
+  ref = og.to_nodal(x)
+  assert l2(g.to_nodal(x.astype(np.float32)), ref) < 2e-6
+  z = ref.astype(np.float32).astype(np.float64)
+  assert l2(g.to_modal(z.astype(np.float32)), og.to_modal(z)) < 2e-6
+
+
+@pytest.mark.parametrize('name', ['T31', 'TL47', 'TL95', 'T106', 'TL159', 'TL179', 'T213'])
+def test_named_grids_whose_longitudes_are_no_power_of_two(name):
+  g = getattr(sh.Grid, name)()
+  og = osht.Grid(longitude_wavenumbers=g.longitude_wavenumbers,
+                 total_wavenumbers=g.total_wavenumbers, longitude_nodes=g.longitude_nodes,
+                 latitude_nodes=g.latitude_nodes)
   x = ost.sht_modal_input(og, 2).astype(np.float64)
   ref = og.to_nodal(x)
   assert l2(g.to_nodal(x.astype(np.float32)), ref) < 2e-6
@@ -82,6 +100,15 @@ def phase_errors(n, lat, fields):
   ref[:, 2::2] = -spectrum[:, 1:n].imag / np.sqrt(np.pi)
   weights = (g.plan.nodes[1] * 2 * np.pi / (2 * n)).astype(np.float32)
   return inverse, l2(run(2, x, 2 * n - 1), ref * weights)
+
+
+@pytest.mark.parametrize('lat', [1, 2, 33, 48])
+@pytest.mark.parametrize('n', LENGTHS)
+def test_full_spectrum(n, lat):
+  inverse, forward = phase_errors(n, lat, 3)
+  bound = np.sqrt(np.log2(2 * n)) * 6e-8
+  assert inverse < bound
+  assert forward < bound
 
 
 # Errors (1e-8) that a twiddle product of one rounded product and one FMA leaves,
