@@ -49,8 +49,9 @@ __device__ __forceinline__ void row_map(int m, int r, int& b, int& row) {
 // out_fourier[b][row][j] for all j from modal rows (inverse contraction).  Two
 // rows share an f32x2 FMA: the loop was bound by its issue slots and its
 // shared-memory reads together, and a value's place in two registers is free.
-// The bound of three CTAs of 128 an SM keeps the accumulators out of memory
-// (four spill: TL255, 64 fields 56 us).  TL159, 75 fields 26.0 -> 24.4 us, TL255,
+// The bound of three CTAs of 128 an SM keeps the accumulators in registers (the
+// 64-row form spills two other values; with four CTAs the accumulators spill:
+// TL255, 64 fields 56 us).  TL159, 75 fields 26.0 -> 24.4 us, TL255,
 // 64 fields 42.4 -> 40.1, T42, 900 fields 11.6 -> 10.5.
 template <int TB>
 __global__ void __launch_bounds__(TB, 3 * 128 / TB)
