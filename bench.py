@@ -41,16 +41,16 @@ FORMS = ('fp32', 'bf16x3', 'tf32x3')
 # each transform phase over the 128 TL255 fields, from one ncu capture of
 # `bench.py --profile-phase <phase>` per phase.
 PHASE_TRAFFIC = {
-    ('bf16x3', 'legendre_inverse'): 75098880 + 17449728,
-    ('bf16x3', 'fourier_inverse'): 67005440 + 22596096,
-    ('bf16x3', 'fourier_forward'): 67136000 + 24715264,
-    ('bf16x3', 'legendre_forward'): 103041024 + 21350656,
-    ('fp32', 'legendre_inverse'): 58467584 + 19169536,
-    ('fp32', 'fourier_inverse'): 67005440 + 22596096,
-    ('fp32', 'fourier_forward'): 67136000 + 24715264,
-    ('fp32', 'legendre_forward'): 84916224 + 27469824,
-    ('tf32x3', 'legendre_inverse'): 118548480 + 34110976,
-    ('tf32x3', 'legendre_forward'): 151210240 + 43932416,
+    ('bf16x3', 'legendre_inverse'): 75171072 + 17750784,
+    ('bf16x3', 'fourier_inverse'): 67006464 + 21573120,
+    ('bf16x3', 'fourier_forward'): 67138560 + 21350912,
+    ('bf16x3', 'legendre_forward'): 103344896 + 21940480,
+    ('fp32', 'legendre_inverse'): 58456576 + 19989504,
+    ('fp32', 'fourier_inverse'): 67006464 + 21573120,
+    ('fp32', 'fourier_forward'): 67138560 + 21350912,
+    ('fp32', 'legendre_forward'): 84777216 + 30014208,
+    ('tf32x3', 'legendre_inverse'): 91981568 + 22877184,
+    ('tf32x3', 'legendre_forward'): 135050240 + 35883776,
 }
 
 

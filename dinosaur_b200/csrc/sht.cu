@@ -428,10 +428,10 @@ int legendre_forward_fp32(dino_plan* p, const float* G, float* out, int nf,
 // one issue slot does both columns' add, multiply or FMA at the plain lane
 // rate (126 lane results per SM and clock, measured for fma and fma.f32x2
 // alike).  With one column per thread the kernels issued in 57-70 % of the
-// slots; now 35 %, and they wait on memory (long scoreboard 44 % of the stall
-// cycles at TL255).  T42 x 900 fields: inverse 18.6 -> 12.4 us, forward 14.7 ->
-// 10.6 us; T85 x 128: 10.7 -> 8.4, 10.5 -> 8.4 us; TL255 x 128: 37.0 -> 37.1,
-// 33.0 -> 31.1 us.  Against direct sums for lengths that are no power of two:
+// slots; now 29-34 %, and they wait on memory (long scoreboard is the largest
+// stall at TL255).  T42 x 900 fields: inverse 18.6 -> 12.4 us, forward 14.7 ->
+// 10.6 us; T85 x 128: 10.7 -> 8.4, 10.5 -> 8.4 us; TL255 x 128: 37.0 -> 32.2,
+// 33.0 -> 29.7 us (with launches overlapping).  Against direct sums for lengths that are no power of two:
 // TL159 x 75 fields 615 -> 10.4 us and 636 -> 10.4 us.
 // ---------------------------------------------------------------------------
 
