@@ -187,7 +187,7 @@ class FusedSIL3Step:
     return buf
 
 
-@dataclasses.dataclass
+@dataclasses.dataclass(eq=False)  # compared and hashed by identity, as a function is
 class FusedShallowWaterStep:
   """One or more filtered SIL3 steps of the shallow-water equations.
 

@@ -5,9 +5,11 @@ import ctypes
 import os
 import re
 
+import numpy as np
 import pytest
 
 from dinosaur_b200 import _lib
+from dinosaur_b200 import time_integration
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
@@ -84,3 +86,12 @@ def test_descriptor_layouts_match_the_header(cname, pyname, tmp_path):
                                         text=True).stdout.split()]
   assert out[0] == ctypes.sizeof(py), (out[0], ctypes.sizeof(py))
   assert out[1:] == [getattr(py, f).offset for f in fields]
+
+
+def test_shallow_water_steps_are_hashable_like_functions():
+  # Step functions serve as keys (of caches, of registries); each is its own.
+  scaling = time_integration.SpectralStepFilter(np.ones(4))
+  a = time_integration.FusedShallowWaterStep(None, 0.1, (scaling,))
+  b = time_integration.FusedShallowWaterStep(None, 0.1, (scaling,))
+  assert {a: 1, b: 2}[a] == 1
+  assert a == a and a != b
